@@ -417,8 +417,11 @@ int run_entropies(const Cx<Real> *states, int n, const std::vector<EntReq> &reqs
                 continue;
             }
         }
-        // Purity straight from tiles when there are enough tiles to fill the GPU.
-        const bool tile_purity = !vn && tiles * static_cast<long long>(list.size()) >= 2 * 152;
+        // Purity straight from tiles when there are enough tiles to fill the GPU;
+        // up to 64 rows rho is cheap to write and the small-set Gram is faster
+        // than one padded 64 x 64 tile, so only its sums follow that rule.
+        const bool many = !vn && tiles * static_cast<long long>(list.size()) >= 2 * 152;
+        const bool tile_purity = many && k > 6;
         std::size_t per_launch = list.size();
         if (!tile_purity) per_launch = std::max<std::size_t>(1, std::min(list.size(), kMaxRhoBytes / rho_bytes));
         for (std::size_t b0 = 0; b0 < list.size(); b0 += per_launch)
@@ -455,7 +458,7 @@ int run_entropies(const Cx<Real> *states, int n, const std::vector<EntReq> &reqs
             const bool large = vn && d > jacobi_max_dim();
             if (large) MG_CUDA(ws.dims.ensure(sizeof(int) * nb));
             MG_CUDA(gram_rho<Real>(states, n, ws.jobs.as<GramJob>(), nbi, k, col, col_stride, ws.rho.as<double>(),
-                                   ws.scratch.p, ws.scratch.bytes, s, large ? ws.dims.as<int>() : nullptr));
+                                   ws.scratch.p, ws.scratch.bytes, s, large ? ws.dims.as<int>() : nullptr, many));
             launches += 2;
             if (!vn)
             {

@@ -476,6 +476,287 @@ __global__ void __launch_bounds__(kGramThreads)
     }
 }
 
+// The Gram of small kept sets (k <= 6: d = 2^k <= 64 rows of rho) over all
+// environment columns of a split. A 64 x 64 tile of k_gram would be mostly
+// padding here (16 x 16 of it for k = 4), so the CTA's threads are dealt
+// out by the job's own d: the lower triangle of rho splits into 4 x 4
+// sub-blocks, and L = small_lanes(d) consecutive threads share one, each
+// taking every L-th column. Chunks of 2048 amplitudes (all rows, the lowest
+// environment modes) are staged in shared memory; their address bits are
+// enumerated in ascending qubit order, so a warp reads 32 neighbouring
+// amplitudes whatever the kept set. Bound by the FP64 rate (exact sums) or
+// FP32 issue (compensated sums, ten operations per product).
+//   Sums kExact: products in FP64 (FP32 operands widened once, when staged).
+//   Sums kCompensated: FP32 runs of at least 256 columns per thread, each a
+//     compensated dot product, added to FP64 totals (see k_gram).
+//   Sums kRuns: plain FP32 runs of as many columns, added to FP64 totals
+//     (purities of many jobs, which need no more).
+// Measured on GB300 against the padded 64 x 64 tile: 200 trajectories of the
+// L = 12 FP64 chain with every observable per layer (regions of 3 and 6
+// modes) 542 -> 193 ms; 48 of the L = 20 FP32 ring with per-layer S_2 and TMI
+// (five-mode quarters) 404 -> 83 ms.
+enum class Sums
+{
+    kExact,
+    kCompensated,
+    kRuns
+};
+constexpr int kSmallThreads = 160;
+constexpr int kSmallChunkBits = 11;
+constexpr int kSmallMaxK = 6;
+
+// Threads per 4 x 4 sub-block: d = 64 has 136 sub-blocks, 32 has 36, 16 has
+// 10, 8 has 3; the products fill at most 160 threads.
+__device__ __forceinline__ int small_lanes(int d) { return d >= 64 ? 1 : d == 32 ? 4 : d == 16 ? 16 : 32; }
+
+template <typename Real, Sums kSums>
+__global__ void __launch_bounds__(kSmallThreads)
+    k_gram_small(const Cx<Real> *__restrict__ states, int n, const GramJob *__restrict__ jobs,
+                 const Collapse *__restrict__ col, std::size_t col_stride, int splits, double *__restrict__ part_out,
+                 int compact, int *__restrict__ dims_out)
+{
+    using SReal = typename std::conditional<kSums == Sums::kExact, double, Real>::type;
+    constexpr int PAD = sizeof(SReal) == 4 ? 2 : 1; // column stride: 16-byte aligned, off the bank period
+    __shared__ GramJob J;
+    __shared__ __align__(16) Cx<SReal> tile[(1 << kSmallChunkBits) + (512 * PAD)];
+    __shared__ std::uint64_t g_lo[32], g_hi[64], cross[64], env_bit[40];
+    __shared__ int s_lo[32], s_hi[64]; // (column << 8) | row of a chunk index's low and high bits
+    __shared__ std::uint64_t s_fixed, s_keptmask, s_envmask;
+    __shared__ int s_k, s_check, s_rowbit[40];
+
+    const int tid = threadIdx.x;
+    const int job = blockIdx.y;
+    for (int i = tid; i < static_cast<int>(sizeof(GramJob) / 4); i += kSmallThreads)
+        reinterpret_cast<int *>(&J)[i] = reinterpret_cast<const int *>(jobs + job)[i];
+    __syncthreads();
+    Collapse cl{0, 0, 1.0, 0};
+    const bool has_col = col != nullptr;
+    if (has_col) cl = col[J.traj * col_stride];
+    const int D = 1 << J.k;
+    if (tid == 0)
+    {
+        // The reduced geometry of a compact job, as in k_gram: measured sites
+        // leave both lists, and the smaller side becomes the rows.
+        std::uint64_t kept = 0;
+        for (int i = 0; i < J.k; ++i) kept |= 1ull << J.kept[i];
+        std::uint64_t env = ((1ull << n) - 1ull) & ~kept;
+        const bool reduce = compact && !J.fermion;
+        const std::uint64_t drop = reduce && cl.parity == 0 ? cl.mask : 0ull;
+        const bool swap = reduce && __popcll(env & ~drop) < __popcll(kept & ~drop);
+        int a = 0;
+        if (swap)
+        {
+            const std::uint64_t t = kept;
+            kept = env;
+            env = t;
+            for (int q = 0; q < n; ++q)
+                if (((kept & ~drop) >> q) & 1ull) s_rowbit[q] = a++;
+        }
+        else
+            for (int i = 0; i < J.k; ++i)
+                if (!((drop >> J.kept[i]) & 1ull)) s_rowbit[J.kept[i]] = a++;
+        s_k = a;
+        s_keptmask = kept & ~drop;
+        s_envmask = env & ~drop;
+        s_fixed = cl.value & drop;
+        s_check = has_col && drop == 0ull ? 1 : 0;
+        if (dims_out != nullptr && blockIdx.x == 0) dims_out[job] = 1 << a;
+    }
+    __syncthreads();
+    const int k = s_k, d = 1 << k;
+    const int dr = d < 4 ? 4 : d; // rows staged (zeros past d)
+    const std::uint64_t keptmask = s_keptmask, envmask = s_envmask;
+    const int nenv = __popcll(envmask);
+    const int cmax = kSmallChunkBits - (k < 2 ? 2 : k);
+    const int c = nenv < cmax ? nenv : cmax; // environment modes in a chunk
+    const int stride = dr + PAD, ncols = 1 << c, bits = k + c;
+    // Chunk index bit b <-> the b-th lowest qubit among the rows' modes and
+    // the c lowest environment modes.
+    if (tid < n && ((envmask >> tid) & 1ull)) env_bit[__popcll(envmask & ((1ull << tid) - 1ull))] = 1ull << tid;
+    if (tid < 64)
+    {
+        std::uint64_t x = 0;
+        if (J.fermion)
+            for (int i = 0; i < J.k; ++i)
+                if ((tid >> i) & 1) x ^= J.below[i];
+        cross[tid] = x;
+    }
+    if (tid < 96)
+    {
+        // Entry tid < 32: low five index bits; else the six high ones.
+        const int v = tid < 32 ? tid : (tid - 32) << 5;
+        std::uint64_t gofs = 0;
+        int pos = 0, b = 0, e = 0;
+        for (int q = 0; q < n && b < bits; ++q)
+        {
+            const bool is_row = (keptmask >> q) & 1ull, is_env = (envmask >> q) & 1ull;
+            if (!is_row && !(is_env && e < c)) continue;
+            if ((v >> b) & 1)
+            {
+                gofs |= 1ull << q;
+                pos |= is_row ? 1 << s_rowbit[q] : 256 << e;
+            }
+            if (is_env) ++e;
+            ++b;
+        }
+        if (tid < 32)
+        {
+            g_lo[tid] = gofs;
+            s_lo[tid] = pos;
+        }
+        else
+        {
+            g_hi[tid - 32] = gofs;
+            s_hi[tid - 32] = pos;
+        }
+    }
+    if (d < dr)
+        for (int i = tid; i < ncols * stride; i += kSmallThreads) tile[i] = Cx<SReal>{SReal(0), SReal(0)};
+    __syncthreads();
+
+    const Cx<Real> *psi = states + (static_cast<std::size_t>(J.traj) << n);
+    const std::uint64_t nchunk = 1ull << (nenv - c);
+    const std::uint64_t beg = nchunk * blockIdx.x / splits, end = nchunk * (blockIdx.x + 1) / splits;
+    const bool check = s_check != 0;
+    const int fermion = J.fermion;
+    const int L = small_lanes(dr), t4 = dr >> 2;
+    const int sub = tid / L, cg = tid % L;
+    const bool active = sub < t4 * (t4 + 1) / 2;
+    int ti = 0, tj = 0;
+    if (active) tile_coords(sub, ti, tj);
+
+    using Run = typename std::conditional<kSums == Sums::kExact, double, float>::type;
+    constexpr bool kFlush = kSums != Sums::kExact;
+    double accr[kFlush ? 4 : 1][kFlush ? 4 : 1], acci[kFlush ? 4 : 1][kFlush ? 4 : 1];
+    Run runr[4][4], runi[4][4];
+    constexpr int NC = kSums == Sums::kCompensated ? 4 : 1;
+    float cmpr[NC][NC], cmpi[NC][NC];
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+        {
+            runr[i][j] = runi[i][j] = Run(0);
+            if constexpr (kFlush) accr[i][j] = acci[i][j] = 0.0;
+            if constexpr (NC == 4) cmpr[i][j] = cmpi[i][j] = 0.f;
+        }
+    int run_cols = 0;
+    const int lane = tid & 31, warp = tid >> 5;
+    for (std::uint64_t ch = beg; ch < end; ++ch)
+    {
+        std::uint64_t base = s_fixed;
+        for (int b = c; b < nenv; ++b)
+            if ((ch >> (b - c)) & 1ull) base |= env_bit[b];
+        if (lane < (1 << bits))
+        {
+            const std::uint64_t gl = base | g_lo[lane];
+            const int pl = s_lo[lane];
+            const int nhi = bits > 5 ? 1 << (bits - 5) : 1;
+#pragma unroll 4
+            for (int h = warp; h < nhi; h += kSmallThreads / 32)
+            {
+                const int p = pl | s_hi[h];
+                const int row = p & 255, cc = p >> 8;
+                const bool neg = fermion && (__popcll(((ch << c) | static_cast<std::uint64_t>(cc)) & cross[row]) & 1);
+                const Cx<Real> v = gather(psi, gl | g_hi[h], cl, check, has_col, neg);
+                tile[cc * stride + row] = Cx<SReal>{static_cast<SReal>(v.re), static_cast<SReal>(v.im)};
+            }
+        }
+        __syncthreads();
+        if (active)
+        {
+            for (int cc = cg; cc < ncols; cc += L)
+            {
+                const Cx<SReal> *pa = tile + cc * stride + ti * 4, *pb = tile + cc * stride + tj * 4;
+                Cx<SReal> a[4], b[4];
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+                {
+                    a[i] = pa[i];
+                    b[i] = pb[i];
+                }
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+#pragma unroll
+                    for (int j = 0; j < 4; ++j)
+                    {
+                        // a * conj(b)
+                        if constexpr (kSums == Sums::kCompensated)
+                        {
+                            comp_fma(a[i].re, b[j].re, runr[i][j], cmpr[i][j]);
+                            comp_fma(a[i].im, b[j].im, runr[i][j], cmpr[i][j]);
+                            comp_fma(a[i].im, b[j].re, runi[i][j], cmpi[i][j]);
+                            comp_fma(-a[i].re, b[j].im, runi[i][j], cmpi[i][j]);
+                        }
+                        else
+                        {
+                            runr[i][j] = fma(a[i].re, b[j].re, runr[i][j]);
+                            runr[i][j] = fma(a[i].im, b[j].im, runr[i][j]);
+                            runi[i][j] = fma(a[i].im, b[j].re, runi[i][j]);
+                            runi[i][j] = fma(-a[i].re, b[j].im, runi[i][j]);
+                        }
+                    }
+            }
+            if constexpr (kFlush)
+            {
+                run_cols += (ncols + L - 1) / L;
+                if (run_cols >= 256 || ch + 1 == end)
+                {
+#pragma unroll
+                    for (int i = 0; i < 4; ++i)
+#pragma unroll
+                        for (int j = 0; j < 4; ++j)
+                        {
+                            accr[i][j] += static_cast<double>(runr[i][j]);
+                            acci[i][j] += static_cast<double>(runi[i][j]);
+                            runr[i][j] = runi[i][j] = Run(0);
+                            if constexpr (NC == 4)
+                            {
+                                accr[i][j] += static_cast<double>(cmpr[i][j]);
+                                acci[i][j] += static_cast<double>(cmpi[i][j]);
+                                cmpr[i][j] = cmpi[i][j] = 0.f;
+                            }
+                        }
+                    run_cols = 0;
+                }
+            }
+        }
+        __syncthreads();
+    }
+
+    // Sum over the L threads of a sub-block, then the split's partial rho
+    // (rows and columns past d, of a reduced job, are zero).
+    double *out = part_out + (static_cast<std::size_t>(job) * splits + blockIdx.x) * static_cast<std::size_t>(D) * D * 2;
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+        {
+            double x, y;
+            if constexpr (kFlush)
+            {
+                x = accr[i][j];
+                y = acci[i][j];
+            }
+            else
+            {
+                x = runr[i][j];
+                y = runi[i][j];
+            }
+            for (int o = L >> 1; o > 0; o >>= 1)
+            {
+                x += __shfl_down_sync(0xffffffffu, x, o, L);
+                y += __shfl_down_sync(0xffffffffu, y, o, L);
+            }
+            const int r = ti * 4 + i, cc = tj * 4 + j;
+            if (active && cg == 0 && r < d && cc < d && r >= cc)
+                reinterpret_cast<double2 *>(out)[r * D + cc] = make_double2(x, y);
+        }
+    if (d < D)
+        for (int i = tid; i < D * D; i += kSmallThreads)
+            if (i / D >= d) reinterpret_cast<double2 *>(out)[i] = make_double2(0.0, 0.0);
+}
+
 __global__ void k_gram_finalize(const double *__restrict__ part, int d, int splits, int njobs, double *__restrict__ rho)
 {
     const std::uint64_t per = static_cast<std::uint64_t>(d) * d;
@@ -863,9 +1144,18 @@ __global__ void k_rho3_finalize(const double *__restrict__ part, int chunks, int
 int gram_splits(int n, int k, int njobs, bool rho)
 {
     if (!rho) return 1;
+    int splits = 1;
+    if (k <= kSmallMaxK)
+    {
+        // About six CTAs per SM, at least one chunk each; the partials of one
+        // job stay within 16 MB.
+        const int most = n > kSmallChunkBits ? std::min(1 << (n - kSmallChunkBits < 10 ? n - kSmallChunkBits : 10),
+                                                        1 << (20 - 2 * k)) : 1;
+        while (njobs * splits < 6 * 152 && splits < most) splits *= 2;
+        return splits;
+    }
     const std::uint64_t E = 1ull << (n - k);
     const int tiles = gram_tiles(k) * njobs;
-    int splits = 1;
     while (tiles * splits < 2 * 152 && E / (2ull * splits) >= static_cast<std::uint64_t>(TK) * 8) splits *= 2;
     return splits;
 }
@@ -881,7 +1171,7 @@ std::size_t gram_scratch_bytes(int n, int k, int njobs, bool rho)
 template <typename Real>
 cudaError_t gram_rho(const Cx<Real> *states, int n, const GramJob *d_jobs, int njobs, int k,
                      const Collapse *collapse, std::size_t collapse_stride, double *rho_out, void *scratch,
-                     std::size_t scratch_bytes, cudaStream_t s, int *dims_out)
+                     std::size_t scratch_bytes, cudaStream_t s, int *dims_out, bool plain_runs)
 {
     if (njobs <= 0) return cudaSuccess;
     const int splits = gram_splits(n, k, njobs, true);
@@ -903,7 +1193,29 @@ cudaError_t gram_rho(const Cx<Real> *states, int n, const GramJob *d_jobs, int n
     // eigenvalues (half-chain spectra of L = 16 and 18: 1.7x faster QL).
     bool comp = false;
     if constexpr (sizeof(Real) == 4) comp = compensated_rho_sums() && n - k >= k + 6;
-    if (comp)
+    if (k <= kSmallMaxK)
+    {
+        const dim3 g(splits, njobs);
+        double *part = static_cast<double *>(scratch);
+        bool launched = false;
+        if constexpr (sizeof(Real) == 4)
+        {
+            if (plain_runs || comp)
+            {
+                if (plain_runs)
+                    k_gram_small<Real, Sums::kRuns><<<g, kSmallThreads, 0, s>>>(
+                        states, n, d_jobs, collapse, collapse_stride, splits, part, compact, dims_out);
+                else
+                    k_gram_small<Real, Sums::kCompensated><<<g, kSmallThreads, 0, s>>>(
+                        states, n, d_jobs, collapse, collapse_stride, splits, part, compact, dims_out);
+                launched = true;
+            }
+        }
+        if (!launched)
+            k_gram_small<Real, Sums::kExact><<<g, kSmallThreads, 0, s>>>(
+                states, n, d_jobs, collapse, collapse_stride, splits, part, compact, dims_out);
+    }
+    else if (comp)
     {
         if constexpr (sizeof(Real) == 4)
             k_gram<Real, double, true, true><<<grid, kGramThreads, 0, s>>>(
@@ -2080,7 +2392,7 @@ cudaError_t gram_purity_tc(const Cx<float> *states, int n, const GramJob *d_jobs
 
 #define MG_INST(R)                                                                                               \
     template cudaError_t gram_rho<R>(const Cx<R> *, int, const GramJob *, int, int, const Collapse *, std::size_t, \
-                                     double *, void *, std::size_t, cudaStream_t, int *);                        \
+                                     double *, void *, std::size_t, cudaStream_t, int *, bool);                  \
     template cudaError_t gram_purity<R>(const Cx<R> *, int, const GramJob *, int, int, const Collapse *,          \
                                         std::size_t, double *, void *, std::size_t, cudaStream_t);               \
     template cudaError_t rho3_sweep<R>(const Cx<R> *, int, int, const int *, int, int, const Collapse *,          \

@@ -43,11 +43,12 @@ inline int gram_tiles(int k)
 // non-fermionic jobs leave out the sites it measured (the state is a product
 // on them, so the spectrum and purity are those of the reduced matrix): rho
 // then holds that 2^k' x 2^k' matrix in its leading rows and columns, zeros
-// elsewhere, and dims_out[job] (nullable) receives 2^k'.
+// elsewhere, and dims_out[job] (nullable) receives 2^k'. plain_runs: FP32
+// states' products may be summed in plain FP32 runs (purities; k <= 6 only).
 template <typename Real>
 cudaError_t gram_rho(const Cx<Real> *states, int n, const GramJob *d_jobs, int njobs, int k,
                      const Collapse *collapse, std::size_t collapse_stride, double *rho_out, void *scratch,
-                     std::size_t scratch_bytes, cudaStream_t s, int *dims_out = nullptr);
+                     std::size_t scratch_bytes, cudaStream_t s, int *dims_out = nullptr, bool plain_runs = false);
 
 // Purity Tr(rho^2) of every job without materialising rho.
 template <typename Real>
