@@ -298,14 +298,14 @@ struct Workspace
 };
 
 // Spectra up to this many rows go to the one-block Jacobi eigensolver, larger
-// ones to Householder tridiagonalisation + QL (MIPT_GB300_JACOBI_MAX_D, at
-// most 64; default 16: from 32 rows on the reduction needs far fewer FP64
-// operations than Jacobi sweeps).
+// ones to Householder tridiagonalisation + Sturm counts (MIPT_GB300_JACOBI_MAX_D, at
+// most 64; default 1: the reduction needs far fewer FP64 operations than
+// Jacobi sweeps; 800 matrices of 8 rows take 0.33 ms by Jacobi).
 int jacobi_max_dim()
 {
     static const int d = [] {
         const char *v = std::getenv("MIPT_GB300_JACOBI_MAX_D");
-        const int x = v ? std::atoi(v) : 16;
+        const int x = v ? std::atoi(v) : 1;
         return std::max(1, std::min(64, x));
     }();
     return d;
@@ -477,16 +477,18 @@ int run_entropies(const Cx<Real> *states, int n, const std::vector<EntReq> &reqs
             else
             {
                 // Large spectra: FP64 Householder tridiagonalisation and
-                // implicit QL of every matrix of the group (eigen.cu).
+                // Sturm counts of every matrix of the group (eigen.cu).
                 MG_CUDA(ws.eig.ensure(sizeof(double) * hermitian_eig_scratch_doubles(d, nbi)));
                 if (!ws.eig_err.p)
                 {
                     MG_CUDA(ws.eig_err.ensure(sizeof(int)));
                     MG_CUDA(cudaMemsetAsync(ws.eig_err.p, 0, sizeof(int), s));
                 }
+                int launched = 0;
                 MG_CUDA(hermitian_eig_entropy(ws.rho.as<double>(), d, nbi, ws.vals.as<double>(), nullptr,
-                                              ws.eig.as<double>(), ws.eig_err.as<int>(), s, ws.dims.as<int>()));
-                launches += 2;
+                                              ws.eig.as<double>(), ws.eig_err.as<int>(), s, ws.dims.as<int>(),
+                                              &launched));
+                launches += launched;
                 k_scatter<<<(nbi + 255) / 256, 256, 0, s>>>(ws.vals.as<double>(), ws.idx.as<int>(), nbi, d_out, 0);
                 ++launches;
             }

@@ -8,44 +8,43 @@
 // from cuSOLVER (heevd / gesvd); here it is computed by two kernels of our
 // own, written from the textbook algorithms:
 //
-//   k_tridiag   one CTA per matrix: Householder reduction of the Hermitian
-//               matrix (row-major, interleaved re/im, the lower triangle
-//               read and updated) to a real
-//               symmetric tridiagonal matrix. Step j reflects the column below
-//               the diagonal onto alpha e_1 with H = I - beta v v^H,
-//               v = x - alpha e_1, alpha = -phase(x_0) |x|, beta = 2 / |v|^2,
-//               and updates the trailing block B <- H B H as
-//               B - v w^H - w v^H with p = beta B v, K = beta/2 v^H p,
-//               w = p - K v. The off-diagonal |alpha| is kept (a Hermitian
-//               tridiagonal matrix with complex off-diagonals is unitarily
-//               similar to the real one with their moduli).
-//   k_tridiag_ql one thread per matrix: eigenvalues of the tridiagonal matrix
-//               by the implicit QL iteration with Wilkinson-type shifts and
-//               plane rotations (the tql1/tqli scheme of EISPACK and
-//               Numerical Recipes, eigenvalues only), then the entropy.
+//   k_tridiag_cluster  Householder reduction of the Hermitian matrix to a
+//               real symmetric tridiagonal matrix, up to 256 rows: the matrix
+//               stays in the shared memory of a cluster of CTAs. A step
+//               reflects the vector x beside the diagonal onto alpha e_1 with
+//               H = I - beta v v^H, v = x - alpha e_1,
+//               alpha = -phase(x_0) |x|, beta = 2 / |v|^2, and updates the
+//               block B that is left, B <- H B H, as B - v w^H - w v^H with
+//               p = beta B v, K = beta/2 v^H p, w = p - K v. The off-diagonal
+//               |alpha| is kept (a Hermitian tridiagonal matrix with complex
+//               off-diagonals is unitarily similar to the real one with their
+//               moduli).
+//   k_tridiag   the same for up to 4096 rows, the matrix (row-major,
+//               interleaved re/im, the lower triangle read and updated) in
+//               global memory: one CTA per matrix, or several with barriers
+//               between them.
+//   k_tridiag_sturm  one thread per eigenvalue (tridiag.cuh), then the
+//               entropy.
 //
 // All reductions run in a fixed order, so results are reproducible.
 // FP64 throughout: GB300's FP64 rate bounds the reduction at about 16/3 d^3
 // flops per matrix (full matrix-vector product, lower-triangle update).
 #include "observables.cuh"
+#include "tridiag.cuh"
 
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
 #include <algorithm>
 #include <cmath>
 #include <cstdint>
+#include <type_traits>
 
 namespace mg
 {
 namespace
 {
 constexpr int kTriThreads = 512;
-constexpr int kQlMaxIter = 60;
-
-__device__ __forceinline__ double2 cmul_conj(double2 a, double2 b) // a * conj(b)
-{
-    return make_double2(a.x * b.x + a.y * b.y, a.y * b.x - a.x * b.y);
-}
 
 // Block sum in a fixed order: per-warp shuffle trees, then warp 0 sums the
 // warp totals. `red` holds at least 32 doubles. Every thread gets the sum.
@@ -252,94 +251,460 @@ __global__ void __launch_bounds__(kTriThreads)
     }
 }
 
-// Implicit QL on one symmetric tridiagonal matrix (diagonal dg[0..d), off-
-// diagonal of[0..d-1), of[j] coupling j and j+1); eigenvalues overwrite dg.
-// Returns false if an eigenvalue needs more than kQlMaxIter sweeps.
-__device__ bool tridiag_ql(double *dg, double *of, int d)
+// The same reduction with the matrix resident in shared memory: one cluster
+// of C CTAs per matrix, CTA r holding the lower-triangle rows i = r (mod C)
+// packed. Rows are eliminated from the last one up, so the block that is left
+// always starts at row and column 0 (aligned with the lanes) and the row that
+// gives the next reflector lies in one CTA. One sweep over the lower triangle per step
+// applies the previous step's rank-2 update and accumulates p = B v for this
+// one, from each entry both as B_ik and as conj(B_ki): sixteen FP64 FMAs per
+// entry read and written once. A lane owns columns k = lane (mod 32): the
+// column sums stay in registers over a warp's rows, and the row sums of two
+// rows share one six-add shuffle tree. CTAs exchange their partial p once per
+// step, behind one cluster barrier; the partials alternate between two
+// buffers, so a CTA that runs ahead never overwrites what another still reads.
+// What bounds it is the FP64 pipe (a warp instruction takes 20 clocks of an
+// SM, however many lanes are on), so whatever is not the sweep runs on as few
+// warps as hold data: the reflector's roots and divisions on one warp, sums on
+// the warps below row m. Measured against the reduction in global memory:
+// 34 launches of 64 matrices of up to 256 rows 533 -> 259 ms, 48 launches of
+// 800 of up to 64 rows 156 -> 62 ms, one of 256 rows 5.4 -> 3.8 ms.
+template <int NCB, int THREADS>
+__global__ void __launch_bounds__(THREADS)
+    k_tridiag_cluster(const double2 *__restrict__ mats, int d, double *__restrict__ diag, double *__restrict__ off,
+                      const int *__restrict__ dims)
 {
-    // Off-diagonals below eps * |T| count as zero: eigenvalues are then
-    // exact to about eps * |T| in absolute terms, far below the entropy's
-    // 1e-15 eigenvalue cut-off for a density matrix.
-    double anorm = 0.0;
-    for (int i = 0; i < d; ++i) anorm = fmax(anorm, fabs(dg[i]) + fabs(of[i]) + (i > 0 ? fabs(of[i - 1]) : 0.0));
-    const double tiny = 2.220446049250313e-16 * anorm;
-    for (int l = 0; l < d; ++l)
+    namespace cg = cooperative_groups;
+    cg::cluster_group cluster = cg::this_cluster();
+    const int C = static_cast<int>(cluster.num_blocks()), r = static_cast<int>(cluster.block_rank());
+    constexpr int NW = THREADS / 32;
+    constexpr int HB = NCB < 4 ? NCB : 4; // column blocks in flight together, at most
+    constexpr int NP = (32 * NCB + THREADS - 1) / THREADS;
+    extern __shared__ __align__(16) double2 csm[];
+    constexpr int DS = 32 * NCB;                                  // >= d; every lane may read a vector
+    double2 *v = csm, *vp = v + DS, *wp = vp + DS, *prow = wp + DS; // reflector, previous v and w, row sums
+    double2 *pcw = prow + DS;                                     // [NW][DS] column sums per warp
+    double2 *pivot = pcw + NW * DS;                               // [2][DS] pivot rows (C > 1)
+    double2 *part = pivot + (C > 1 ? 2 * DS : 0);                 // [2][C][DS] every CTA's partial p (C > 1)
+    double2 *rows = part + (C > 1 ? 2 * C * DS : 0);              // packed rows
+    __shared__ double red[NW], s_nt, s_beta;
+    const int mat = blockIdx.x / C;
+    const double2 *a = mats + static_cast<std::size_t>(mat) * d * d;
+    double *dg = diag + static_cast<std::size_t>(mat) * d;
+    double *of = off + static_cast<std::size_t>(mat) * d;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int dm = dims != nullptr ? dims[mat] : d;
+    // Local row li is row li * C + r and starts at row_at(li, r).
+    auto row_at = [C](int li, int rr) { return li * (rr + 1) + C * (li * (li - 1) / 2); };
+    auto warp_sum = [](double x) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+        return x;
+    };
+    // Sum of red[0 .. active) in every lane of a warp.
+    auto red_sum = [&](int active) {
+        double x = lane < active ? red[lane] : 0.0;
+#pragma unroll
+        for (int o = NW / 2; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+        return __shfl_sync(0xffffffffu, x, 0);
+    };
+
+    for (int li = warp; li * C + r < dm; li += NW)
     {
-        int iter = 0;
-        for (;;)
-        {
-            int m = l;
-            for (; m + 1 < d; ++m)
-            {
-                const double dd = fabs(dg[m]) + fabs(dg[m + 1]);
-                if (fabs(of[m]) <= 2.220446049250313e-16 * dd || fabs(of[m]) <= tiny) break;
-            }
-            if (m == l) break;
-            if (++iter > kQlMaxIter) return false;
-            // Shift from the leading 2x2 block's eigenvalue nearer dg[l].
-            double g = (dg[l + 1] - dg[l]) / (2.0 * of[l]);
-            double r = hypot(g, 1.0);
-            g = dg[m] - dg[l] + of[l] / (g + copysign(r, g));
-            double s = 1.0, c = 1.0, p = 0.0;
-            int i = m - 1;
-            bool underflow = false;
-            for (; i >= l; --i)
-            {
-                const double f = s * of[i], b = c * of[i];
-                // The entries of a density matrix's tridiagonal form are at
-                // most 1 in modulus, so f^2 + g^2 needs no scaling; one
-                // reciprocal square root gives r, s and c (a shorter
-                // dependent chain than hypot and a division).
-                const double t = fma(f, f, g * g);
-                if (t == 0.0)
-                {
-                    of[i + 1] = 0.0;
-                    dg[i + 1] -= p;
-                    of[m] = 0.0;
-                    underflow = true;
-                    break;
-                }
-                const double ir = rsqrt(t);
-                r = t * ir;
-                of[i + 1] = r;
-                s = f * ir;
-                c = g * ir;
-                g = dg[i + 1] - p;
-                r = (dg[i] - g) * s + 2.0 * c * b;
-                p = s * r;
-                dg[i + 1] = g + p;
-                g = c * r - b;
-            }
-            if (underflow) continue;
-            dg[l] -= p;
-            of[l] = g;
-            of[m] = 0.0;
-        }
+        const int i = li * C + r;
+        for (int k = lane; k <= i; k += 32) rows[row_at(li, r) + k] = a[static_cast<std::size_t>(i) * d + k];
     }
-    return true;
+    for (int k = tid; k < DS; k += THREADS) v[k] = vp[k] = wp[k] = make_double2(0.0, 0.0);
+    // Row i to every CTA's pivot buffer (its owner calls it).
+    auto push_row = [&](int i, int buf) {
+        const double2 *src = rows + row_at(i / C, r);
+        for (int k = tid; k <= i; k += THREADS)
+        {
+            const double2 t = src[k];
+            for (int q = 0; q < C; ++q) cluster.map_shared_rank(pivot + buf * DS, q)[k] = t;
+        }
+    };
+    if (C > 1)
+    {
+        __syncthreads();
+        if ((dm - 1) % C == r) push_row(dm - 1, dm & 1);
+        cluster.sync();
+    }
+    else
+        __syncthreads();
+
+    for (int m = dm - 1; m >= 1; --m)
+    {
+        // Row m with the previous update applied; x = its conjugate transpose.
+        const double2 *rm = C > 1 ? pivot + ((m + 1) & 1) * DS : rows + row_at(m, 0);
+        const int aw = (m + 31) / 32 < NW ? (m + 31) / 32 : NW; // warps with an entry below m
+        if (warp < aw)
+        {
+            const double2 vm = vp[m], wm = wp[m];
+            double s = 0.0;
+            for (int k = tid; k < m; k += THREADS)
+            {
+                const double2 b = rm[k], pv = vp[k], pw = wp[k];
+                double2 x;
+                x.x = b.x - (vm.x * pw.x + vm.y * pw.y) - (wm.x * pv.x + wm.y * pv.y);
+                x.y = -(b.y - (vm.y * pw.x - vm.x * pw.y) - (wm.y * pv.x - wm.x * pv.y));
+                v[k] = x;
+                if (k < m - 1) s += x.x * x.x + x.y * x.y;
+            }
+            s = warp_sum(s);
+            if (lane == 0) red[warp] = s;
+        }
+        __syncthreads();
+        if (warp == 0)
+        {
+            const double sigma = red_sum(aw);
+            const double2 x0 = v[m - 1];
+            const double s0 = x0.x * x0.x + x0.y * x0.y;
+            // Roots from reciprocal roots (440 clocks; a division takes 650);
+            // hypot where the square is near underflow.
+            double ax0, ir;
+            if (s0 > 1e-280)
+            {
+                ir = rsqrt(s0);
+                ax0 = s0 * ir;
+            }
+            else
+            {
+                ax0 = hypot(x0.x, x0.y);
+                ir = ax0 > 0.0 ? 1.0 / ax0 : 0.0;
+            }
+            const bool reflect = !(sigma <= 1e-280); // else tridiagonal in this row already (NaN goes on)
+            const double t2 = s0 + sigma;
+            const double norm = reflect ? t2 * rsqrt(t2) : ax0;
+            const double top = ax0 + norm;
+            __syncwarp();
+            if (lane == 0)
+            {
+                if (r == 0)
+                {
+                    const double2 vm = vp[m], wm = wp[m];
+                    dg[m] = rm[m].x - 2.0 * (vm.x * wm.x + vm.y * wm.y);
+                    of[m - 1] = norm;
+                }
+                v[m - 1] = ir > 0.0 ? make_double2(x0.x * ir * top, x0.y * ir * top) : make_double2(top, 0.0);
+                s_nt = reflect ? norm * top : 0.0; // |v|^2 / 2
+            }
+        }
+        __syncthreads();
+        if (m == 1) break;
+        const double nt = s_nt;
+        // beta is needed after the sweep: one warp divides meanwhile.
+        if (warp == NW - 1 && lane == 0) s_beta = nt > 0.0 ? 1.0 / nt : 0.0;
+        if (!(nt > 0.0))
+        {
+            // No reflector, but the sweep still applies the previous update; a
+            // NaN comes here too and stays one.
+            for (int k = tid; k < m; k += THREADS) v[k] = make_double2(0.0 * nt, 0.0 * nt);
+            __syncthreads();
+        }
+
+        // The sweep: pairs of local rows dealt to the warps in snake order.
+        double2 pc[NCB];
+#pragma unroll
+        for (int c = 0; c < NCB; ++c) pc[c] = make_double2(0.0, 0.0);
+        const int lrows = m > r ? (m - r + C - 1) / C : 0; // local rows below m
+        const int pairs = (lrows + 1) / 2;
+        for (int t = 0; t * NW < pairs; ++t)
+        {
+            const int g = (t & 1) ? t * NW + NW - 1 - warp : t * NW + warp;
+            if (g >= pairs) continue;
+            const int l0 = 2 * g, l1 = 2 * g + 1;
+            const int i0 = l0 * C + r, i1 = l1 < lrows ? l1 * C + r : -1;
+            double2 *q0 = rows + row_at(l0, r), *q1 = rows + row_at(l1, r);
+            const double2 v0 = v[i0], vp0 = vp[i0], wp0 = wp[i0];
+            const int ic = i1 < 0 ? i0 : i1;
+            const double2 v1 = v[ic], vp1 = vp[ic], wp1 = wp[ic];
+            double s0r = 0.0, s0i = 0.0, s1r = 0.0, s1i = 0.0;
+            // N column blocks from c0 on: independent chains for the 64-clock
+            // latency, and no block that the row pair does not reach.
+            auto blocks = [&](auto first, auto count) {
+                constexpr int c0 = decltype(first)::value, N = decltype(count)::value;
+                double ar[2][N], ai[2][N];
+#pragma unroll
+                for (int cc = 0; cc < N; ++cc)
+                {
+                    const int c = c0 + cc, k = 32 * c + lane;
+                    const double2 vk = v[k], vpk = vp[k], wpk = wp[k];
+                    // Entries past the diagonal load and add zeros.
+                    auto entry = [&](double2 *q, int i, double2 vi, double2 vpi, double2 wpi, double &sr, double &si) {
+                        double2 b = make_double2(0.0, 0.0);
+                        if (k <= i) b = q[k];
+                        b.x = fma(-vpi.x, wpk.x, b.x);
+                        b.x = fma(-vpi.y, wpk.y, b.x);
+                        b.x = fma(-wpi.x, vpk.x, b.x);
+                        b.x = fma(-wpi.y, vpk.y, b.x);
+                        b.y = fma(-vpi.y, wpk.x, b.y);
+                        b.y = fma(vpi.x, wpk.y, b.y);
+                        b.y = fma(-wpi.y, vpk.x, b.y);
+                        b.y = fma(wpi.x, vpk.y, b.y);
+                        b.x = k <= i ? b.x : 0.0;
+                        b.y = k < i ? b.y : 0.0;
+                        if (k <= i) q[k] = b;
+                        sr = b.x * vk.x;
+                        sr = fma(-b.y, vk.y, sr);
+                        si = b.x * vk.y;
+                        si = fma(b.y, vk.x, si);
+                        const double bx = k < i ? b.x : 0.0;
+                        pc[c].x = fma(bx, vi.x, pc[c].x);
+                        pc[c].x = fma(b.y, vi.y, pc[c].x);
+                        pc[c].y = fma(bx, vi.y, pc[c].y);
+                        pc[c].y = fma(-b.y, vi.x, pc[c].y);
+                    };
+                    entry(q0, i0, v0, vp0, wp0, ar[0][cc], ai[0][cc]);
+                    entry(q1, i1, v1, vp1, wp1, ar[1][cc], ai[1][cc]);
+                }
+#pragma unroll
+                for (int cc = 0; cc < N; ++cc)
+                {
+                    s0r += ar[0][cc];
+                    s0i += ai[0][cc];
+                    s1r += ar[1][cc];
+                    s1i += ai[1][cc];
+                }
+            };
+            const int nblk = (ic >> 5) + 1;
+            using std::integral_constant;
+            auto tail = [&](auto first, int left) {
+                if (left == 1)
+                    blocks(first, integral_constant<int, 1>{});
+                else if (HB >= 2 && left == 2)
+                    blocks(first, integral_constant<int, (HB >= 2 ? 2 : 1)>{});
+                else if (HB >= 3 && left == 3)
+                    blocks(first, integral_constant<int, (HB >= 3 ? 3 : 1)>{});
+                else
+                    blocks(first, integral_constant<int, HB>{});
+            };
+            tail(integral_constant<int, 0>{}, nblk < HB ? nblk : HB);
+            if constexpr (NCB > HB)
+                if (nblk > HB) tail(integral_constant<int, HB>{}, nblk - HB);
+            // Four sums over the warp: value (lane >> 3) ends in its lanes.
+            const bool up = lane & 16, up2 = lane & 8;
+            double x = up ? s1r : s0r, y = up ? s1i : s0i;
+            x += __shfl_xor_sync(0xffffffffu, up ? s0r : s1r, 16);
+            y += __shfl_xor_sync(0xffffffffu, up ? s0i : s1i, 16);
+            double z = up2 ? y : x;
+            z += __shfl_xor_sync(0xffffffffu, up2 ? x : y, 8);
+            z += __shfl_xor_sync(0xffffffffu, z, 4);
+            z += __shfl_xor_sync(0xffffffffu, z, 2);
+            z += __shfl_xor_sync(0xffffffffu, z, 1);
+            if ((lane & 7) == 0)
+            {
+                const int i = up ? i1 : i0;
+                if (i >= 0) reinterpret_cast<double *>(prow + i)[up2 ? 1 : 0] = z;
+            }
+        }
+        const int sw = pairs < NW ? pairs : NW; // warps that swept rows
+        if (warp < sw)
+        {
+#pragma unroll
+            for (int c = 0; c < NCB; ++c)
+                if (32 * c + lane < m) pcw[warp * DS + 32 * c + lane] = pc[c];
+        }
+        __syncthreads();
+        double2 p[NP];
+        if (warp < aw)
+        {
+#pragma unroll
+            for (int u = 0; u < NP; ++u)
+            {
+                const int k = u * THREADS + tid;
+                p[u] = make_double2(0.0, 0.0);
+                if (k >= m) continue;
+                if (k % C == r) p[u] = prow[k];
+#pragma unroll
+                for (int q = 0; q < NW; ++q)
+                {
+                    if (q >= sw) break;
+                    const double2 t = pcw[q * DS + k];
+                    p[u].x += t.x;
+                    p[u].y += t.y;
+                }
+            }
+        }
+        if (C > 1)
+        {
+            double2 *mine = part + ((m & 1) * C + r) * DS;
+#pragma unroll
+            for (int u = 0; u < NP; ++u)
+            {
+                const int k = u * THREADS + tid;
+                if (k >= m) continue;
+                for (int q = 0; q < C; ++q) cluster.map_shared_rank(mine, q)[k] = p[u];
+            }
+            if ((m - 1) % C == r) push_row(m - 1, m & 1);
+            cluster.sync();
+            const double2 *all = part + (m & 1) * C * DS;
+#pragma unroll
+            for (int u = 0; u < NP; ++u)
+            {
+                const int k = u * THREADS + tid;
+                p[u] = make_double2(0.0, 0.0);
+                if (k >= m) continue;
+                for (int q = 0; q < C; q += 2)
+                {
+                    const double2 t0 = all[q * DS + k], t1 = all[(q + 1) * DS + k];
+                    p[u].x += t0.x + t1.x;
+                    p[u].y += t0.y + t1.y;
+                }
+            }
+        }
+        const double beta = s_beta;
+        // p = beta B v, K = beta/2 Re(v^H p) (real for Hermitian B), w = p - K v.
+        if (warp < aw)
+        {
+            double s = 0.0;
+#pragma unroll
+            for (int u = 0; u < NP; ++u)
+            {
+                const int k = u * THREADS + tid;
+                if (k >= m) continue;
+                p[u].x *= beta;
+                p[u].y *= beta;
+                s += v[k].x * p[u].x + v[k].y * p[u].y;
+            }
+            s = warp_sum(s);
+            if (lane == 0) red[warp] = s;
+        }
+        __syncthreads();
+        if (warp < aw)
+        {
+            const double K = 0.5 * beta * red_sum(aw);
+#pragma unroll
+            for (int u = 0; u < NP; ++u)
+            {
+                const int k = u * THREADS + tid;
+                if (k >= m) continue;
+                const double2 vk = v[k];
+                vp[k] = vk;
+                wp[k] = make_double2(p[u].x - K * vk.x, p[u].y - K * vk.y);
+            }
+        }
+        __syncthreads();
+    }
+    if (tid == 0 && r == 0)
+    {
+        // Row 0 (local row 0 of CTA 0) with the last update.
+        dg[0] = rows[0].x - 2.0 * (vp[0].x * wp[0].x + vp[0].y * wp[0].y);
+        of[dm - 1] = 0.0;
+        for (int i = dm; i < d; ++i) dg[i] = of[i] = 0.0;
+    }
+    cluster.sync(); // no CTA leaves while another may read its rows
 }
 
-__global__ void k_tridiag_ql(double *__restrict__ diag, double *__restrict__ off, int d, int nb,
-                             double *__restrict__ entropy, int *__restrict__ err, const int *__restrict__ dims)
+// Eigenvalues of every reduced matrix, one thread per eigenvalue (grid:
+// matrices x chunks of blockDim eigenvalues), and the entropy terms
+// -lambda log2 lambda over lambda > 1e-15; with one chunk per matrix the sum
+// too. The implicit QL iteration that this replaces is one serial chain of
+// about d^2 plane rotations per matrix at GB300's 64-clock FP64 latency. The 34
+// launches of 64 matrices of up to 256 rows: QL 972 ms, this 43 ms; one matrix
+// of 256 rows: 1.4 to 20 ms, this 0.9 ms.
+constexpr double kEigCutoff = 1e-15;
+
+__global__ void __launch_bounds__(128)
+    k_tridiag_sturm(double *__restrict__ diag, const double *__restrict__ off, int d, double *__restrict__ terms,
+                    double *__restrict__ entropy, int *__restrict__ err, const int *__restrict__ dims, int want_all)
 {
-    const int jb = blockIdx.x * blockDim.x + threadIdx.x;
-    if (jb >= nb) return;
-    double *dg = diag + static_cast<std::size_t>(jb) * d;
-    double *of = off + static_cast<std::size_t>(jb) * d;
+    extern __shared__ __align__(16) double2 de[];
+    float2 *df = reinterpret_cast<float2 *>(de + d);
+    __shared__ double red[33];
+    const int jb = blockIdx.x;
     const int dm = dims != nullptr ? dims[jb] : d;
-    if (!tridiag_ql(dg, of, dm))
+    const double *dg = diag + static_cast<std::size_t>(jb) * d;
+    const double *of = off + static_cast<std::size_t>(jb) * d;
+    // |T| (largest row sum; a NaN or an infinity anywhere makes `sum` one).
+    double top = 0.0, sum = 0.0;
+    for (int i = threadIdx.x; i < dm; i += blockDim.x)
     {
-        atomicOr(err, 1);
-        entropy[jb] = NAN;
-        return;
+        const double e0 = i > 0 ? fabs(of[i - 1]) : 0.0, e1 = i + 1 < dm ? fabs(of[i]) : 0.0;
+        const double t = fabs(dg[i]) + e0 + e1;
+        top = fmax(top, t);
+        sum += t;
+        de[i] = make_double2(dg[i], e0 * e0);
     }
+    sum = block_sum(sum, red);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) top = fmax(top, __shfl_xor_sync(0xffffffffu, top, o));
+    __syncthreads();
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = top;
+    __syncthreads();
+    top = red[0];
+    for (int q = 1; q < static_cast<int>(blockDim.x >> 5); ++q) top = fmax(top, red[q]);
+    const bool finite = sum - sum == 0.0;
+    const double floor2 = kTinyE2 * top * top, inv = top > 0.0 ? 1.0 / top : 0.0;
+    for (int i = threadIdx.x; i < dm; i += blockDim.x)
+    {
+        if (i > 0 && de[i].y < floor2) de[i].y = floor2;
+        df[i] = sturm_entry32(de[i], inv, i);
+    }
+    __syncthreads();
+    const int idx = blockIdx.y * blockDim.x + threadIdx.x;
+    double term = 0.0;
+    if (finite && idx < dm)
+    {
+        const double bound = top * (1.0 + 1e-14);
+        const double l =
+            top > 0.0 ? sturm_eigenvalue(de, df, dm, idx, top, bound, want_all ? -2.0 * bound : kEigCutoff) : 0.0;
+        if (want_all) diag[static_cast<std::size_t>(jb) * d + idx] = l;
+        if (l > kEigCutoff) term = -l * log2(l);
+    }
+    if (!finite && blockIdx.y == 0 && threadIdx.x == 0) atomicOr(err, 1);
+    if (gridDim.y == 1)
+    {
+        const double s = block_sum(term, red);
+        if (threadIdx.x == 0) entropy[jb] = !finite ? NAN : (fabs(s) < 1e-12 ? 0.0 : s);
+    }
+    else if (idx < d)
+        terms[static_cast<std::size_t>(jb) * d + idx] = finite ? term : NAN;
+}
+
+// entropy[job] = the sum of its d terms (fixed order).
+__global__ void __launch_bounds__(128) k_entropy_sum(const double *__restrict__ terms, int d, double *__restrict__ entropy)
+{
+    __shared__ double red[33];
     double s = 0.0;
-    for (int i = 0; i < dm; ++i)
+    for (int i = threadIdx.x; i < d; i += blockDim.x) s += terms[static_cast<std::size_t>(blockIdx.x) * d + i];
+    s = block_sum(s, red);
+    if (threadIdx.x == 0) entropy[blockIdx.x] = fabs(s) < 1e-12 ? 0.0 : s;
+}
+
+// Shared memory of k_tridiag_cluster for d rows over C CTAs.
+std::size_t cluster_smem(int d, int C, int warps)
+{
+    const int lr = d / C, vectors = 4 + warps + (C > 1 ? 2 + 2 * C : 0);
+    const std::size_t packed = static_cast<std::size_t>(lr) * C + static_cast<std::size_t>(C) * lr * (lr - 1) / 2;
+    return sizeof(double2) * (packed + static_cast<std::size_t>(vectors) * std::max(d, 32));
+}
+
+template <int NCB, int THREADS>
+cudaError_t launch_cluster(const double2 *rho, int d, int nb, int C, double *diag, double *off, cudaStream_t s,
+                           const int *dims)
+{
+    const std::size_t smem = cluster_smem(d, C, THREADS / 32);
+    cudaError_t e = cudaFuncSetAttribute(k_tridiag_cluster<NCB, THREADS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         static_cast<int>(smem));
+    if (e != cudaSuccess) return e;
+    if (C > 8)
     {
-        const double l = dg[i];
-        if (l > 1e-15) s -= l * log2(l);
+        e = cudaFuncSetAttribute(k_tridiag_cluster<NCB, THREADS>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+        if (e != cudaSuccess) return e;
     }
-    entropy[jb] = fabs(s) < 1e-12 ? 0.0 : s;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(nb * C);
+    cfg.blockDim = dim3(THREADS);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = C;
+    at.val.clusterDim.y = at.val.clusterDim.z = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, k_tridiag_cluster<NCB, THREADS>, rho, d, diag, off, dims);
 }
 } // namespace
 
@@ -351,51 +716,80 @@ std::size_t hermitian_eig_scratch_doubles(int d, int nb)
 }
 
 cudaError_t hermitian_eig_entropy(double *rho, int d, int nb, double *entropy_out, double *eig_out, double *scratch,
-                                  int *err, cudaStream_t s, const int *dims)
+                                  int *err, cudaStream_t s, const int *dims, int *launched)
 {
+    if (launched) *launched = 0;
     if (nb <= 0) return cudaSuccess;
     if (d < 2 || d > 4096) return cudaErrorInvalidValue;
     double *diag = eig_out ? eig_out : scratch;
     double *off = scratch + static_cast<std::size_t>(d) * nb;
     double2 *pglob = reinterpret_cast<double2 *>(scratch + 2 * static_cast<std::size_t>(d) * nb);
     unsigned *bars = reinterpret_cast<unsigned *>(scratch + 4 * static_cast<std::size_t>(d) * nb);
-    const std::size_t smem = 2 * sizeof(double2) * d;
-    cudaError_t e = cudaFuncSetAttribute(k_tridiag, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
-    if (e != cudaSuccess) return e;
-    // Fewer matrices than SMs: spread each matrix over `parts` resident CTAs
-    // (cooperative launch), at least 16 trailing rows per CTA.
-    int dev = 0, sms = 0, per_sm = 0;
-    int parts = 1;
-    if (cudaGetDevice(&dev) == cudaSuccess &&
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess &&
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_tridiag, kTriThreads, smem) == cudaSuccess &&
-        per_sm > 0)
+    int dev = 0, sms = 0;
+    cudaError_t e = cudaSuccess;
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0)
+        sms = 152;
+    if (d <= 256)
     {
-        const int resident = sms * per_sm;
-        parts = std::max(1, std::min({resident / nb, d / 16, 64}));
-    }
-    cudaGetLastError();
-    if (parts > 1)
-    {
-        e = cudaMemsetAsync(bars, 0, sizeof(unsigned) * nb, s);
-        if (e != cudaSuccess) return e;
-        int dd = d;
-        void *args[] = {&rho, &dd, &diag, &off, &parts, &pglob, &bars, &err, &dims};
-        e = cudaLaunchCooperativeKernel(reinterpret_cast<const void *>(&k_tridiag), dim3(nb * parts),
-                                        dim3(kTriThreads), args, smem, s);
+        // The smallest cluster whose shared memory holds the matrix (four CTAs
+        // for 256 rows, else one); more CTAs, down to 16 rows each, while SMs
+        // would stay idle.
+        int C = d > 128 ? 4 : 1;
+        while (C < 16 && nb * C * 2 <= sms && d / (2 * C) >= 16) C *= 2;
+        const double2 *r2 = reinterpret_cast<const double2 *>(rho);
+        e = d <= 32    ? launch_cluster<1, 32>(r2, d, nb, C, diag, off, s, dims)
+            : d == 64  ? launch_cluster<2, 128>(r2, d, nb, C, diag, off, s, dims)
+            : d == 128 ? launch_cluster<4, 256>(r2, d, nb, C, diag, off, s, dims)
+                       : launch_cluster<8, 256>(r2, d, nb, C, diag, off, s, dims);
     }
     else
     {
-        k_tridiag<<<nb, kTriThreads, smem, s>>>(reinterpret_cast<double2 *>(rho), d, diag, off, 1, nullptr, nullptr,
-                                                err, dims);
-        e = cudaGetLastError();
+        const std::size_t smem = 2 * sizeof(double2) * d;
+        e = cudaFuncSetAttribute(k_tridiag, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+        if (e != cudaSuccess) return e;
+        // Fewer matrices than SMs: spread each matrix over `parts` resident CTAs
+        // (cooperative launch), at least 16 trailing rows per CTA.
+        int per_sm = 0, parts = 1;
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_tridiag, kTriThreads, smem) == cudaSuccess &&
+            per_sm > 0)
+        {
+            const int resident = sms * per_sm;
+            parts = std::max(1, std::min({resident / nb, d / 16, 64}));
+        }
+        cudaGetLastError();
+        if (parts > 1)
+        {
+            e = cudaMemsetAsync(bars, 0, sizeof(unsigned) * nb, s);
+            if (e != cudaSuccess) return e;
+            int dd = d;
+            void *args[] = {&rho, &dd, &diag, &off, &parts, &pglob, &bars, &err, &dims};
+            e = cudaLaunchCooperativeKernel(reinterpret_cast<const void *>(&k_tridiag), dim3(nb * parts),
+                                            dim3(kTriThreads), args, smem, s);
+        }
+        else
+        {
+            k_tridiag<<<nb, kTriThreads, smem, s>>>(reinterpret_cast<double2 *>(rho), d, diag, off, 1, nullptr, nullptr,
+                                                    err, dims);
+            e = cudaGetLastError();
+        }
     }
     if (e != cudaSuccess) return e;
-    // One thread per matrix, spread over every SM: the QL sweep is a serial
-    // FP64 chain per matrix, so few threads per SM run it fastest.
-    const int sm_count = sms > 0 ? sms : 152;
-    const int tpb = std::max(1, std::min(32, (nb + sm_count - 1) / sm_count));
-    k_tridiag_ql<<<(nb + tpb - 1) / tpb, tpb, 0, s>>>(diag, off, d, nb, entropy_out, err, dims);
+    // One thread per eigenvalue: CTAs of up to 128, or of one warp each while
+    // that spreads a few matrices over idle SMs (two warps of one SM would
+    // share its FP64 pipe).
+    const int tpb = static_cast<long long>(nb) * ((d + 31) / 32) <= 2 * sms ? 32 : std::min(128, (d + 31) / 32 * 32);
+    const int chunks = (d + tpb - 1) / tpb;
+    const std::size_t sm = (sizeof(double2) + sizeof(float2)) * d;
+    e = cudaFuncSetAttribute(k_tridiag_sturm, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(sm));
+    if (e != cudaSuccess) return e;
+    // The terms take the place of the p vectors, which the reduction is done with.
+    double *terms = reinterpret_cast<double *>(pglob);
+    k_tridiag_sturm<<<dim3(nb, chunks), tpb, sm, s>>>(diag, off, d, terms, entropy_out, err, dims, eig_out != nullptr);
+    e = cudaGetLastError();
+    if (launched) *launched = chunks == 1 ? 2 : 3;
+    if (e != cudaSuccess || chunks == 1) return e;
+    k_entropy_sum<<<nb, 128, 0, s>>>(terms, d, entropy_out);
     return cudaGetLastError();
 }
 

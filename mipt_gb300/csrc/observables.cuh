@@ -93,19 +93,18 @@ cudaError_t jacobi_entropy(const double *rho, int d, int njobs, double *entropy_
                            cudaStream_t s);
 
 // Von Neumann entropies (bits) of Hermitian matrices rho[job][d][d]
-// (destroyed) for 2 <= d <= 4096: FP64 Householder tridiagonalisation (one
-// CTA per matrix, or, with fewer matrices than resident CTAs, several CTAs
-// per matrix in a cooperative launch), then implicit QL, one thread per
-// matrix (eigen.cu).
-// eig_out (nullable) receives each matrix's eigenvalues (unordered);
-// scratch holds hermitian_eig_scratch_doubles(d, njobs) doubles. A QL
-// iteration limit that runs out sets bit 1 of *err and writes NaN; a timed-out
-// barrier between the CTAs of one matrix sets bit 2.
+// (destroyed; d a power of two) for 2 <= d <= 4096: FP64 Householder
+// tridiagonalisation, then Sturm counts, one thread per eigenvalue (eigen.cu).
+// eig_out (nullable) receives each matrix's eigenvalues (ascending); scratch
+// holds hermitian_eig_scratch_doubles(d, njobs) doubles. A matrix that is not
+// finite sets bit 1 of *err and gives NaN; a timed-out barrier between the CTAs
+// of one matrix sets bit 2. launched (nullable) receives the kernel launches.
 // dims (nullable): the rows of each matrix that hold data (the rest of
-// its d x d block is zero); the reduction and QL then run on those only.
+// its d x d block is zero); the eigensolver then runs on those only.
 std::size_t hermitian_eig_scratch_doubles(int d, int njobs);
 cudaError_t hermitian_eig_entropy(double *rho, int d, int njobs, double *entropy_out, double *eig_out,
-                                  double *scratch, int *err, cudaStream_t s, const int *dims = nullptr);
+                                  double *scratch, int *err, cudaStream_t s, const int *dims = nullptr,
+                                  int *launched = nullptr);
 
 // Three-site RDMs of every trajectory, for `count` triples subs[3*i..].
 // out[traj][i][8][8] complex row-major. fermion selects the fermionic trace
