@@ -988,145 +988,238 @@ __global__ void __launch_bounds__(256) k_jacobi(const double *__restrict__ rho, 
 }
 
 // ------------------------------------------------------------- three sites
-constexpr int R3_THREADS = 256;
+constexpr int R3_THREADS = 128;
+constexpr int R3_RUN = 16;      // environment columns per FP32 run
+constexpr int R3_VALUES = 72;   // re, im of the 36 lower-triangle entries
+constexpr int R3_GROUPS = 8;    // chunk groups of the final sum
 
+// s + c += x with the addition's rounding error kept (Knuth's TwoSum).
+__device__ __forceinline__ void comp_add(float x, float &s, float &c)
+{
+    const float t = __fadd_rn(s, x);
+    const float z = __fsub_rn(t, s);
+    c = __fadd_rn(c, __fadd_rn(__fsub_rn(s, __fsub_rn(t, z)), __fsub_rn(x, z)));
+    s = t;
+}
+
+// One chunk of environment columns of one triple: each thread holds the
+// lower triangle of its columns' sum in registers. Sites that a pending
+// collapse measured keep their outcome, so only the matching columns are
+// visited; the scattered column counter advances by a masked increment.
+// FP32 states: sums of 16 columns in FP32 (packed FMAs) join a compensated
+// pair of FP32 numbers per value in shared memory, and the pairs are added
+// the same way over the threads: FP64 additions cost an SM 20 clocks a warp
+// (and FP32 -> FP64 conversions 17), so the former FP64 shuffle trees over 72
+// values per warp took most of the time. FP64 states: FP64 sums throughout.
+// Measured on GB300, 20 ring triples of an n = 20 FP32 state, the whole call:
+// 306 -> 88 us.
 template <typename Real>
 __global__ void __launch_bounds__(R3_THREADS)
     k_rho3(const Cx<Real> *__restrict__ states, int n, const int *__restrict__ subs, int fermion,
            const Collapse *__restrict__ col, std::size_t col_stride, int chunks, double *__restrict__ part)
 {
-    __shared__ std::uint64_t lo_tab[256];
-    __shared__ std::uint64_t off[8], cross[8];
-    __shared__ int isign[8];
-    __shared__ std::int8_t env[64];
-    __shared__ double red[R3_THREADS / 32][72];
-    const int tid = threadIdx.x;
+    constexpr bool kF32 = sizeof(Real) == 4;
+    // FP32: (sum, compensation) per value and thread; FP64: the value.
+    extern __shared__ __align__(16) double r3_smem[];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int tri = blockIdx.y, traj = blockIdx.z;
     const int q[3] = {subs[3 * tri], subs[3 * tri + 1], subs[3 * tri + 2]};
-    const int nenv = n - 3;
-    if (tid == 0)
-    {
-        int e = 0;
-        for (int b = 0; b < n; ++b)
-            if (b != q[0] && b != q[1] && b != q[2]) env[e++] = static_cast<std::int8_t>(b);
-    }
-    __syncthreads();
-    if (tid < 256)
-    {
-        const int nb = nenv < 8 ? nenv : 8;
-        std::uint64_t o = 0;
-        for (int b = 0; b < nb; ++b)
-            if ((tid >> b) & 1) o |= 1ull << env[b];
-        lo_tab[tid] = o;
-    }
-    if (tid < 8)
-    {
-        std::uint64_t o = 0, x = 0;
-        int par = 0;
-        for (int i = 0; i < 3; ++i)
-            if ((tid >> i) & 1)
-            {
-                o |= 1ull << q[i];
-                for (int b = 0; b < nenv; ++b)
-                    if (env[b] < q[i]) x ^= 1ull << b;
-                for (int j = i + 1; j < 3; ++j)
-                    if (((tid >> j) & 1) && q[i] > q[j]) par ^= 1;
-            }
-        off[tid] = o;
-        cross[tid] = fermion ? x : 0ull;
-        isign[tid] = (fermion && par) ? -1 : 1;
-    }
+    const std::uint64_t all = (1ull << n) - 1ull;
+    const std::uint64_t qmask = (1ull << q[0]) | (1ull << q[1]) | (1ull << q[2]);
     Collapse cl{0, 0, 1.0, 0};
     const bool has_col = col != nullptr;
     if (has_col) cl = col[traj * col_stride];
-    __syncthreads();
-
+    const std::uint64_t free_env = all & ~qmask & ~cl.mask, fixed = cl.value & ~qmask;
+    const int nfree = __popcll(free_env);
+    // Row offsets, their signs (bit r of neg), rows the collapse removes.
+    std::uint64_t off[8], cross[8];
+    unsigned neg = 0, gone = 0;
+#pragma unroll
+    for (int r = 0; r < 8; ++r)
+    {
+        std::uint64_t o = 0, x = 0;
+        int par = 0;
+#pragma unroll
+        for (int i = 0; i < 3; ++i)
+            if ((r >> i) & 1)
+            {
+                o |= 1ull << q[i];
+                x ^= all & ~qmask & ((1ull << q[i]) - 1ull);
+#pragma unroll
+                for (int j = i + 1; j < 3; ++j)
+                    if (((r >> j) & 1) && q[i] > q[j]) par ^= 1;
+            }
+        off[r] = o;
+        cross[r] = fermion ? x : 0ull;
+        if (fermion && par) neg |= 1u << r;
+        if (((o ^ cl.value) & cl.mask & qmask) != 0) gone |= 1u << r;
+    }
+    // Column e: the thread's index on the seven lowest free modes, a counter
+    // on the others.
+    std::uint64_t lo = fixed, rest = free_env;
+    bool inside = true;
+    for (int b = 0; b < 7; ++b)
+    {
+        const std::uint64_t bit = rest & (~rest + 1ull);
+        rest &= rest - (rest ? 1ull : 0ull);
+        if ((tid >> b) & 1)
+        {
+            lo |= bit;
+            inside = inside && bit != 0;
+        }
+    }
+    const std::uint64_t steps = nfree > 7 ? 1ull << (nfree - 7) : 1ull;
+    const std::uint64_t beg = steps * blockIdx.x / chunks, end = steps * (blockIdx.x + 1) / chunks;
+    std::uint64_t hi = 0;
+    {
+        std::uint64_t m = rest;
+        for (std::uint64_t c = beg; c != 0 && m != 0; c >>= 1)
+        {
+            if (c & 1ull) hi |= m & (~m + 1ull);
+            m &= m - 1ull;
+        }
+    }
     const Cx<Real> *psi = states + (static_cast<std::size_t>(traj) << n);
-    const std::uint64_t E = 1ull << nenv;
-    const std::uint64_t per = (E + chunks - 1) / chunks;
-    const std::uint64_t beg = blockIdx.x * per, end = beg + per < E ? beg + per : E;
+    const Real sc = static_cast<Real>(cl.scale);
     Real ar[36], ai[36];
 #pragma unroll
     for (int i = 0; i < 36; ++i) ar[i] = ai[i] = Real(0);
-    const Real sc = static_cast<Real>(cl.scale);
-    for (std::uint64_t e = beg + tid; e < end; e += R3_THREADS)
-    {
-        std::uint64_t hi = 0;
-        for (int b = 8; b < nenv; ++b)
-            if ((e >> b) & 1ull) hi |= 1ull << env[b];
-        const std::uint64_t eo = hi | lo_tab[e & 255];
-        Cx<Real> v[8];
-#pragma unroll
-        for (int r = 0; r < 8; ++r)
+    float2 *pairs = reinterpret_cast<float2 *>(r3_smem) + tid;
+    if constexpr (kF32)
+#pragma unroll 4
+        for (int t = 0; t < R3_VALUES; ++t) pairs[t * R3_THREADS] = make_float2(0.f, 0.f);
+    auto flush = [&]() {
+        if constexpr (kF32)
         {
-            const std::uint64_t a = eo | off[r];
-            Cx<Real> x = psi[a];
-            if (has_col)
+#pragma unroll
+            for (int t = 0; t < 36; ++t)
             {
-                if ((a & cl.mask) != cl.value)
-                    x = Cx<Real>{Real(0), Real(0)};
-                else
+                float2 x = pairs[(2 * t) * R3_THREADS], y = pairs[(2 * t + 1) * R3_THREADS];
+                comp_add(ar[t], x.x, x.y);
+                comp_add(ai[t], y.x, y.y);
+                pairs[(2 * t) * R3_THREADS] = x;
+                pairs[(2 * t + 1) * R3_THREADS] = y;
+                ar[t] = ai[t] = 0.f;
+            }
+        }
+    };
+    int run = 0;
+    if (inside)
+        for (std::uint64_t c = beg; c < end; ++c)
+        {
+            const std::uint64_t eo = lo | hi;
+            Cx<Real> v[8];
+#pragma unroll
+            for (int r = 0; r < 8; ++r) v[r] = psi[eo | off[r]];
+            hi = ((hi | ~rest) + 1ull) & rest;
+            if (has_col || fermion)
+            {
+#pragma unroll
+                for (int r = 0; r < 8; ++r)
                 {
-                    x.re *= sc;
-                    x.im *= sc;
+                    if (has_col)
+                        v[r] = (gone >> r) & 1u ? Cx<Real>{Real(0), Real(0)} : Cx<Real>{v[r].re * sc, v[r].im * sc};
+                    if (((__popcll(eo & cross[r]) & 1) ^ ((neg >> r) & 1u)) != 0) v[r] = Cx<Real>{-v[r].re, -v[r].im};
                 }
             }
-            const int sg = ((__popcll(e & cross[r]) & 1) ? -1 : 1) * isign[r];
-            if (sg < 0)
+            int t = 0;
+#pragma unroll
+            for (int r = 0; r < 8; ++r)
+#pragma unroll
+                for (int cc = 0; cc <= r; ++cc, ++t)
+                {
+                    if constexpr (kF32)
+                    {
+                        float2 acc = make_float2(ar[t], ai[t]);
+                        acc = __ffma2_rn(make_float2(v[r].re, v[r].im), make_float2(v[cc].re, v[cc].re), acc);
+                        acc = __ffma2_rn(make_float2(v[r].im, -v[r].re), make_float2(v[cc].im, v[cc].im), acc);
+                        ar[t] = acc.x;
+                        ai[t] = acc.y;
+                    }
+                    else
+                    {
+                        ar[t] = fma(v[r].re, v[cc].re, ar[t]);
+                        ar[t] = fma(v[r].im, v[cc].im, ar[t]);
+                        ai[t] = fma(v[r].im, v[cc].re, ai[t]);
+                        ai[t] = fma(-v[r].re, v[cc].im, ai[t]);
+                    }
+                }
+            if (kF32 && ++run == R3_RUN)
             {
-                x.re = -x.re;
-                x.im = -x.im;
+                flush();
+                run = 0;
             }
-            v[r] = x;
         }
-        int t = 0;
-#pragma unroll
-        for (int r = 0; r < 8; ++r)
-#pragma unroll
-            for (int c = 0; c <= r; ++c, ++t)
-            {
-                ar[t] = fma(v[r].re, v[c].re, ar[t]);
-                ar[t] = fma(v[r].im, v[c].im, ar[t]);
-                ai[t] = fma(v[r].im, v[c].re, ai[t]);
-                ai[t] = fma(-v[r].re, v[c].im, ai[t]);
-            }
-    }
-    const int warp = tid >> 5, lane = tid & 31;
-#pragma unroll
-    for (int t = 0; t < 36; ++t)
+    if constexpr (kF32)
     {
-        double x = static_cast<double>(ar[t]), y = static_cast<double>(ai[t]);
-        for (int o = 16; o > 0; o /= 2)
+        if (run > 0) flush();
+    }
+    else
+    {
+#pragma unroll
+        for (int t = 0; t < 36; ++t)
         {
-            x += __shfl_down_sync(0xffffffffu, x, o);
-            y += __shfl_down_sync(0xffffffffu, y, o);
-        }
-        if (lane == 0)
-        {
-            red[warp][2 * t] = x;
-            red[warp][2 * t + 1] = y;
+            r3_smem[(2 * t) * R3_THREADS + tid] = ar[t];
+            r3_smem[(2 * t + 1) * R3_THREADS + tid] = ai[t];
         }
     }
     __syncthreads();
-    if (tid < 72)
+    double *out = part + ((static_cast<std::size_t>(traj) * gridDim.y + tri) * chunks + blockIdx.x) * R3_VALUES;
+    for (int t = warp; t < R3_VALUES; t += R3_THREADS / 32)
     {
-        double s = 0.0;
-        for (int w = 0; w < R3_THREADS / 32; ++w) s += red[w][tid];
-        part[((static_cast<std::size_t>(traj) * gridDim.y + tri) * chunks + blockIdx.x) * 72 + tid] = s;
+        if constexpr (kF32)
+        {
+            const float2 *p = reinterpret_cast<const float2 *>(r3_smem) + t * R3_THREADS + lane;
+            float x = 0.f, e = 0.f;
+#pragma unroll
+            for (int i = 0; i < R3_THREADS / 32; ++i)
+            {
+                const float2 y = p[32 * i];
+                comp_add(y.x, x, e);
+                e += y.y;
+            }
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1)
+            {
+                const float y = __shfl_xor_sync(0xffffffffu, x, o), f = __shfl_xor_sync(0xffffffffu, e, o);
+                comp_add(y, x, e);
+                e += f;
+            }
+            if (lane == 0) out[t] = static_cast<double>(x) + static_cast<double>(e);
+        }
+        else
+        {
+            const double *p = r3_smem + t * R3_THREADS + lane;
+            double x = 0.0;
+#pragma unroll
+            for (int i = 0; i < R3_THREADS / 32; ++i) x += p[32 * i];
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+            if (lane == 0) out[t] = x;
+        }
     }
 }
 
-__global__ void k_rho3_finalize(const double *__restrict__ part, int chunks, int total_triples, double *__restrict__ out)
+// Sum over the chunks (eight interleaved groups, then the groups in order)
+// and the mirrored 8 x 8 block.
+__global__ void __launch_bounds__(R3_VALUES *R3_GROUPS)
+    k_rho3_finalize(const double *__restrict__ part, int chunks, int total_triples, double *__restrict__ out)
 {
+    __shared__ double red[R3_GROUPS][R3_VALUES];
     const int id = blockIdx.x;
     if (id >= total_triples) return;
+    const int v = threadIdx.x % R3_VALUES, g = threadIdx.x / R3_VALUES;
+    double x = 0.0;
+    for (int c = g; c < chunks; c += R3_GROUPS) x += part[(static_cast<std::size_t>(id) * chunks + c) * R3_VALUES + v];
+    red[g][v] = x;
+    __syncthreads();
     const int t = threadIdx.x;
     if (t >= 36) return;
     double sr = 0.0, si = 0.0;
-    for (int c = 0; c < chunks; ++c)
+    for (int i = 0; i < R3_GROUPS; ++i)
     {
-        sr += part[(static_cast<std::size_t>(id) * chunks + c) * 72 + 2 * t];
-        si += part[(static_cast<std::size_t>(id) * chunks + c) * 72 + 2 * t + 1];
+        sr += red[i][2 * t];
+        si += red[i][2 * t + 1];
     }
     int r = 0;
     while ((r + 1) * (r + 2) / 2 <= t) ++r;
@@ -1139,6 +1232,15 @@ __global__ void k_rho3_finalize(const double *__restrict__ part, int chunks, int
         o[(c * 8 + r) * 2] = sr;
         o[(c * 8 + r) * 2 + 1] = -si;
     }
+}
+
+// Chunks per triple: about three CTAs per SM over all triples, at least one
+// FP32 run (or 4 FP64 columns) per thread.
+int rho3_chunks(int n, long long triples, bool fp64)
+{
+    const std::uint64_t steps = n - 3 > 7 ? 1ull << (n - 10) : 1ull;
+    const std::uint64_t want = std::max<long long>(1, (3 * 152 + triples - 1) / triples);
+    return static_cast<int>(std::max<std::uint64_t>(1, std::min<std::uint64_t>(want, steps / (fp64 ? 4 : R3_RUN))));
 }
 
 int gram_splits(int n, int k, int njobs, bool rho)
@@ -1296,9 +1398,10 @@ cudaError_t jacobi_entropy(const double *rho, int d, int njobs, double *entropy_
 
 std::size_t rho3_scratch_bytes(int n, int batch, int count)
 {
-    const std::uint64_t E = 1ull << (n - 3);
-    int chunks = static_cast<int>(std::min<std::uint64_t>(std::max<std::uint64_t>(1, E / (R3_THREADS * 16)), 256));
-    return sizeof(double) * 72 * static_cast<std::size_t>(chunks) * count * batch;
+    // Enough for any smaller batch too: chunks * triples stays below the
+    // CTAs wanted plus the triples.
+    const std::size_t triples = static_cast<std::size_t>(count) * batch;
+    return sizeof(double) * R3_VALUES * std::min(3 * 152 + triples, triples * rho3_chunks(n, 1, true));
 }
 
 template <typename Real>
@@ -1307,15 +1410,19 @@ cudaError_t rho3_sweep(const Cx<Real> *states, int n, int batch, const int *d_su
                        std::size_t scratch_bytes, cudaStream_t s)
 {
     if (count <= 0 || batch <= 0) return cudaSuccess;
-    const std::uint64_t E = 1ull << (n - 3);
-    int chunks = static_cast<int>(std::min<std::uint64_t>(std::max<std::uint64_t>(1, E / (R3_THREADS * 16)), 256));
-    if (rho3_scratch_bytes(n, batch, count) > scratch_bytes) return cudaErrorInvalidValue;
-    dim3 grid(chunks, count, batch);
-    k_rho3<Real><<<grid, R3_THREADS, 0, s>>>(states, n, d_subs, fermion, collapse, collapse_stride, chunks,
-                                             static_cast<double *>(scratch));
-    cudaError_t e = cudaGetLastError();
+    const int chunks = rho3_chunks(n, static_cast<long long>(count) * batch, sizeof(Real) == 8);
+    if (sizeof(double) * R3_VALUES * static_cast<std::size_t>(chunks) * count * batch > scratch_bytes)
+        return cudaErrorInvalidValue;
+    constexpr int smem = sizeof(double) * R3_VALUES * R3_THREADS;
+    cudaError_t e = cudaFuncSetAttribute(k_rho3<Real>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return e;
-    k_rho3_finalize<<<count * batch, 64, 0, s>>>(static_cast<const double *>(scratch), chunks, count * batch, out);
+    dim3 grid(chunks, count, batch);
+    k_rho3<Real><<<grid, R3_THREADS, smem, s>>>(states, n, d_subs, fermion, collapse, collapse_stride, chunks,
+                                                static_cast<double *>(scratch));
+    e = cudaGetLastError();
+    if (e != cudaSuccess) return e;
+    k_rho3_finalize<<<count * batch, R3_VALUES * R3_GROUPS, 0, s>>>(static_cast<const double *>(scratch), chunks,
+                                                                    count * batch, out);
     return cudaGetLastError();
 }
 
