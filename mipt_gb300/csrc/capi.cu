@@ -1835,7 +1835,7 @@ int upload_draws(mipt_gb300_batch *b, const std::vector<TrajectoryDraw> &draws, 
             {
                 b->any_meas[t] = 1;
                 b->max_chunks[t] = std::max(b->max_chunks[t], M.nchunks);
-                const PassGeom &hg = fused_hist_geometry(plans[t % b->ncolour].back(), b->cfg.fp64 == 0);
+                const PassGeom &hg = plans[t % b->ncolour].back().geom;
                 const int ml = local_measured_count(hg, M.chunk[0]);
                 if ((std::size_t{1} << (hg.n_nl + ml)) > kHistScratch) b->fusable[t] = 0;
                 if (M.chunk[0] >> ne) b->fusable[t] = 0;
@@ -2243,7 +2243,7 @@ int batch_execute(mipt_gb300_batch *b, cudaStream_t s)
                     ++L;
                 }
                 Mark m(b, K_MEASURE, s);
-                MG_CUDA(launch_measure(count, ne, fused ? &fused_hist_geometry(plan.back(), sizeof(Real) == 4) : nullptr,
+                MG_CUDA(launch_measure(count, ne, fused ? &plan.back().geom : nullptr,
                                        b->kmax, b->cmin, ci, meas + t, T,
                                        b->part.as<double>(), b->bins.as<double>(),
                                        std::size_t{1} << b->cfg.chunk_bits, forced ? forced + t : nullptr, T,

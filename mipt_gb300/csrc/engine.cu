@@ -13,14 +13,12 @@
 #include "engine.cuh"
 
 #include <algorithm>
-#include <array>
 #include <atomic>
 #include <cmath>
 #include <cstdlib>
 #include <cstring>
 #include <stdexcept>
 
-#include <cooperative_groups.h>
 #include <cuda.h>
 #include <cudaTypedefs.h>
 
@@ -378,114 +376,6 @@ __device__ void value_histogram(const T *val, int k, const int *lm, int m_loc, d
     }
 }
 
-// Born histogram of an FP32 tile straight from the registers of the pass's
-// last round, in a fixed order. Squared magnitudes are folded over the
-// unmeasured register bits in registers (pairwise FP32 adds); every thread
-// then stores its 2^RB values to S[(warp * 2^RB + r) * L + lane] (L lanes per
-// warp; S needs 2^k floats), and the bins are summed from there: bin `bin`
-// collects the entries whose measured bits spell it, over all values of the
-// unmeasured lane and warp bits, G threads per bin each summing a fixed
-// slice and a shuffle tree joining the G partial sums. `mmask` is the measured
-// set in tile positions (bin bit i <-> i-th measured position from the
-// bottom); out[bin] as in value_histogram. Rounding: pairwise register folds
-// and shuffle trees plus sequential runs of at most 2^(TB - log2 G) terms in
-// FP32, within the reference's scheme of FP32 runs of 64
-// (cpp/include/mipt/cuda/reduce_sweep.cuh:59-96); the per-bin result is
-// widened to FP64.
-template <int RB>
-__device__ void register_histogram(const Cx<float> (&amp)[1 << RB], const Round &Z, int TB, std::uint32_t mmask,
-                                   int m_loc, float *S, int *tab, double *out)
-{
-    constexpr int NA = 1 << RB;
-    const int tid = threadIdx.x;
-    const int nl = TB < 5 ? TB : 5;
-    const int L = 1 << nl;
-    const unsigned lanes = TB >= 5 ? 0xffffffffu : ((1u << L) - 1u);
-    float p[NA];
-#pragma unroll
-    for (int r = 0; r < NA; ++r) p[r] = norm2(amp[r]);
-    unsigned um_reg = 0;
-#pragma unroll
-    for (int i = 0; i < RB; ++i)
-        if (!((mmask >> Z.reg[i]) & 1u)) um_reg |= 1u << i;
-#pragma unroll
-    for (int i = 0; i < RB; ++i)
-        if ((um_reg >> i) & 1u)
-        {
-#pragma unroll
-            for (int r = 0; r < NA; ++r)
-                if (!((r >> i) & 1)) p[r] += p[r | (1 << i)];
-        }
-    // tab[q], q < k: offset in S of tile position q; tab[16 + t]: offset of
-    // the t-th unmeasured thread bit; tab[31]: their count.
-    for (int q = tid; q < 16; q += blockDim.x)
-    {
-        int st = 0;
-        for (int j = 0; j < RB; ++j)
-            if (Z.reg[j] == q) st = (1 << j) * L;
-        for (int j = 0; j < TB; ++j)
-            if (Z.tid[j] == q) st = j < nl ? (1 << j) : (1 << (j - nl)) * NA * L;
-        tab[q] = st;
-    }
-    if (tid == 0)
-    {
-        int uc = 0;
-        for (int j = 0; j < TB; ++j)
-            if (!((mmask >> Z.tid[j]) & 1u)) tab[16 + uc++] = j < nl ? (1 << j) : (1 << (j - nl)) * NA * L;
-        tab[31] = uc;
-    }
-    __syncthreads(); // the tile buffer is free; tab is ready
-    {
-        float *row = S + (static_cast<std::size_t>((tid >> 5) * NA) << nl) + (tid & 31);
-#pragma unroll
-        for (int r = 0; r < NA; ++r) row[r << nl] = p[r];
-    }
-    __syncthreads();
-    const int uc = tab[31];
-    const int nbin = 1 << m_loc;
-    const int T = blockDim.x;
-    const int G = nbin >= T ? 1 : (T / nbin < 32 ? T / nbin : 32);
-    const int per = (1 << uc) / G > 0 ? (1 << uc) / G : 1;
-    for (int w = tid / G; w < nbin; w += T / G)
-    {
-        const int sub = tid % G;
-        int off = 0;
-        {
-            std::uint32_t mm = mmask;
-            for (int i = 0; i < m_loc; ++i)
-            {
-                const int q = __ffs(mm) - 1;
-                mm &= mm - 1u;
-                if ((w >> i) & 1) off += tab[q];
-            }
-        }
-        float s = 0.f;
-        // This lane's terms c0 .. c0 + cnt - 1 (cnt is 0 or `per`, a power of
-        // two). The offsets of the unmeasured bits are distinct powers of
-        // two, so the terms are visited in Gray-code order of their low bits:
-        // each step flips one bit of the offset.
-        const int c0 = sub * per;
-        const int cnt = (1 << uc) - c0 < per ? (1 << uc) - c0 : per;
-        if (cnt > 0)
-        {
-            int o = off;
-            for (int t = 0; t < uc; ++t)
-                if ((c0 >> t) & 1) o += tab[16 + t];
-            for (int i = 0;;)
-            {
-                s += S[o];
-                if (++i >= cnt) break;
-                o ^= tab[16 + __ffs(i) - 1];
-            }
-        }
-        for (int d = G >> 1; d > 0; d >>= 1) s += __shfl_down_sync(lanes, s, d, G);
-        if (sub == 0) out[w] = static_cast<double>(s);
-    }
-}
-
-// Position of tile bit p once tile bit x is removed (CTA-local offset).
-__device__ __forceinline__ int opos_d(int p, int x) { return p > x ? p - 1 : p; }
-
 // XOR swizzle of one local tile bit: bits >= 5 also flip low bit (p mod 5),
 // so any five lanes whose tile bits have distinct residues mod 5 touch
 // distinct shared-memory banks. Linear over GF(2): swz(a ^ b) = swz(a) ^ swz(b).
@@ -520,64 +410,6 @@ __device__ __forceinline__ void apply_slot(Cx<Real> (&a)[NA], const Cx<Real> *__
     }
 }
 
-
-// FP32 variant of apply_slot on Blackwell's packed FP32x2 FMA: for
-// acc += u * in, acc = fma2({u.re, u.re}, {in.re, in.im}, acc) then
-// acc = fma2({-u.im, u.im}, {in.im, in.re}, acc) -- two packed FMAs per
-// complex multiply-add instead of four scalar ones.
-template <int S, int NA>
-__device__ __forceinline__ void apply_slot_f2(Cx<float> (&a)[NA], const Cx<float> *__restrict__ Us)
-{
-    constexpr int lo = 2 * S;
-    float2 ur[16], ui[16];
-#pragma unroll
-    for (int e = 0; e < 16; ++e)
-    {
-        const Cx<float> u = Us[e];
-        ur[e] = make_float2(u.re, u.re);
-        ui[e] = make_float2(-u.im, u.im);
-    }
-#pragma unroll
-    for (int g = 0; g < NA / 4; ++g)
-    {
-        const int base = ((g >> lo) << (lo + 2)) | (g & ((1 << lo) - 1));
-        float2 in[4], sw[4];
-#pragma unroll
-        for (int c = 0; c < 4; ++c)
-        {
-            const Cx<float> v = a[base | (c << lo)];
-            in[c] = make_float2(v.re, v.im);
-            sw[c] = make_float2(v.im, v.re);
-        }
-#pragma unroll
-        for (int r = 0; r < 4; ++r)
-        {
-            float2 acc = __fmul2_rn(ur[4 * r], in[0]);
-            acc = __ffma2_rn(ui[4 * r], sw[0], acc);
-#pragma unroll
-            for (int c = 1; c < 4; ++c)
-            {
-                acc = __ffma2_rn(ur[4 * r + c], in[c], acc);
-                acc = __ffma2_rn(ui[4 * r + c], sw[c], acc);
-            }
-            a[base | (r << lo)] = Cx<float>{acc.x, acc.y};
-        }
-    }
-}
-
-template <int S, typename Real, int NA>
-__device__ __forceinline__ void apply_slot_fast(Cx<Real> (&a)[NA], const Cx<Real> *__restrict__ Us, bool packed)
-{
-    if constexpr (sizeof(Real) == 4)
-    {
-        if (packed)
-        {
-            apply_slot_f2<S>(a, Us);
-            return;
-        }
-    }
-    apply_slot<S>(a, Us);
-}
 
 // Parity-selected 2x2 gate on register bit 2S of a parity-sector state: the
 // pair (r, r | bit 2S) gets Us[0..3] when the parity of the element's other
@@ -647,23 +479,25 @@ __device__ __forceinline__ bool tile_bar_wait(std::uint64_t *bar, std::uint32_t 
     return false;
 }
 
-// One thread: fetches the tile whose first amplitude has batch-global index
-// gb (trajectory << n | tile base) into `tile` in plain tile order with one
-// TMA tensor load. Dimension d of the map covers global index bits [lo[d],
-// lo[d] + bits[d]) (the last one also the trajectory index above bit n); its
-// coordinate is those bits of gb, 0 on local runs.
-__device__ __forceinline__ void tile_tma_load(void *tile, const CUtensorMap *map, const TileTma &t, const PassGeom &g,
-                                              std::uint64_t gb, std::uint64_t *bar)
+// One thread: fetches half `half` (top tile bit) of the tile whose first
+// amplitude has batch-global index gb (trajectory << n | tile base), 2^box_bits
+// amplitudes, into `tile` with one TMA tensor load. Dimension d of the map
+// covers global index bits [lo[d], lo[d] + bits[d]) (the last one also the
+// trajectory index above bit n); its coordinate is those bits of gb, 0 on local
+// runs but for the half.
+__device__ __forceinline__ void tile_tma_load(void *tile, const CUtensorMap *map, const TileTma &t, int box_bits,
+                                              std::uint64_t gb, int half, std::uint64_t *bar)
 {
     int c[5] = {0, 0, 0, 0, 0};
     for (int d = 0; d < t.rank; ++d)
     {
         const std::uint64_t v = gb >> t.lo[d];
         c[d] = static_cast<int>(d + 1 == t.rank ? v : (v & ((1ull << t.bits[d]) - 1)));
+        if (half && d == t.half_dim) c[d] += 1 << (t.bits[d] - 1);
     }
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)),
-                 "r"(static_cast<std::uint32_t>(sizeof(Cx<float>) << g.k))
+                 "r"(static_cast<std::uint32_t>(sizeof(Cx<float>) << box_bits))
                  : "memory");
     const std::uint32_t dst = smem_u32(tile), mb = smem_u32(bar);
     const unsigned long long m = reinterpret_cast<unsigned long long>(map);
@@ -797,33 +631,22 @@ __device__ std::uint32_t build_item_prefix(std::uint32_t *pref, std::uint32_t *r
     return total;
 }
 
-// One tiled pass with register rounds: global -> registers (lanes on the
+// One FP64 tiled pass with register rounds: global -> registers (lanes on the
 // contiguous low qubits), gates applied in registers, swizzled shared-memory
 // transposes between rounds, registers -> global, optional fused histogram.
 // Work items are (trajectory, tile) pairs, item = trajectory * 2^n_nl + tile;
 // the CTA at flat index c runs items c, c + C, ... with C the number of CTAs,
 // so one launch shape serves both one item per CTA (C = items) and a
-// persistent grid. With TMA (FP32, persistent grid) tiles arrive by one TMA
-// tensor load each into the shared tile buffer in plain tile order: the load
-// of the CTA's next item is issued as soon as the current item's last
-// transpose has read the buffer, so it streams under the last gate round, the
-// stores and the histogram, whose values then use their own 2^k floats after
-// the tile buffer. A load wait that runs out sets bit 8 of *err and ends the
-// CTA.
-template <typename Real, int RB, bool TMA, bool PAR>
-__global__ void __launch_bounds__(RB == 5 && sizeof(Real) == 4 ? 512 : 256)
+// persistent grid.
+template <typename Real, int RB, bool PAR>
+__global__ void __launch_bounds__(256)
     k_pass_rounds(Cx<Real> *__restrict__ states, PassPlan P, const Cx<Real> *__restrict__ gates,
                   std::size_t gate_stride, const Collapse *__restrict__ col_in, std::size_t col_stride,
                   const LayerMeas *__restrict__ meas, std::size_t meas_stride, double *__restrict__ partials,
-                  int fuse_hist, int packed, int batch, const __grid_constant__ CUtensorMap tmap, TileTma tt,
-                  int *err, std::uint64_t col_keep, int col_scaled, int sparse, int withhold_first_load)
+                  int fuse_hist, int batch, std::uint64_t col_keep, int col_scaled, int sparse)
 {
     constexpr int NA = 1 << RB;
-    extern __shared__ __align__(128) unsigned char smem_dyn[];
-    // TMA tensor loads need a 128-byte aligned destination; the launch adds
-    // 128 bytes of dynamic shared memory for the shift.
-    unsigned char *smem_raw = smem_dyn;
-    if constexpr (TMA) smem_raw += (128u - (smem_u32(smem_dyn) & 127u)) & 127u;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
     Cx<Real> *tile = reinterpret_cast<Cx<Real> *>(smem_raw);
     __shared__ Cx<Real> U[kMaxPassGates][16];
     __shared__ double red[8];
@@ -836,41 +659,15 @@ __global__ void __launch_bounds__(RB == 5 && sizeof(Real) == 4 ? 512 : 256)
     std::uint64_t items = static_cast<std::uint64_t>(batch) << g.n_nl;
     if (sp_on)
     {
-        // The item prefix table follows the tile (and, with TMA, the
-        // histogram values) in dynamic shared memory.
+        // The item prefix table follows the tile in dynamic shared memory.
         __shared__ std::uint32_t sred[32];
-        std::uint32_t *pref = reinterpret_cast<std::uint32_t *>(
-            smem_raw + (sizeof(Cx<Real>) << g.k) + (TMA ? (sizeof(float) << g.k) : 0));
+        std::uint32_t *pref = reinterpret_cast<std::uint32_t *>(smem_raw + (sizeof(Cx<Real>) << g.k));
         for (int i = 0; i < g.n_nl; ++i) sp.nlq |= 1ull << g.nl[i];
         items = build_item_prefix(pref, sred, g, sp.nlq, col_in, col_stride, batch);
         sp.pref = pref;
     }
     const std::uint64_t step = static_cast<std::uint64_t>(gridDim.x) * gridDim.y;
     const std::uint64_t first = static_cast<std::uint64_t>(blockIdx.y) * gridDim.x + blockIdx.x;
-    __shared__ __align__(8) std::uint64_t tile_bar;
-    __shared__ int tile_fail;
-    std::uint32_t tile_phase = 0;
-    // Batch-global index of the first amplitude of an item's tile.
-    auto item_base = [&](std::uint64_t it) {
-        int bb;
-        std::uint64_t tt_;
-        decode_item(it, sp_on, sp, g, col_in, col_stride, batch, bb, tt_);
-        return (static_cast<std::uint64_t>(bb) << g.n) | scatter_bits(tt_, g.nl, g.n_nl);
-    };
-    if constexpr (TMA)
-    {
-        if (tid == 0)
-        {
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&tile_bar)) : "memory");
-            asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-            tile_fail = 0;
-        }
-        __syncthreads();
-        // withhold_first_load (a test hook): CTA 0 does not issue its first
-        // tile load, so its bounded wait runs out and the pass reports it.
-        const bool withhold = withhold_first_load != 0 && first == 0;
-        if (tid == 0 && first < items && !withhold) tile_tma_load(tile, &tmap, tt, g, item_base(first), &tile_bar);
-    }
     int cur_b = -1;
     for (std::uint64_t item = first; item < items; item += step)
     {
@@ -904,42 +701,7 @@ __global__ void __launch_bounds__(RB == 5 && sizeof(Real) == 4 ? 512 : 256)
         }
         const Real scale = static_cast<Real>(cl.scale);
 
-        const std::uint64_t next = item + step;
         Cx<Real> amp[NA];
-        if constexpr (TMA)
-        {
-            // This item's tile is in the tile buffer in plain tile order.
-            if (!tile_bar_wait(&tile_bar, tile_phase)) tile_fail = 1;
-            tile_phase ^= 1u;
-            const Round &R = P.round[0];
-            std::uint64_t gt = base;
-            std::uint32_t jt = 0;
-            for (int i = 0; i < TB; ++i)
-                if ((tid >> i) & 1)
-                {
-                    gt |= 1ull << g.pos[R.tid[i]];
-                    jt |= 1u << R.tid[i];
-                }
-            std::uint64_t gr[RB];
-            std::uint32_t jr[RB];
-#pragma unroll
-            for (int i = 0; i < RB; ++i)
-            {
-                gr[i] = 1ull << g.pos[R.reg[i]];
-                jr[i] = 1u << R.reg[i];
-            }
-#pragma unroll
-            for (int r = 0; r < NA; ++r)
-            {
-                std::uint32_t j = jt;
-#pragma unroll
-                for (int i = 0; i < RB; ++i)
-                    if ((r >> i) & 1) j |= jr[i];
-                amp[r] = tile[j];
-            }
-            if (has_col) apply_keep_bits(amp, collapse_keep_bits<RB, PAR>(gt, gr, cl), scale);
-        }
-        else
         {
             const Round &R = P.round[0];
             std::uint64_t gt = base;
@@ -959,21 +721,7 @@ __global__ void __launch_bounds__(RB == 5 && sizeof(Real) == 4 ? 512 : 256)
             }
             if (has_col) apply_keep_bits(amp, collapse_keep_bits<RB, PAR>(gt, gr, cl), scale);
         }
-        __syncthreads(); // gate matrices visible; round-0 reads of the tile buffer are done
-        if constexpr (TMA)
-        {
-            if (tile_fail)
-            {
-                if (tid == 0)
-                {
-                    atomicOr(err, 8);
-                    tile_bar_wait(&tile_bar, tile_phase ^ 1u); // let the load land before leaving
-                }
-                return;
-            }
-            if (P.rounds == 1 && next < items && tid == 0) tile_tma_load(tile, &tmap, tt, g, item_base(next), &tile_bar);
-        }
-
+        __syncthreads(); // gate matrices visible
         for (int ri = 0; ri < P.rounds; ++ri)
         {
             const Round &R = P.round[ri];
@@ -1014,14 +762,6 @@ __global__ void __launch_bounds__(RB == 5 && sizeof(Real) == 4 ? 512 : 256)
                         if ((r >> i) & 1) p ^= rb_[i];
                     amp[r] = tile[p];
                 }
-                if constexpr (TMA)
-                {
-                    if (ri == P.rounds - 1 && next < items)
-                    {
-                        __syncthreads(); // the last reads of the tile buffer for this item are done
-                        if (tid == 0) tile_tma_load(tile, &tmap, tt, g, item_base(next), &tile_bar);
-                    }
-                }
             }
             if constexpr (PAR)
             {
@@ -1030,28 +770,28 @@ __global__ void __launch_bounds__(RB == 5 && sizeof(Real) == 4 ? 512 : 256)
                     if (P.gates.kind[R.slot[0]])
                         apply_parity_slot<0>(amp, U[R.slot[0]], tpar);
                     else
-                        apply_slot_fast<0>(amp, U[R.slot[0]], packed != 0);
+                        apply_slot<0>(amp, U[R.slot[0]]);
                 }
                 if (RB >= 4 && R.slot[1] >= 0)
                 {
                     if (P.gates.kind[R.slot[1]])
                         apply_parity_slot<(RB >= 4 ? 1 : 0)>(amp, U[R.slot[1]], tpar);
                     else
-                        apply_slot_fast<(RB >= 4 ? 1 : 0)>(amp, U[R.slot[1]], packed != 0);
+                        apply_slot<(RB >= 4 ? 1 : 0)>(amp, U[R.slot[1]]);
                 }
                 if (RB >= 6 && R.slot[2] >= 0)
                 {
                     if (P.gates.kind[R.slot[2]])
                         apply_parity_slot<(RB >= 6 ? 2 : 0)>(amp, U[R.slot[2]], tpar);
                     else
-                        apply_slot_fast<(RB >= 6 ? 2 : 0)>(amp, U[R.slot[2]], packed != 0);
+                        apply_slot<(RB >= 6 ? 2 : 0)>(amp, U[R.slot[2]]);
                 }
             }
             else
             {
-                if (R.slot[0] >= 0) apply_slot_fast<0>(amp, U[R.slot[0]], packed != 0);
-                if (RB >= 4 && R.slot[1] >= 0) apply_slot_fast<(RB >= 4 ? 1 : 0)>(amp, U[R.slot[1]], packed != 0);
-                if (RB >= 6 && R.slot[2] >= 0) apply_slot_fast<(RB >= 6 ? 2 : 0)>(amp, U[R.slot[2]], packed != 0);
+                if (R.slot[0] >= 0) apply_slot<0>(amp, U[R.slot[0]]);
+                if (RB >= 4 && R.slot[1] >= 0) apply_slot<(RB >= 4 ? 1 : 0)>(amp, U[R.slot[1]]);
+                if (RB >= 6 && R.slot[2] >= 0) apply_slot<(RB >= 6 ? 2 : 0)>(amp, U[R.slot[2]]);
             }
         }
 
@@ -1077,22 +817,7 @@ __global__ void __launch_bounds__(RB == 5 && sizeof(Real) == 4 ? 512 : 256)
         if (fuse_hist)
         {
             const LayerMeas &M = meas[b * meas_stride];
-            if constexpr (sizeof(Real) == 4)
-            {
-                if (M.nchunks > 0)
-                {
-                    const std::uint64_t chunk = M.chunk[0];
-                    std::uint32_t mmask = 0;
-                    for (int i = 0; i < g.k; ++i)
-                        if ((chunk >> g.pos[i]) & 1ull) mmask |= 1u << i;
-                    const int m_loc = __popc(mmask);
-                    double *part = partials + static_cast<std::size_t>(b) * kHistScratch + (tix << m_loc);
-                    float *S = reinterpret_cast<float *>(smem_raw + (TMA ? (sizeof(Cx<float>) << g.k) : 0));
-                    __shared__ int tab[32];
-                    register_histogram<RB>(amp, Z, TB, mmask, m_loc, S, tab, part);
-                }
-            }
-            else if (M.nchunks > 0)
+            if (M.nchunks > 0)
             {
                 __syncthreads(); // the tile buffer is free
                 Real *val = reinterpret_cast<Real *>(smem_raw);
@@ -1122,195 +847,474 @@ __global__ void __launch_bounds__(RB == 5 && sizeof(Real) == 4 ? 512 : 256)
 }
 
 
-// One tiled pass of a 2^14-amplitude tile split across the two CTAs of a
-// thread-block cluster (tile bit x = CTA rank): 256 threads x 32 amplitudes
-// per CTA, 64 KB of shared memory and at most 128 registers per thread, so two
-// CTAs fit on an SM and the load, gate and store phases of different CTAs
-// overlap. Transposes go through distributed shared memory.
-template <int RB>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(1 << (13 - RB), 2)
-    k_pass_cluster(Cx<float> *__restrict__ states, PassPlan P, const Cx<float> *__restrict__ gates,
-                   std::size_t gate_stride, const Collapse *__restrict__ col_in, std::size_t col_stride,
-                   const LayerMeas *__restrict__ meas, std::size_t meas_stride, double *__restrict__ partials,
-                   int fuse_hist)
+// Shared-memory place of one tile bit of k_pass_quads' tile: the 128-byte
+// swizzle of the TMA loads, which flips the 16-byte chunk index (tile bits 1..3)
+// by tile bits 4..6. Linear over GF(2): place(a ^ b) = place(a) ^ place(b).
+__host__ __device__ __forceinline__ std::uint32_t quad_place(int p)
 {
-    constexpr int NA = 1 << RB, TB = 13 - RB;
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    Cx<float> *tile = reinterpret_cast<Cx<float> *>(smem_raw);
-    __shared__ Cx<float> U[kMaxPassGates][16];
-    __shared__ double red[8];
-    namespace cg = cooperative_groups;
-    cg::cluster_group cluster = cg::this_cluster();
-    const unsigned rank = cluster.block_rank();
-    Cx<float> *peer = cluster.map_shared_rank(tile, static_cast<int>(rank ^ 1u));
+    return (1u << p) ^ (p >= 4 && p <= 6 ? 1u << (p - 3) : 0u);
+}
 
-    const PassGeom &g = P.geom;
-    const int tid = threadIdx.x;
-    const int b = blockIdx.y;
-    const std::uint64_t tix = blockIdx.x >> 1;
-    Cx<float> *psi = states + (static_cast<std::size_t>(b) << g.n);
-    const std::uint64_t base = scatter_bits(tix, g.nl, g.n_nl);
-    for (int i = tid; i < P.gates.count * 16; i += blockDim.x)
-        U[i / 16][i % 16] = gates[b * gate_stride + static_cast<std::size_t>(P.gates.gate[i / 16]) * 16 + (i % 16)];
-    Collapse cl{0, 0, 1.0, 0};
-    const bool has_col = col_in != nullptr;
-    if (has_col) cl = col_in[b * col_stride];
-    const float scale = static_cast<float>(cl.scale);
-
-    // n <= 32: every amplitude index fits in 32 bits.
-    const std::uint32_t cmask = static_cast<std::uint32_t>(cl.mask), cval = static_cast<std::uint32_t>(cl.value);
-    Cx<float> amp[NA];
+// A 4x4 gate on register-index bits (2S, 2S+1) of 16 amplitudes; U[e] holds
+// {re, re, -im, im} of matrix entry e (two packed FMAs per complex product).
+template <int S> __device__ __forceinline__ void apply_quad(Cx<float> (&a)[16], const float4 *__restrict__ U)
+{
+    constexpr int lo = 2 * S;
+    float2 ur[16], ui[16];
+#pragma unroll
+    for (int e = 0; e < 16; ++e)
     {
-        const ClusterRound &R = P.cround[0];
-        std::uint32_t gt = static_cast<std::uint32_t>(base) | (rank << g.pos[R.x]);
-        for (int i = 0; i < TB; ++i)
-            if ((tid >> i) & 1) gt |= 1u << g.pos[R.tid[i]];
-        std::uint32_t gr[RB];
-#pragma unroll
-        for (int i = 0; i < RB; ++i) gr[i] = 1u << g.pos[R.reg[i]];
-#pragma unroll
-        for (int r = 0; r < NA; ++r)
-        {
-            std::uint32_t gi = gt;
-#pragma unroll
-            for (int i = 0; i < RB; ++i)
-                if ((r >> i) & 1) gi |= gr[i];
-            Cx<float> v = psi[gi];
-            if (has_col)
-            {
-                const float f = ((gi & cmask) == cval) ? scale : 0.f;
-                v.re *= f;
-                v.im *= f;
-            }
-            amp[r] = v;
-        }
+        const float4 u = U[e];
+        ur[e] = make_float2(u.x, u.y);
+        ui[e] = make_float2(u.z, u.w);
     }
-    __syncthreads();
-
-    for (int ri = 0; ri < P.cluster_rounds; ++ri)
+#pragma unroll
+    for (int g = 0; g < 4; ++g)
     {
-        const ClusterRound &R = P.cround[ri];
-        if (ri > 0)
+        const int base = ((g >> lo) << (lo + 2)) | (g & ((1 << lo) - 1));
+        float2 in[4], sw[4];
+#pragma unroll
+        for (int c = 0; c < 4; ++c)
         {
-            const ClusterRound &A = P.cround[ri - 1];
-            const int xa = A.x;
-            // write: my elements have bit xa == rank, so they are all home here
-            std::uint32_t sa = 0;
-            for (int i = 0; i < TB; ++i)
-                if ((tid >> i) & 1) sa ^= swz1(opos_d(A.tid[i], xa));
-            std::uint32_t ra[RB];
-#pragma unroll
-            for (int i = 0; i < RB; ++i) ra[i] = swz1(opos_d(A.reg[i], xa));
-            if (ri > 1) cluster.sync(); // the peer has finished reading my buffer
-#pragma unroll
-            for (int r = 0; r < NA; ++r)
-            {
-                std::uint32_t p = sa;
-#pragma unroll
-                for (int i = 0; i < RB; ++i)
-                    if ((r >> i) & 1) p ^= ra[i];
-                tile[p] = amp[r];
-            }
-            cluster.sync();
-            // read in the storage coordinates of round A; home CTA = bit xa
-            std::uint32_t sb = 0;
-            unsigned hb = 0;
-            for (int i = 0; i < TB; ++i)
-                if ((tid >> i) & 1)
-                {
-                    if (R.tid[i] == xa)
-                        hb ^= 1u;
-                    else
-                        sb ^= swz1(opos_d(R.tid[i], xa));
-                }
-            if (rank)
-            {
-                if (R.x == xa)
-                    hb ^= 1u;
-                else
-                    sb ^= swz1(opos_d(R.x, xa));
-            }
-            std::uint32_t rbv[RB];
-            unsigned rh[RB];
-#pragma unroll
-            for (int i = 0; i < RB; ++i)
-            {
-                rh[i] = R.reg[i] == xa ? 1u : 0u;
-                rbv[i] = R.reg[i] == xa ? 0u : swz1(opos_d(R.reg[i], xa));
-            }
-#pragma unroll
-            for (int r = 0; r < NA; ++r)
-            {
-                std::uint32_t p = sb;
-                unsigned h = hb;
-#pragma unroll
-                for (int i = 0; i < RB; ++i)
-                    if ((r >> i) & 1)
-                    {
-                        p ^= rbv[i];
-                        h ^= rh[i];
-                    }
-                amp[r] = (h == rank) ? tile[p] : peer[p];
-            }
+            const Cx<float> v = a[base | (c << lo)];
+            in[c] = make_float2(v.re, v.im);
+            sw[c] = make_float2(v.im, v.re);
         }
-        if (R.slot[0] >= 0) apply_slot<0>(amp, U[R.slot[0]]);
-        if (R.slot[1] >= 0) apply_slot<1>(amp, U[R.slot[1]]);
-        if (RB >= 6 && R.slot[2] >= 0) apply_slot<(RB >= 6 ? 2 : 0)>(amp, U[R.slot[2]]);
-    }
-
-    const ClusterRound &Z = P.cround[P.cluster_rounds - 1];
-    {
-        std::uint32_t gt = static_cast<std::uint32_t>(base) | (rank << g.pos[Z.x]);
-        for (int i = 0; i < TB; ++i)
-            if ((tid >> i) & 1) gt |= 1u << g.pos[Z.tid[i]];
-        std::uint32_t gr[RB];
 #pragma unroll
-        for (int i = 0; i < RB; ++i) gr[i] = 1u << g.pos[Z.reg[i]];
-#pragma unroll
-        for (int r = 0; r < NA; ++r)
+        for (int r = 0; r < 4; ++r)
         {
-            std::uint32_t gi = gt;
+            float2 acc = __fmul2_rn(ur[4 * r], in[0]);
+            acc = __ffma2_rn(ui[4 * r], sw[0], acc);
 #pragma unroll
-            for (int i = 0; i < RB; ++i)
-                if ((r >> i) & 1) gi |= gr[i];
-            psi[gi] = amp[r];
-        }
-    }
-
-    // The peer may still read my buffer for the last transpose.
-    if (P.cluster_rounds > 1) cluster.sync();
-    if (fuse_hist)
-    {
-        const LayerMeas &M = meas[b * meas_stride];
-        if (M.nchunks > 0)
-        {
-            float *val = reinterpret_cast<float *>(smem_raw);
-            const int xz = Z.x;
-            std::uint32_t jt = 0;
-            for (int i = 0; i < TB; ++i)
-                if ((tid >> i) & 1) jt |= 1u << opos_d(Z.tid[i], xz);
-#pragma unroll
-            for (int r = 0; r < NA; ++r)
+            for (int c = 1; c < 4; ++c)
             {
-                std::uint32_t j = jt;
-#pragma unroll
-                for (int i = 0; i < RB; ++i)
-                    if ((r >> i) & 1) j |= 1u << opos_d(Z.reg[i], xz);
-                val[j] = norm2(amp[r]);
+                acc = __ffma2_rn(ur[4 * r + c], in[c], acc);
+                acc = __ffma2_rn(ui[4 * r + c], sw[c], acc);
             }
-            __syncthreads();
-            const std::uint64_t chunk = M.chunk[0];
-            const PassGeom &h = P.hgeom;
-            int lm[kMaxLocal + 1];
-            int m_loc = 0;
-            for (int i = 0; i < h.k; ++i)
-                if ((chunk >> h.pos[i]) & 1ull) lm[m_loc++] = i;
-            const std::uint64_t t2 = (tix << 1) | rank;
-            double *part = partials + static_cast<std::size_t>(b) * kHistScratch + (t2 << m_loc);
-            value_histogram(val, h.k, lm, m_loc, part, red);
+            a[base | (r << lo)] = Cx<float>{acc.x, acc.y};
         }
     }
 }
+
+// The parity-selected 2x2 gate of apply_parity_slot on 16 amplitudes.
+template <int S> __device__ __forceinline__ void apply_quad_parity(Cx<float> (&a)[16], const float4 *__restrict__ U, int tpar)
+{
+    Cx<float> us[8];
+#pragma unroll
+    for (int e = 0; e < 8; ++e) us[e] = Cx<float>{U[e].x, U[e].w};
+    apply_parity_slot<S>(a, us, tpar);
+}
+
+// FP32 tiled pass in rounds of two bonds on 16 amplitudes. The tile of 2^k
+// amplitudes stays in shared memory: in a round every thread takes two groups
+// of 16 amplitudes in turn (virtual thread index tid + 2^(k-5) * group),
+// applies up to two gates and writes them back in place, with one barrier
+// between rounds; the last round stores to global memory. Work items and the
+// persistent grid are those of k_pass_rounds.
+// What bounds it: packed FMAs issue at half the rate of scalar ones, so a
+// bond's 16 FMAs per amplitude take 2,048 clocks of a 2^14 tile, and a round
+// moves 256 KB through shared memory (2,048 clocks) beside the gate matrices'
+// broadcasts; the barriers keep the two from overlapping fully. Sixteen warps
+// of at most 128 registers hide the latencies better than eight: 64 amplitudes
+// and 255 registers per thread with three bonds per round (the kernel this
+// replaces) took 282 ms for the 96 launches of 32 L = 24 trajectories, this
+// 249 ms; 256 threads that read the next group ahead and keep the matrices in
+// registers took 270 ms.
+// With TMA the tile arrives as two half tiles (tile bit k-1), each with its own
+// barrier and in the 128-byte swizzle that keeps the rounds' accesses free of
+// bank conflicts (except when a round holds tile bit 0 in registers). Where the
+// first and the last round keep bit k-1 as the group bit (split), the next
+// item's first half is loaded as soon as the last round has read group 0, the
+// second half after group 1, under the last round's gates, stores and
+// histogram. A load wait that runs out sets bit 8 of *err and ends the CTA.
+// The Born histogram is folded over unmeasured register bits in registers, the
+// rest is summed from shared memory in a fixed order: FP32 pairwise sums and
+// runs of at most 32 terms, widened to FP64.
+template <bool TMA, bool PAR>
+__global__ void __launch_bounds__(512, 1)
+    k_pass_quads(Cx<float> *__restrict__ states, const __grid_constant__ PassPlan P,
+                 const Cx<float> *__restrict__ gates, std::size_t gate_stride, const Collapse *__restrict__ col_in,
+                 std::size_t col_stride, const LayerMeas *__restrict__ meas, std::size_t meas_stride,
+                 double *__restrict__ partials, int fuse_hist, int batch, const __grid_constant__ CUtensorMap tmap,
+                 const __grid_constant__ TileTma tt, int *err, std::uint64_t col_keep, int col_scaled, int sparse,
+                 int withhold_first_load)
+{
+    // The swizzle pattern repeats every 1024 bytes.
+    extern __shared__ __align__(1024) unsigned char smem_quads[];
+    unsigned char *smem_raw = smem_quads;
+    const PassGeom &g = P.geom;
+    const int k = g.k, TB = k - 4, nt = blockDim.x, tid = threadIdx.x;
+    Cx<float> *tile = reinterpret_cast<Cx<float> *>(smem_raw);
+    float *S = reinterpret_cast<float *>(smem_raw + (sizeof(Cx<float>) << k));
+    std::uint32_t *s_off = reinterpret_cast<std::uint32_t *>(S + (std::size_t{1} << k)); // [rounds][nt]
+    std::uint32_t *pref = s_off + P.rounds * nt;
+    __shared__ float4 U[kMaxPassGates][16];
+    __shared__ __align__(8) std::uint64_t bar[2];
+    __shared__ std::uint64_t s_tix;
+    __shared__ int tile_fail, tab[32], s_b;
+    __shared__ float red[16];
+
+    const bool sp_on = sparse != 0;
+    ItemSpace sp{nullptr, 0};
+    std::uint64_t items = static_cast<std::uint64_t>(batch) << g.n_nl;
+    if (sp_on)
+    {
+        __shared__ std::uint32_t sred[32];
+        for (int i = 0; i < g.n_nl; ++i) sp.nlq |= 1ull << g.nl[i];
+        items = build_item_prefix(pref, sred, g, sp.nlq, col_in, col_stride, batch);
+        sp.pref = pref;
+    }
+    const std::uint64_t step = static_cast<std::uint64_t>(gridDim.x) * gridDim.y;
+    const std::uint64_t first_item = static_cast<std::uint64_t>(blockIdx.y) * gridDim.x + blockIdx.x;
+    // This thread's shared-memory place in each round (group 0) and its global
+    // offsets in the first and last.
+    for (int ri = 0; ri < P.rounds; ++ri)
+    {
+        std::uint32_t o = 0;
+        for (int i = 0; i + 1 < TB; ++i)
+            if ((tid >> i) & 1) o ^= quad_place(P.round[ri].tid[i]);
+        s_off[ri * nt + tid] = o * 8;
+    }
+    const Round &Z = P.round[P.rounds - 1];
+    std::uint32_t g_first = 0, g_last = 0;
+    for (int i = 0; i + 1 < TB; ++i)
+        if ((tid >> i) & 1)
+        {
+            g_first |= 1u << g.pos[P.round[0].tid[i]];
+            g_last |= 1u << g.pos[Z.tid[i]];
+        }
+    // Thread 0: decodes an item for everyone and, with TMA, loads the halves
+    // of its tile whose bits are set in `halves`.
+    auto fetch_item = [&](std::uint64_t it, int halves) {
+        int bb;
+        std::uint64_t tx;
+        decode_item(it, sp_on, sp, g, col_in, col_stride, batch, bb, tx);
+        s_b = bb;
+        s_tix = tx;
+        if constexpr (TMA)
+        {
+            const std::uint64_t gb = (static_cast<std::uint64_t>(bb) << g.n) | scatter_bits(tx, g.nl, g.n_nl);
+            for (int h = 0; h < 2; ++h)
+                if ((halves >> h) & 1)
+                    tile_tma_load(tile + (static_cast<std::size_t>(h) << (k - 1)), &tmap, tt, k - 1, gb, h, &bar[h]);
+        }
+    };
+    std::uint32_t phase = 0;
+    if (tid == 0)
+    {
+        if constexpr (TMA)
+        {
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&bar[0])) : "memory");
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&bar[1])) : "memory");
+            asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        }
+        tile_fail = 0;
+        // withhold_first_load (a test hook): CTA 0 does not issue its first
+        // tile load, so its bounded wait runs out and the pass reports it.
+        if (first_item < items) fetch_item(first_item, withhold_first_load != 0 && first_item == 0 ? 0 : 3);
+    }
+    int b = -1, m_loc = 0;
+    bool hist = false;
+    std::uint32_t mmask = 0;
+    const bool has_col = col_in != nullptr;
+    Collapse cl{0, 0, 1.0, 0};
+    // The collapse over round 0's thread bits (mask, value) and register bits.
+    std::uint32_t c_mask = 0, c_value = 0, c_keep = 0xffffu;
+    float scale = 1.f;
+    for (std::uint64_t item = first_item; item < items; item += step)
+    {
+        __syncthreads(); // the item is decoded; the previous one's shared-memory reads are complete
+        const std::uint64_t tix = s_tix;
+        const std::uint32_t base = static_cast<std::uint32_t>(scatter_bits(tix, g.nl, g.n_nl));
+        if (s_b != b)
+        {
+            b = s_b;
+            for (int i = tid; i < P.gates.count * 16; i += nt)
+            {
+                const Cx<float> u =
+                    gates[b * gate_stride + static_cast<std::size_t>(P.gates.gate[i / 16]) * 16 + (i % 16)];
+                U[i / 16][i % 16] = make_float4(u.re, u.re, -u.im, u.im);
+            }
+            if (has_col)
+            {
+                // col_keep < all ones: the residual of a collapse that an earlier
+                // pass of the layer applied to every tile it visited; only the
+                // bits of the tiles it skipped are left. A parity condition is not
+                // (that pass's gates may have changed the stored bits' parity).
+                cl = col_in[b * col_stride];
+                cl.mask &= col_keep;
+                cl.value &= col_keep;
+                if (!col_scaled)
+                {
+                    cl.scale = 1.0;
+                    cl.parity = 0;
+                }
+                std::uint32_t rpos = 0;
+                c_keep = 0xffffu;
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+                {
+                    const std::uint32_t bit = 1u << g.pos[P.round[0].reg[i]];
+                    rpos |= bit;
+                    const std::uint32_t pat = static_cast<std::uint32_t>(reg_bit_pattern(i)) & 0xffffu;
+                    if (cl.mask & bit) c_keep &= (cl.value & bit) ? pat : ~pat;
+                }
+                c_mask = static_cast<std::uint32_t>(cl.mask) & ~rpos;
+                c_value = static_cast<std::uint32_t>(cl.value) & c_mask;
+                scale = static_cast<float>(cl.scale);
+            }
+            if (fuse_hist)
+            {
+                const LayerMeas &M = meas[b * meas_stride];
+                hist = M.nchunks > 0;
+                const std::uint64_t chunk = hist ? M.chunk[0] : 0ull;
+                mmask = 0;
+                for (int i = 0; i < k; ++i)
+                    if ((chunk >> g.pos[i]) & 1ull) mmask |= 1u << i;
+                m_loc = __popc(mmask);
+                // Virtual thread t keeps value r at S[((t / 32) * 16 + r) * 32 + t % 32].
+                // tab[q], q < k: offset in S of tile position q; tab[16 + t]:
+                // offset of the t-th unmeasured thread bit; tab[31]: their count.
+                if (tid < 16)
+                {
+                    int st = 0;
+                    for (int j = 0; j < 4; ++j)
+                        if (Z.reg[j] == tid) st = 32 << j;
+                    for (int j = 0; j < TB; ++j)
+                        if (Z.tid[j] == tid) st = j < 5 ? 1 << j : 512 << (j - 5);
+                    tab[tid] = st;
+                }
+                if (tid == 0)
+                {
+                    int uc = 0;
+                    for (int j = 0; j < TB; ++j)
+                        if (!((mmask >> Z.tid[j]) & 1u)) tab[16 + uc++] = j < 5 ? 1 << j : 512 << (j - 5);
+                    tab[31] = uc;
+                }
+            }
+            __syncthreads(); // gate matrices and the histogram table are visible
+        }
+        Cx<float> *psi = states + (static_cast<std::size_t>(b) << g.n);
+        const std::uint64_t next = item + step;
+
+#pragma unroll 1
+        for (int ri = 0; ri < P.rounds; ++ri)
+        {
+            const Round &R = P.round[ri];
+            const bool first = ri == 0, last = ri + 1 == P.rounds;
+            if (!first) __syncthreads(); // the previous round's writes are visible
+            const std::uint32_t so0 = s_off[ri * nt + tid];
+            const std::uint32_t gt0 = base | (first ? g_first : g_last);
+            std::uint32_t ra[4], gr[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+            {
+                ra[i] = quad_place(R.reg[i]) * 8;
+                gr[i] = 1u << g.pos[R.reg[i]];
+            }
+            const int gbit = R.tid[TB - 1];
+            auto place_of = [&](int grp) { return grp ? so0 ^ quad_place(gbit) * 8 : so0; };
+            auto index_of = [&](int grp) { return grp ? gt0 | 1u << g.pos[gbit] : gt0; };
+            auto read = [&](Cx<float>(&a)[16], int grp) {
+                if (TMA || !first)
+                {
+                    if (TMA && first && (grp == 0 || P.split))
+                    {
+                        bool ok = tile_fail == 0 && tile_bar_wait(&bar[grp], phase);
+                        if (!P.split) ok = ok && tile_bar_wait(&bar[1], phase);
+                        if (!ok) tile_fail = 1;
+                    }
+                    const std::uint32_t so = place_of(grp);
+#pragma unroll
+                    for (int r = 0; r < 16; ++r)
+                    {
+                        std::uint32_t p = so;
+#pragma unroll
+                        for (int i = 0; i < 4; ++i)
+                            if ((r >> i) & 1) p ^= ra[i];
+                        a[r] = *reinterpret_cast<const Cx<float> *>(smem_raw + p);
+                    }
+                }
+                else
+                {
+                    const Cx<float> *src = psi + index_of(grp);
+#pragma unroll
+                    for (int r = 0; r < 16; ++r)
+                    {
+                        std::uint32_t p = 0;
+#pragma unroll
+                        for (int i = 0; i < 4; ++i)
+                            if ((r >> i) & 1) p |= gr[i];
+                        a[r] = src[p];
+                    }
+                }
+            };
+            const int sl0 = R.slot[0], sl1 = R.slot[1];
+            auto process = [&](Cx<float>(&a)[16], int grp) {
+                if (first && has_col)
+                {
+                    if (PAR && cl.parity != 0)
+                    {
+                        const std::uint64_t g64[4] = {gr[0], gr[1], gr[2], gr[3]};
+                        apply_keep_bits(a, collapse_keep_bits<4, PAR>(index_of(grp), g64, cl), scale);
+                    }
+                    else
+                    {
+                        const std::uint32_t keep = ((index_of(grp) ^ c_value) & c_mask) == 0 ? c_keep : 0u;
+#pragma unroll
+                        for (int r = 0; r < 16; ++r)
+                            a[r] = (keep >> r) & 1u ? Cx<float>{a[r].re * scale, a[r].im * scale} : Cx<float>{0.f, 0.f};
+                    }
+                }
+                const int tpar =
+                    PAR ? (__popc(base) + __popc(static_cast<unsigned>(tid)) + __popc(static_cast<unsigned>(grp))) & 1 : 0;
+                if (sl0 >= 0)
+                {
+                    if (PAR && P.gates.kind[sl0])
+                        apply_quad_parity<0>(a, U[sl0], tpar);
+                    else
+                        apply_quad<0>(a, U[sl0]);
+                }
+                if (sl1 >= 0)
+                {
+                    if (PAR && P.gates.kind[sl1])
+                        apply_quad_parity<1>(a, U[sl1], tpar);
+                    else
+                        apply_quad<1>(a, U[sl1]);
+                }
+                if (!last)
+                {
+                    const std::uint32_t so = place_of(grp);
+#pragma unroll
+                    for (int r = 0; r < 16; ++r)
+                    {
+                        std::uint32_t p = so;
+#pragma unroll
+                        for (int i = 0; i < 4; ++i)
+                            if ((r >> i) & 1) p ^= ra[i];
+                        *reinterpret_cast<Cx<float> *>(smem_raw + p) = a[r];
+                    }
+                    return;
+                }
+                Cx<float> *dst = psi + index_of(grp);
+#pragma unroll
+                for (int r = 0; r < 16; ++r)
+                {
+                    std::uint32_t p = 0;
+#pragma unroll
+                    for (int i = 0; i < 4; ++i)
+                        if ((r >> i) & 1) p |= gr[i];
+                    dst[p] = a[r];
+                }
+                if (hist)
+                {
+                    float w[16];
+#pragma unroll
+                    for (int r = 0; r < 16; ++r) w[r] = norm2(a[r]);
+#pragma unroll
+                    for (int i = 0; i < 4; ++i)
+                        if (!((mmask >> R.reg[i]) & 1u))
+                        {
+#pragma unroll
+                            for (int r = 0; r < 16; ++r)
+                                if (!((r >> i) & 1)) w[r] += w[r | (1 << i)];
+                        }
+                    float *row = S + (((tid >> 5) + grp * (nt >> 5)) << 9) + (tid & 31);
+#pragma unroll
+                    for (int r = 0; r < 16; ++r) row[r << 5] = w[r];
+                }
+            };
+#pragma unroll 1
+            for (int grp = 0; grp < 2; ++grp)
+            {
+                Cx<float> a[16];
+                read(a, grp);
+                if (last)
+                {
+                    // This group is read: its half of the tile (all of it after
+                    // group 1) may take the next item's amplitudes.
+                    __syncthreads();
+                    if constexpr (TMA)
+                    {
+                        if (tile_fail)
+                        {
+                            if (tid == 0)
+                            {
+                                atomicOr(err, 8);
+                                // Let loads in flight land before leaving.
+                                tile_bar_wait(&bar[0], phase);
+                                tile_bar_wait(&bar[1], phase);
+                            }
+                            return;
+                        }
+                    }
+                    if (tid == 0 && next < items)
+                    {
+                        if (grp == 0 && P.split) fetch_item(next, 1);
+                        if (grp == 1) fetch_item(next, P.split ? 2 : 3);
+                    }
+                }
+                process(a, grp);
+            }
+        }
+        phase ^= 1u;
+        if (hist)
+        {
+            __syncthreads();
+            // Bin w collects the entries whose measured bits spell it: sums over
+            // the unmeasured thread bits, 2^g_log threads per bin, a shuffle tree
+            // in each warp and, for bins of several warps, their totals in order.
+            const int uc = tab[31];
+            int g_log = (31 - __clz(nt)) - m_loc;
+            g_log = g_log < 0 ? 0 : (g_log > uc ? uc : g_log);
+            const int per_log = uc - g_log, w_log = g_log < 5 ? g_log : 5;
+            double *out = partials + static_cast<std::size_t>(b) * kHistScratch + (tix << m_loc);
+            for (int w = tid >> g_log; w < (1 << m_loc); w += nt >> g_log)
+            {
+                int o = 0;
+                std::uint32_t mm = mmask;
+                for (int i = 0; i < m_loc; ++i)
+                {
+                    const int q = __ffs(mm) - 1;
+                    mm &= mm - 1u;
+                    if ((w >> i) & 1) o += tab[q];
+                }
+                const int sub = tid & ((1 << g_log) - 1);
+                for (int t = 0; t < g_log; ++t)
+                    if ((sub >> t) & 1) o += tab[16 + t];
+                float x = 0.f;
+                // Gray-code order: each step flips one bit of the offset.
+                for (int i = 0;;)
+                {
+                    x += S[o];
+                    if (++i >= (1 << per_log)) break;
+                    o ^= tab[16 + g_log + __ffs(i) - 1];
+                }
+                // The bin's threads in this warp (an aligned segment) stay together.
+                const unsigned seg = (w_log == 5 ? 0xffffffffu : (1u << (1 << w_log)) - 1u)
+                                     << ((tid & 31) & ~((1 << w_log) - 1));
+                for (int d = 1 << w_log >> 1; d > 0; d >>= 1) x += __shfl_down_sync(seg, x, d, 1 << w_log);
+                if (g_log > 5)
+                {
+                    if ((tid & 31) == 0) red[tid >> 5] = x;
+                }
+                else if (sub == 0)
+                    out[w] = static_cast<double>(x);
+            }
+            if (g_log > 5)
+            {
+                __syncthreads();
+                if (tid < (1 << m_loc))
+                {
+                    float x = 0.f;
+                    for (int i = 0; i < (1 << (g_log - 5)); ++i) x += red[(tid << (g_log - 5)) + i];
+                    out[tid] = static_cast<double>(x);
+                }
+            }
+        }
+    }
+}
+
 
 template <typename Real>
 __global__ void __launch_bounds__(kPassThreads) k_hist(const Cx<Real> *__restrict__ states, int n, int kmax, int cmin,
@@ -1709,27 +1713,6 @@ __global__ void k_collapse(Cx<Real> *states, std::uint64_t dim, std::uint64_t to
     }
 }
 
-// MIPT_GB300_CLUSTER_PASS=1 selects the two-CTA cluster kernel for FP32
-// passes (default: the single-CTA register-round kernel, measured faster).
-bool use_cluster_kernel()
-{
-    static const bool on = [] {
-        const char *v = std::getenv("MIPT_GB300_CLUSTER_PASS");
-        return v && v[0] == '1';
-    }();
-    return on;
-}
-
-// MIPT_GB300_PACKED_FMA=0 disables the packed FP32x2 gate arithmetic.
-bool use_packed_fma()
-{
-    static const bool on = [] {
-        const char *v = std::getenv("MIPT_GB300_PACKED_FMA");
-        return !(v && v[0] == '0');
-    }();
-    return on;
-}
-
 // The register-round pass runs on a persistent grid (resident CTAs loop over
 // the (trajectory, tile) items; measured 1.5 % faster at L=24 than one CTA per
 // item); MIPT_GB300_PERSISTENT_PASS=0 launches one CTA per item instead.
@@ -1811,20 +1794,6 @@ __host__ __device__ void histogram_geometry(int n, int kmax, int cmin, std::uint
     while (c < k && g.pos[c] == c) ++c;
     g.c = c;
     g.n_nl = n - k;
-}
-
-int fp32_register_bits()
-{
-    static const int rb = [] {
-        const char *v = std::getenv("MIPT_GB300_RB");
-        return (v && v[0] == '5') ? 5 : 6;
-    }();
-    return rb;
-}
-
-const PassGeom &fused_hist_geometry(const PassPlan &p, bool fp32)
-{
-    return (fp32 && p.cluster_rounds > 0 && use_cluster_kernel()) ? p.hgeom : p.geom;
 }
 
 int local_measured_count(const PassGeom &g, std::uint64_t chunk)
@@ -2006,6 +1975,153 @@ bool rounds_dfs(RoundSearch &S, std::size_t b, std::vector<std::uint32_t> &lanes
     return false;
 }
 
+// Rounds of k_pass_quads: two bonds on 16 amplitudes per thread. The first and
+// last round read and write global memory with the four lowest tile bits as
+// lanes; in between, four lanes should flip the four low bits of the
+// shared-memory place (quad_place: bits 0, 1 or 4, 2 or 5, 3 or 6) for
+// conflict-free 8-byte accesses. The last thread bit is the group; the pass is
+// split when bit k-1 is the group of the first and last rounds.
+struct QuadSearch
+{
+    int k, nr;
+    std::vector<std::pair<int, int>> bonds;
+    std::vector<int> assign, load;
+    int best_cost;
+    std::vector<int> best;
+};
+
+std::uint32_t quad_regs(const QuadSearch &S, const std::vector<int> &assign, int r)
+{
+    std::uint32_t reg = 0;
+    for (std::size_t b = 0; b < S.bonds.size(); ++b)
+        if (assign[b] == r) reg |= (1u << S.bonds[b].first) | (1u << S.bonds[b].second);
+    return reg;
+}
+
+// Bank lanes that a middle round's free bits cannot supply (0..4).
+int quad_missing_lanes(std::uint32_t reg)
+{
+    int miss = (reg & 1u) ? 1 : 0;
+    for (int i = 1; i < 4; ++i)
+        if (((reg >> i) & 1u) && ((reg >> (i + 3)) & 1u)) ++miss;
+    return miss;
+}
+
+void quad_dfs(QuadSearch &S, std::size_t b)
+{
+    if (b == S.bonds.size())
+    {
+        int cost = 0;
+        for (int r = 0; r < S.nr; ++r)
+        {
+            const std::uint32_t reg = quad_regs(S, S.assign, r);
+            if (r == 0 || r == S.nr - 1)
+            {
+                if (reg & 15u) return;
+                if ((reg >> (S.k - 1)) & 1u) cost += 4;
+            }
+            else
+                cost += quad_missing_lanes(reg);
+            // A full last round gives the next tile's load more to hide under.
+            if (r == S.nr - 1 && S.load[r] < 2) cost += 1;
+        }
+        if (S.best_cost < 0 || cost < S.best_cost)
+        {
+            S.best_cost = cost;
+            S.best = S.assign;
+        }
+        return;
+    }
+    for (int r = 0; r < S.nr; ++r)
+    {
+        if (S.load[r] >= 2) continue;
+        S.assign[b] = r;
+        ++S.load[r];
+        quad_dfs(S, b + 1);
+        --S.load[r];
+        if (S.best_cost == 0) return;
+    }
+}
+
+bool plan_quads(PassPlan &p)
+{
+    const int k = p.geom.k;
+    p.rounds = 0;
+    p.rb = 4;
+    p.split = 0;
+    if (k < 10 || k > 14 || p.geom.c < 4) return false;
+    QuadSearch S;
+    S.k = k;
+    for (int i = 0; i < p.gates.count; ++i) S.bonds.push_back({p.gates.la[i], p.gates.lb[i]});
+    const int nb = static_cast<int>(S.bonds.size());
+    for (int nr = std::max(1, (nb + 1) / 2); nr <= std::min(kMaxRounds, (nb + 1) / 2 + 2); ++nr)
+    {
+        S.nr = nr;
+        S.assign.assign(nb, -1);
+        S.load.assign(nr, 0);
+        S.best_cost = -1;
+        quad_dfs(S, 0);
+        if (S.best_cost < 0) continue;
+        p.split = 1;
+        for (int r = 0; r < nr; ++r)
+        {
+            Round &R = p.round[r];
+            const bool io = r == 0 || r == nr - 1;
+            std::uint32_t used = quad_regs(S, S.best, r);
+            // Lanes first, then the group, the register fill, the warp bits.
+            std::vector<int> lane;
+            auto take = [&](int q) {
+                lane.push_back(q);
+                used |= 1u << q;
+            };
+            for (int i = 0; i < 4; ++i)
+            {
+                if (!((used >> i) & 1u))
+                    take(i);
+                else if (!io && i > 0 && !((used >> (i + 3)) & 1u))
+                    take(i + 3);
+            }
+            auto lowest_free = [&]() {
+                for (int q = 0; q < k; ++q)
+                    if (!((used >> q) & 1u)) return q;
+                return -1;
+            };
+            int group = k - 1;
+            while ((used >> group) & 1u) --group;
+            if (io && group != k - 1) p.split = 0;
+            used |= 1u << group;
+            while (lane.size() < 5) take(lowest_free());
+            int slot = 0;
+            for (int s = 0; s < 3; ++s) R.slot[s] = -1;
+            for (int bI = 0; bI < nb; ++bI)
+                if (S.best[bI] == r)
+                {
+                    R.reg[2 * slot] = static_cast<std::int8_t>(S.bonds[bI].first);
+                    R.reg[2 * slot + 1] = static_cast<std::int8_t>(S.bonds[bI].second);
+                    R.slot[slot++] = static_cast<std::int16_t>(bI);
+                }
+            for (int i = 2 * slot; i < 4; ++i)
+            {
+                const int q = lowest_free();
+                R.reg[i] = static_cast<std::int8_t>(q);
+                used |= 1u << q;
+            }
+            int t = 0;
+            for (int q : lane) R.tid[t++] = static_cast<std::int8_t>(q);
+            for (int q = lowest_free(); q >= 0; q = lowest_free())
+            {
+                R.tid[t++] = static_cast<std::int8_t>(q);
+                used |= 1u << q;
+            }
+            R.tid[t++] = static_cast<std::int8_t>(group);
+            if (t != k - 4) return false;
+        }
+        p.rounds = nr;
+        return true;
+    }
+    return false;
+}
+
 // Schedules a pass's bonds into register rounds; returns false when the tile
 // is too small or no schedule fits kMaxRounds.
 bool plan_rounds(PassPlan &p, int rb)
@@ -2013,6 +2129,8 @@ bool plan_rounds(PassPlan &p, int rb)
     const int k = p.geom.k;
     p.rounds = 0;
     p.rb = rb;
+    p.split = 0;
+    if (rb == 4) return plan_quads(p);
     if (k < rb + 5 || k > 15) return false;
     RoundSearch S;
     S.k = k;
@@ -2071,184 +2189,6 @@ bool plan_rounds(PassPlan &p, int rb)
 }
 } // namespace
 
-namespace
-{
-// MIPT_GB300_CLUSTER_RB=5 selects 32 amplitudes per thread (256 threads per
-// CTA) for the cluster kernel instead of 64 (128 threads).
-int cluster_register_bits()
-{
-    static const int rb = [] {
-        const char *v = std::getenv("MIPT_GB300_CLUSTER_RB");
-        return (v && v[0] == '5') ? 5 : 6;
-    }();
-    return rb;
-}
-
-// Position of tile bit p once tile bit x is removed (the CTA-local offset).
-inline int opos(int p, int x) { return p > x ? p - 1 : p; }
-
-// Lanes 0..3 must flip the four low shared-memory bank bits (residues
-// {0,1,2,3} mod 5 of their offset positions) for conflict-free 8-byte access.
-bool lanes_ok(const int *l, int x)
-{
-    int seen = 0;
-    for (int i = 0; i < 4; ++i)
-    {
-        const int r = opos(l[i], x) % 5;
-        if (r > 3 || ((seen >> r) & 1)) return false;
-        seen |= 1 << r;
-    }
-    return true;
-}
-
-struct CSearch
-{
-    int k, nr, rb;
-    std::vector<std::pair<int, int>> bonds;
-    std::vector<int> assign, load;
-    std::vector<ClusterRound> out;
-};
-
-// Chooses x and lanes for rounds in order; the read side of round i uses the
-// storage coordinates of round i-1's x.
-bool cluster_choose(CSearch &S, int r, int prev_x)
-{
-    if (r == S.nr) return true;
-    const int k = S.k;
-    std::uint32_t reg = 0;
-    std::vector<int> mine;
-    for (std::size_t b = 0; b < S.bonds.size(); ++b)
-        if (S.assign[b] == r)
-        {
-            reg |= (1u << S.bonds[b].first) | (1u << S.bonds[b].second);
-            mine.push_back(static_cast<int>(b));
-        }
-    const bool first = r == 0, last = r == S.nr - 1;
-    for (int x = k - 1; x >= 0; --x)
-    {
-        if ((reg >> x) & 1u) continue;
-        // candidate lane sets: {0,1,2,3} first, then any four free bits
-        std::vector<std::array<int, 4>> cands;
-        if (!(reg & 0xFu) && x > 3) cands.push_back({0, 1, 2, 3});
-        if (!first && !last)
-        {
-            std::vector<int> freeb;
-            for (int q = 0; q < k; ++q)
-                if (!((reg >> q) & 1u) && q != x) freeb.push_back(q);
-            const int F = static_cast<int>(freeb.size());
-            for (int a = 0; a < F; ++a)
-                for (int b2 = a + 1; b2 < F; ++b2)
-                    for (int c = b2 + 1; c < F; ++c)
-                        for (int d = c + 1; d < F; ++d)
-                            cands.push_back({freeb[a], freeb[b2], freeb[c], freeb[d]});
-        }
-        for (auto l : cands)
-        {
-            // order lanes so lane i has residue i in the read coordinates
-            const int xr = first ? x : prev_x; // read (or load) coordinates
-            std::array<int, 4> ord{};
-            bool ok = true;
-            int seen = 0;
-            for (int q : l)
-            {
-                const int rr = opos(q, xr) % 5;
-                if (rr > 3 || ((seen >> rr) & 1)) { ok = false; break; }
-                seen |= 1 << rr;
-                ord[rr] = q;
-            }
-            if (!ok) continue;
-            if (!first && !lanes_ok(ord.data(), prev_x)) continue;
-            if (!last && !lanes_ok(ord.data(), x)) continue;
-            if ((first || last) && !(ord[0] == 0 && ord[1] == 1 && ord[2] == 2 && ord[3] == 3)) continue;
-            ClusterRound R{};
-            int slot = 0;
-            R.slot[0] = R.slot[1] = R.slot[2] = -1;
-            std::uint32_t used = (1u << x) | (1u << ord[0]) | (1u << ord[1]) | (1u << ord[2]) | (1u << ord[3]);
-            for (int b : mine)
-            {
-                R.reg[2 * slot] = static_cast<std::int8_t>(S.bonds[b].first);
-                R.reg[2 * slot + 1] = static_cast<std::int8_t>(S.bonds[b].second);
-                used |= (1u << S.bonds[b].first) | (1u << S.bonds[b].second);
-                R.slot[slot] = static_cast<std::int16_t>(b);
-                ++slot;
-            }
-            for (int i = 2 * slot; i < S.rb; ++i)
-                for (int q = 0; q < k; ++q)
-                    if (!((used >> q) & 1u))
-                    {
-                        R.reg[i] = static_cast<std::int8_t>(q);
-                        used |= 1u << q;
-                        break;
-                    }
-            int t = 0;
-            for (int i = 0; i < 4; ++i) R.tid[t++] = static_cast<std::int8_t>(ord[i]);
-            for (int q = 0; q < k; ++q)
-                if (!((used >> q) & 1u)) R.tid[t++] = static_cast<std::int8_t>(q);
-            if (t != k - 1 - S.rb) continue;
-            R.x = static_cast<std::int8_t>(x);
-            S.out[r] = R;
-            if (cluster_choose(S, r + 1, x)) return true;
-        }
-    }
-    return false;
-}
-
-bool cluster_dfs(CSearch &S, std::size_t b)
-{
-    if (b == S.bonds.size()) return cluster_choose(S, 0, -1);
-    for (int r = 0; r < S.nr; ++r)
-    {
-        if (S.load[r] >= S.rb / 2) continue;
-        S.assign[b] = r;
-        ++S.load[r];
-        if (cluster_dfs(S, b + 1)) return true;
-        --S.load[r];
-    }
-    return false;
-}
-
-bool plan_cluster_rounds(PassPlan &p, int rb)
-{
-    p.cluster_rounds = 0;
-    p.cluster_rb = rb;
-    if (p.geom.k != 14) return false;
-    CSearch S;
-    S.k = 14;
-    S.rb = rb;
-    for (int i = 0; i < p.gates.count; ++i) S.bonds.push_back({p.gates.la[i], p.gates.lb[i]});
-    const int nb = static_cast<int>(S.bonds.size());
-    const int slots = rb / 2;
-    for (int nr = std::max(1, (nb + slots - 1) / slots); nr <= kMaxRounds; ++nr)
-    {
-        S.nr = nr;
-        S.assign.assign(nb, -1);
-        S.load.assign(nr, 0);
-        S.out.assign(nr, ClusterRound{});
-        if (!cluster_dfs(S, 0)) continue;
-        for (int r = 0; r < nr; ++r) p.cround[r] = S.out[r];
-        p.cluster_rounds = nr;
-        // Histogram geometry of a half tile: the tile bits other than the last
-        // round's x are local; tile-index bit 0 is the CTA rank (qubit of x).
-        const int xz = p.cround[nr - 1].x;
-        PassGeom h{};
-        h.n = p.geom.n;
-        h.k = 13;
-        int a = 0;
-        for (int q = 0; q < 14; ++q)
-            if (q != xz) h.pos[a++] = p.geom.pos[q];
-        h.n_nl = p.geom.n_nl + 1;
-        h.nl[0] = p.geom.pos[xz];
-        for (int i = 0; i < p.geom.n_nl; ++i) h.nl[i + 1] = p.geom.nl[i];
-        int c = 0;
-        while (c < 13 && h.pos[c] == c) ++c;
-        h.c = c;
-        p.hgeom = h;
-        return true;
-    }
-    return false;
-}
-} // namespace
-
 std::vector<PassPlan> plan_layer(int n, const std::vector<Bond> &bonds, int kmax, int cmin, int rb)
 {
     if (n > 32) throw std::invalid_argument("engine supports at most 32 qubits");
@@ -2261,7 +2201,6 @@ std::vector<PassPlan> plan_layer(int n, const std::vector<Bond> &bonds, int kmax
         p.geom = make_geom(n, (1ull << kmax) - 1ull);
         p.gates.count = 0;
         plan_rounds(p, rb);
-        if (rb >= 5) plan_cluster_rounds(p, cluster_register_bits());
         return {p};
     }
     // Try first tiles made of a low contiguous block, optionally with the top
@@ -2288,13 +2227,9 @@ std::vector<PassPlan> plan_layer(int n, const std::vector<Bond> &bonds, int kmax
         if (unpaired)
         {
             p.rounds = 0;
-            p.cluster_rounds = 0;
             continue;
         }
         plan_rounds(p, rb);
-        bool parity = false;
-        for (int j = 0; j < p.gates.count; ++j) parity = parity || p.gates.kind[j];
-        if (rb >= 5 && !parity) plan_cluster_rounds(p, cluster_register_bits());
     }
     return best;
 }
@@ -2331,12 +2266,13 @@ PFN_cuTensorMapEncodeTiled_v12000 tile_map_encoder()
     return fn;
 }
 
-// Tensor map over `batch` FP32 states of 2^n amplitudes whose box is one tile
-// of geometry g in plain tile order. The global index bits split into runs of
-// local or non-local qubits; local runs longer than 8 bits split into boxes of
-// at most 256; the last run also carries the trajectory index. Needs local
-// positions in ascending qubit order, a local run at bit 0 (the innermost box
-// then spans >= 16 bytes) and at most 5 dimensions; false otherwise.
+// Tensor map over `batch` FP32 states of 2^n amplitudes whose box is half a
+// tile of geometry g (its top local bit fixed) in tile order under the 128-byte
+// swizzle. The global index bits split into runs of local or non-local
+// qubits: the four lowest (128 bytes) are the innermost dimension, later local
+// runs longer than 8 bits split into boxes of at most 256; the last run also
+// carries the trajectory index. Needs local positions in ascending qubit order
+// with qubits 0..3 among them and at most 5 dimensions; false otherwise.
 bool encode_tile_map(CUtensorMap &map, TileTma &t, const Cx<float> *states, int batch, const PassGeom &g)
 {
     std::memset(&map, 0, sizeof(map));
@@ -2346,15 +2282,16 @@ bool encode_tile_map(CUtensorMap &map, TileTma &t, const Cx<float> *states, int 
         if (g.pos[i] <= g.pos[i - 1]) return false;
     bool local[kMaxQubits] = {};
     for (int i = 0; i < g.k; ++i) local[g.pos[i]] = true;
-    if (!local[0]) return false;
+    if (!(local[0] && local[1] && local[2] && local[3]) || g.k < 5) return false;
     int q = 0;
     while (q < g.n)
     {
         int len = 1;
-        while (q + len < g.n && local[q + len] == local[q] && (!local[q] || len < 8)) ++len;
+        while (q + len < g.n && local[q + len] == local[q] && (!local[q] || len < (q == 0 ? 4 : 8))) ++len;
         if (t.rank == 5) return false;
         t.lo[t.rank] = q;
         t.bits[t.rank] = len;
+        if (local[q]) t.half_dim = t.rank;
         ++t.rank;
         q += len;
     }
@@ -2365,14 +2302,14 @@ bool encode_tile_map(CUtensorMap &map, TileTma &t, const Cx<float> *states, int 
         const bool loc = local[t.lo[d]];
         dims[d] = 1ull << t.bits[d];
         if (d + 1 == t.rank) dims[d] *= static_cast<cuuint64_t>(batch);
-        box[d] = loc ? (1u << t.bits[d]) : 1u;
+        box[d] = loc ? (1u << (t.bits[d] - (d == t.half_dim ? 1 : 0))) : 1u;
         es[d] = 1;
         if (d > 0) strides[d - 1] = (1ull << t.lo[d]) * sizeof(Cx<float>);
     }
     if (dims[t.rank - 1] >= (1ull << 32)) return false;
     return tile_map_encoder()(&map, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, static_cast<cuuint32_t>(t.rank),
                               const_cast<Cx<float> *>(states), dims, strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                              CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                              CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
@@ -2387,41 +2324,64 @@ int take_withheld_load()
     return c > 0 ? 1 : 0;
 }
 
-// Launches k_pass_rounds<Real, RB, TMA, PAR> on its grid.
-template <typename Real, int RB, bool TMA, bool PAR>
+// Launches k_pass_rounds<Real, RB, PAR> on its grid.
+template <typename Real, int RB, bool PAR>
 cudaError_t launch_rounds(Cx<Real> *states, int batch, const PassPlan &plan, const Cx<Real> *layer_gates,
                           std::size_t gate_stride, const Collapse *collapse_in, std::size_t collapse_stride,
                           const LayerMeas *meas, std::size_t meas_stride, double *partials, int fuse_hist,
-                          const CUtensorMap &map, const TileTma &tt, int *err, cudaStream_t s,
-                          std::uint64_t col_keep, int col_scaled, int sparse)
+                          cudaStream_t s, std::uint64_t col_keep, int col_scaled, int sparse)
 {
-    const void *fn = reinterpret_cast<const void *>(&k_pass_rounds<Real, RB, TMA, PAR>);
-    const std::size_t smem = (sizeof(Cx<Real>) << plan.geom.k) + (TMA ? (sizeof(float) << plan.geom.k) + 128 : 0) +
+    const void *fn = reinterpret_cast<const void *>(&k_pass_rounds<Real, RB, PAR>);
+    const std::size_t smem = (sizeof(Cx<Real>) << plan.geom.k) +
                              (sparse ? sizeof(std::uint32_t) * (static_cast<std::size_t>(batch) + 1) : 0);
     cudaError_t e = ensure_smem_attr<Real>(fn, smem);
     if (e != cudaSuccess) return e;
     const int threads = 1 << (plan.geom.k - RB);
     const dim3 pgrid = pass_grid(fn, threads, smem, dim3(1u << plan.geom.n_nl, batch));
-    k_pass_rounds<Real, RB, TMA, PAR><<<pgrid, threads, smem, s>>>(states, plan, layer_gates, gate_stride, collapse_in,
-                                                               collapse_stride, meas, meas_stride, partials,
-                                                               fuse_hist, use_packed_fma() ? 1 : 0, batch, map, tt,
-                                                               err, col_keep, col_scaled, sparse,
-                                                               TMA ? take_withheld_load() : 0);
+    k_pass_rounds<Real, RB, PAR><<<pgrid, threads, smem, s>>>(states, plan, layer_gates, gate_stride, collapse_in,
+                                                          collapse_stride, meas, meas_stride, partials, fuse_hist,
+                                                          batch, col_keep, col_scaled, sparse);
     return cudaGetLastError();
 }
 
+// Dynamic shared memory of k_pass_quads without the sparse item table.
+std::size_t quad_smem(const PassPlan &p)
+{
+    return (sizeof(Cx<float>) << p.geom.k) + (sizeof(float) << p.geom.k) +
+           (sizeof(std::uint32_t) * static_cast<std::size_t>(p.rounds) << (p.geom.k - 5));
+}
+
+// Launches k_pass_quads<TMA, PAR> on its grid.
+template <bool TMA, bool PAR>
+cudaError_t launch_quads(Cx<float> *states, int batch, const PassPlan &plan, const Cx<float> *layer_gates,
+                         std::size_t gate_stride, const Collapse *collapse_in, std::size_t collapse_stride,
+                         const LayerMeas *meas, std::size_t meas_stride, double *partials, int fuse_hist,
+                         const CUtensorMap &map, const TileTma &tt, int *err, cudaStream_t s, std::uint64_t col_keep,
+                         int col_scaled, int sparse)
+{
+    const void *fn = reinterpret_cast<const void *>(&k_pass_quads<TMA, PAR>);
+    const int threads = 1 << (plan.geom.k - 5);
+    const std::size_t smem =
+        quad_smem(plan) + (sparse ? sizeof(std::uint32_t) * (static_cast<std::size_t>(batch) + 1) : 0);
+    cudaError_t e = ensure_smem_attr<float>(fn, smem);
+    if (e != cudaSuccess) return e;
+    const dim3 pgrid = pass_grid(fn, threads, smem, dim3(1u << plan.geom.n_nl, batch));
+    k_pass_quads<TMA, PAR><<<pgrid, threads, smem, s>>>(states, plan, layer_gates, gate_stride, collapse_in,
+                                                       collapse_stride, meas, meas_stride, partials, fuse_hist, batch,
+                                                       map, tt, err, col_keep, col_scaled, sparse,
+                                                       TMA ? take_withheld_load() : 0);
+    return cudaGetLastError();
+}
 
 bool sparse_pass_supported(const PassPlan &plan, bool fp32, int batch)
 {
     if (plan.rounds <= 0 || plan.geom.n_nl <= 0 || batch < 1) return false;
-    if (fp32 && plan.cluster_rounds > 0 && use_cluster_kernel()) return false;
-    if (fp32 && plan.rb != 5 && plan.rb != 6) return false;
-    if (!fp32 && plan.rb != 5) return false;
+    if (plan.rb != (fp32 ? 4 : 5)) return false;
     if ((static_cast<std::uint64_t>(batch) << plan.geom.n_nl) >= (1ull << 31)) return false;
-    // Tile (+ histogram values and alignment with TMA) + item table.
-    const std::size_t base = fp32 ? (sizeof(Cx<float>) << plan.geom.k) + (sizeof(float) << plan.geom.k) + 128
-                                  : (sizeof(Cx<double>) << plan.geom.k);
-    return base + sizeof(std::uint32_t) * (static_cast<std::size_t>(batch) + 1) <= (200u << 10);
+    // Tile, histogram values, alignment and place table (FP32) + item table.
+    const std::size_t table = sizeof(std::uint32_t) * (static_cast<std::size_t>(batch) + 1);
+    if (!fp32) return (sizeof(Cx<double>) << plan.geom.k) + table <= (200u << 10);
+    return quad_smem(plan) + table <= (220u << 10);
 }
 
 template <typename Real>
@@ -2435,64 +2395,33 @@ cudaError_t launch_pass(Cx<Real> *states, int batch, const PassPlan &plan, const
     if ((sparse || col_keep != ~0ull || !col_scaled) && !sparse_pass_supported(plan, sizeof(Real) == 4, batch))
         return cudaErrorInvalidValue;
     if (sparse && (collapse_in == nullptr || fuse_hist)) return cudaErrorInvalidValue;
-    if constexpr (sizeof(Real) == 4)
-    {
-        if (plan.cluster_rounds > 0 && use_cluster_kernel())
-        {
-            const std::size_t smem = sizeof(Cx<float>) << 13;
-            dim3 cgrid(2u << plan.geom.n_nl, batch);
-            cudaError_t e;
-            if (plan.cluster_rb == 6)
-            {
-                e = cudaFuncSetAttribute(reinterpret_cast<const void *>(&k_pass_cluster<6>),
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
-                if (e != cudaSuccess) return e;
-                k_pass_cluster<6><<<cgrid, 128, smem, s>>>(states, plan, layer_gates, gate_stride, collapse_in,
-                                                           collapse_stride, meas, meas_stride, partials, fuse_hist);
-            }
-            else
-            {
-                e = cudaFuncSetAttribute(reinterpret_cast<const void *>(&k_pass_cluster<5>),
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
-                if (e != cudaSuccess) return e;
-                k_pass_cluster<5><<<cgrid, 256, smem, s>>>(states, plan, layer_gates, gate_stride, collapse_in,
-                                                           collapse_stride, meas, meas_stride, partials, fuse_hist);
-            }
-            return cudaGetLastError();
-        }
-    }
     if (plan.rounds > 0)
     {
-#define MG_ROUNDS(RBV, TMAV, PARV)                                                                                    \
-    launch_rounds<Real, RBV, TMAV, PARV>(states, batch, plan, layer_gates, gate_stride, collapse_in, collapse_stride, \
-                                         meas, meas_stride, partials, fuse_hist, map, tt, err, s, col_keep,            \
-                                         col_scaled, sparse)
-        CUtensorMap map;
-        TileTma tt{};
-        std::memset(&map, 0, sizeof(map));
         const bool par = parity_mode != 0;
         if constexpr (sizeof(Real) == 4)
         {
+            if (plan.rb != 4) return cudaErrorInvalidValue;
+            CUtensorMap map;
+            TileTma tt{};
             const bool tma = use_persistent_pass() && use_tile_tma() && err != nullptr &&
                              encode_tile_map(map, tt, states, batch, plan.geom);
-            if (plan.rb == 6)
-            {
-                if (tma) return par ? MG_ROUNDS(6, true, true) : MG_ROUNDS(6, true, false);
-                return par ? MG_ROUNDS(6, false, true) : MG_ROUNDS(6, false, false);
-            }
-            if (plan.rb == 5)
-            {
-                if (tma) return par ? MG_ROUNDS(5, true, true) : MG_ROUNDS(5, true, false);
-                return par ? MG_ROUNDS(5, false, true) : MG_ROUNDS(5, false, false);
-            }
-            return cudaErrorInvalidValue;
+            if (!tma) std::memset(&map, 0, sizeof(map));
+#define MG_QUADS(TMAV, PARV)                                                                                          \
+    launch_quads<TMAV, PARV>(states, batch, plan, layer_gates, gate_stride, collapse_in, collapse_stride, meas,        \
+                             meas_stride, partials, fuse_hist, map, tt, err, s, col_keep, col_scaled, sparse)
+            if (tma) return par ? MG_QUADS(true, true) : MG_QUADS(true, false);
+            return par ? MG_QUADS(false, true) : MG_QUADS(false, false);
+#undef MG_QUADS
         }
         else
         {
             if (plan.rb != 5) return cudaErrorInvalidValue;
-            return par ? MG_ROUNDS(5, false, true) : MG_ROUNDS(5, false, false);
-        }
+#define MG_ROUNDS(PARV)                                                                                               \
+    launch_rounds<Real, 5, PARV>(states, batch, plan, layer_gates, gate_stride, collapse_in, collapse_stride, meas,    \
+                                 meas_stride, partials, fuse_hist, s, col_keep, col_scaled, sparse)
+            return par ? MG_ROUNDS(true) : MG_ROUNDS(false);
 #undef MG_ROUNDS
+        }
     }
     const std::size_t smem = pass_smem<Real>(plan.geom.k);
     cudaError_t e = ensure_smem_attr<Real>(reinterpret_cast<const void *>(&k_pass<Real>), smem);

@@ -29,7 +29,7 @@ struct Bond
 
 // One register round of a pass: every thread holds 2^rb amplitudes whose
 // register-index bit i is local tile bit reg[i]; thread-index bit i is local
-// bit tid[i] (the first five, one per residue mod 5, are the warp lanes).
+// bit tid[i] (the first five are the warp lanes; FP32: the last is the group).
 // slot[s] >= 0 applies pass gate slot[s] on register bits (2s, 2s+1).
 struct Round
 {
@@ -40,25 +40,13 @@ struct Round
 
 constexpr int kMaxRounds = 8;
 
-// Register round of the two-CTA cluster kernel: the 2^14-amplitude tile is
-// split between the two CTAs of a cluster by tile bit x (CTA rank = bit x);
-// each thread holds 32 amplitudes (register bits reg[0..5)), thread-index bit
-// i is tile bit tid[i]. slot[s] >= 0 applies pass gate slot[s] on register
-// bits (2s, 2s+1).
-struct ClusterRound
-{
-    std::int8_t reg[6];
-    std::int8_t tid[8];
-    std::int8_t x;
-    std::int16_t slot[3];
-};
-
 // TMA view of a pass's tiles: dimension d of the tensor map covers global
 // index bits [lo[d], lo[d] + bits[d]) of the batch of states (the last one
 // also the trajectory bits above bit n); local runs are whole box dimensions.
 struct TileTma
 {
     int rank;
+    int half_dim; // the dimension whose upper half is the tile's second half box
     int lo[5];
     int bits[5];
 };
@@ -69,11 +57,8 @@ struct PassPlan
     PassGates gates;
     int rounds; // 0: tile too small for register rounds (shared-memory kernel)
     int rb;     // register bits per thread
+    int split;  // rb 4: the first and last rounds' groups are the tile's halves
     Round round[kMaxRounds];
-    int cluster_rounds; // > 0: FP32 two-CTA cluster schedule available
-    int cluster_rb;     // register bits per thread of that schedule
-    ClusterRound cround[kMaxRounds];
-    PassGeom hgeom; // histogram geometry of one CTA's half tile (cluster kernel)
 };
 
 // Splits one layer's bonds into tiled passes of at most kmax local qubits
@@ -81,14 +66,9 @@ struct PassPlan
 // schedules each pass's bonds into register rounds of rb register bits.
 std::vector<PassPlan> plan_layer(int n, const std::vector<Bond> &bonds, int kmax, int cmin, int rb);
 
-// Geometry of the per-tile histogram partials a pass writes when it fuses
-// the layer's Born histogram (a half tile for the cluster kernel).
-const PassGeom &fused_hist_geometry(const PassPlan &p, bool fp32);
-
-// Register bits per thread of the register-round pass kernel (FP32: 6 by
-// default, MIPT_GB300_RB=5 for 32 amplitudes per thread; FP64: 5).
-int fp32_register_bits();
-template <typename Real> inline int register_bits() { return sizeof(Real) == 4 ? fp32_register_bits() : 5; }
+// Register bits per thread of the pass kernels (FP32 k_pass_quads: 4, FP64
+// k_pass_rounds: 5).
+template <typename Real> inline int register_bits() { return sizeof(Real) == 4 ? 4 : 5; }
 
 // Tile geometry used for a stand-alone histogram of the sites in `chunk`:
 // low contiguous qubits, then as many unmeasured qubits as fit, so that few
