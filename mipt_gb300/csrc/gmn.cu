@@ -24,11 +24,12 @@
 // -(Re Tr(rho W) + d) / 2.
 //
 // GB300 mapping: P_C needs the spectrum of an 8x8 Hermitian matrix; eight
-// lanes share one problem, lane c holding column c, and diagonalise by a
-// parallel cyclic Jacobi (round-robin: 4 disjoint rotations per round, 7
-// rounds per sweep) with column exchanges by warp shuffles. W and Q are staged
-// in shared memory for the partial-transpose gathers; the ADMM state streams
-// from global memory. Compute-bound on the FP32 pipes.
+// lanes share one, lane c holding column c, and diagonalise by a parallel
+// cyclic Jacobi (round-robin: 4 disjoint rotations per round, 7 rounds per
+// sweep) with column exchanges by warp shuffles. The six projections of an
+// iteration run on six such groups, the twelve spectra of a certificate on
+// twelve. The ADMM state, W and Q are in shared memory. Bound by the latency of
+// the Jacobi rounds at a few thousand states, by FP32 issue above.
 #include "mipt_gb300.h"
 
 #include "common.cuh"
@@ -57,7 +58,6 @@ constexpr int kLanes = 8;
 // iterations on average, against 91.9 % and 136 at 1.0.
 constexpr double kDefaultSigma = 0.1;
 constexpr int kThreads = 256;
-constexpr int kProbPerBlock = kThreads / kLanes;
 
 template <typename Real> struct C2
 {
@@ -236,124 +236,140 @@ struct GmnArrays
     float *res; // FP32 residual of each state's last iteration
 };
 
+// `iters` ADMM iterations. Six 8-lane groups share a problem, one per box
+// projection (group b: U_m for even b, V_m for odd, m = b / 2 + 1): the six
+// eigenproblems of an iteration do not depend on one another, and one
+// after the other in one group they were a serial chain that left most of the
+// chip idle at a few thousand states. The ADMM state stays in shared memory for
+// the launch. Every entry is formed by the same operations as one group would
+// form it, and the residual's terms are added in that order, so iterates and
+// iteration counts do not depend on the split. Measured with the certificates'
+// split below: 2,048 states, 600 iterations at most, 552 -> 152 ms; 32,768
+// states, 200 at most, 768 -> 532 ms.
+constexpr int kBoxes = 6;
+constexpr int kIterProblems = 2; // per CTA: 96 threads, three full warps
+constexpr int kIterThreads = kIterProblems * kBoxes * kLanes;
+
+// Shared memory of one problem, in complex numbers: W, Q_1..3, projection
+// scratch per box, U, V, Yh, Zh.
+constexpr int kIterShared = 64 + 192 + kBoxes * 64 + 4 * 192;
+
 template <typename Real>
-__global__ void __launch_bounds__(kThreads) k_gmn_iterate(GmnArrays a, int iters)
+__global__ void __launch_bounds__(kIterThreads) k_gmn_iterate(GmnArrays a, int iters)
 {
-    // Per problem: W (64), Q_1..3 (192), projection scratch (64) -- dynamic.
     extern __shared__ __align__(16) unsigned char gmn_smem[];
-    auto sW = reinterpret_cast<C2<Real>(*)[64]>(gmn_smem);
-    auto sQ = reinterpret_cast<C2<Real>(*)[3][64]>(gmn_smem + sizeof(C2<Real>) * 64 * kProbPerBlock);
-    auto sR = reinterpret_cast<C2<Real>(*)[64]>(gmn_smem + sizeof(C2<Real>) * 256 * kProbPerBlock);
-    const int g = threadIdx.x / kLanes, c = threadIdx.x % kLanes;
-    const int prob = blockIdx.x * kProbPerBlock + g;
+    __shared__ float terms[kIterProblems][kBoxes][8][8];
+    const int slot = threadIdx.x / (kBoxes * kLanes);
+    const int box = threadIdx.x / kLanes % kBoxes, c = threadIdx.x % kLanes;
+    const int prob = blockIdx.x * kIterProblems + slot;
     const int lane = threadIdx.x & 31, gbase = lane & ~7;
     const unsigned gmask = 0xFFu << gbase;
-    if (prob >= a.count || a.done[prob]) return; // whole 8-lane groups leave together
-    const Real sigma = static_cast<Real>(a.sigma[prob]);
-    const C2<Real> *rho = static_cast<const C2<Real> *>(a.rho) + static_cast<std::size_t>(prob) * 64;
-    C2<Real> *U = static_cast<C2<Real> *>(a.U) + static_cast<std::size_t>(prob) * 192;
-    C2<Real> *V = static_cast<C2<Real> *>(a.V) + static_cast<std::size_t>(prob) * 192;
-    C2<Real> *Yh = static_cast<C2<Real> *>(a.Yh) + static_cast<std::size_t>(prob) * 192;
-    C2<Real> *Zh = static_cast<C2<Real> *>(a.Zh) + static_cast<std::size_t>(prob) * 192;
-    C2<Real> *Wg = static_cast<C2<Real> *>(a.W) + static_cast<std::size_t>(prob) * 64;
-    C2<Real> *Qg = static_cast<C2<Real> *>(a.Q) + static_cast<std::size_t>(prob) * 192;
+    const bool live = prob < a.count && !a.done[prob];
+    if (!__syncthreads_or(live)) return;
+    C2<Real> *sW = reinterpret_cast<C2<Real> *>(gmn_smem) + static_cast<std::size_t>(slot) * kIterShared;
+    C2<Real> *sQ = sW + 64, *sR = sQ + 192 + box * 64;
+    C2<Real> *U = sQ + 192 + kBoxes * 64, *V = U + 192, *Yh = V + 192, *Zh = Yh + 192;
+    const std::size_t at = static_cast<std::size_t>(live ? prob : 0);
+    const Real sigma = live ? static_cast<Real>(a.sigma[at]) : Real(1);
+    const C2<Real> *rho = static_cast<const C2<Real> *>(a.rho) + at * 64;
+    C2<Real> *gU = static_cast<C2<Real> *>(a.U) + at * 192, *gV = static_cast<C2<Real> *>(a.V) + at * 192;
+    C2<Real> *gY = static_cast<C2<Real> *>(a.Yh) + at * 192, *gZ = static_cast<C2<Real> *>(a.Zh) + at * 192;
+    const int self = box * kLanes + c; // thread within the problem
+    if (live)
+        for (int i = self; i < 192; i += kBoxes * kLanes)
+        {
+            U[i] = gU[i];
+            V[i] = gV[i];
+            Yh[i] = gY[i];
+            Zh[i] = gZ[i];
+        }
+    __syncthreads();
     const Real two_over_sigma = Real(2) / sigma;
-    // Residual of the launch's last iteration: |dYh|^2 + |dZh|^2 (primal) plus
-    // sigma^2 (|dU|^2 + |dV|^2) (dual), over this lane's column.
-    float resid = 0.f;
+    const int bm = box / 2 + 1, bo = (bm - 1) * 64; // this group's m
+    const bool is_u = (box & 1) == 0;
     for (int it = 0; it < iters; ++it)
     {
         const bool last = it + 1 == iters;
-        // x-step: W column c.
-#pragma unroll
-        for (int r = 0; r < 8; ++r)
-        {
-            C2<Real> w = cscale(rho[c * 8 + r], -two_over_sigma);
-#pragma unroll
-            for (int m = 1; m <= 3; ++m)
+        // x-step: W column c, rows box and box + 6.
+        if (live)
+            for (int r = box; r < 8; r += kBoxes)
             {
-                const int s = pt_src(r, c, m);
-                const int o = (m - 1) * 64;
-                w = cadd(w, csub(U[o + s], Yh[o + s]));           // PT_m(a_m)
-                w = cadd(w, csub(V[o + c * 8 + r], Zh[o + c * 8 + r])); // b_m
-            }
-            sW[g][c * 8 + r] = cscale(w, Real(1) / Real(3));
-        }
-        __syncwarp(gmask);
-        // Q_m = (a_m + PT_m(W - b_m)) / 2.
+                C2<Real> w = cscale(rho[c * 8 + r], -two_over_sigma);
 #pragma unroll
-        for (int m = 1; m <= 3; ++m)
-        {
-            const int o = (m - 1) * 64;
-#pragma unroll
-            for (int r = 0; r < 8; ++r)
-            {
-                const int s = pt_src(r, c, m);
-                const C2<Real> am = csub(U[o + c * 8 + r], Yh[o + c * 8 + r]);
-                const C2<Real> wb = csub(sW[g][s], csub(V[o + s], Zh[o + s]));
-                sQ[g][m - 1][c * 8 + r] = cscale(cadd(am, wb), Real(0.5));
-            }
-        }
-        __syncwarp(gmask);
-        // Every lane has read its old U, V, Yh, Zh entries: new values may be written.
-#pragma unroll 1
-        for (int m = 1; m <= 3; ++m)
-        {
-            const int o = (m - 1) * 64;
-            C2<Real> X[8];
-            // U_m = P_C(Q_m + Yh_m); Yh_m += Q_m - U_m.
-#pragma unroll
-            for (int r = 0; r < 8; ++r) X[r] = cadd(sQ[g][m - 1][c * 8 + r], Yh[o + c * 8 + r]);
-            C2<Real> X0[8];
-#pragma unroll
-            for (int r = 0; r < 8; ++r) X0[r] = X[r];
-            project_box(X, c, gbase, gmask, sR[g]);
-#pragma unroll
-            for (int r = 0; r < 8; ++r)
-            {
-                if (last)
+                for (int m = 1; m <= 3; ++m)
                 {
-                    const C2<Real> dy = csub(csub(X0[r], X[r]), Yh[o + c * 8 + r]);
-                    const C2<Real> du = csub(X[r], U[o + c * 8 + r]);
-                    resid += float(dy.re * dy.re + dy.im * dy.im) +
-                             float(sigma * sigma * (du.re * du.re + du.im * du.im));
+                    const int s = pt_src(r, c, m);
+                    const int o = (m - 1) * 64;
+                    w = cadd(w, csub(U[o + s], Yh[o + s]));           // PT_m(a_m)
+                    w = cadd(w, csub(V[o + c * 8 + r], Zh[o + c * 8 + r])); // b_m
                 }
-                U[o + c * 8 + r] = X[r];
-                Yh[o + c * 8 + r] = csub(X0[r], X[r]);
+                sW[c * 8 + r] = cscale(w, Real(1) / Real(3));
             }
-            // V_m = P_C(W - PT_m(Q_m) + Zh_m); Zh_m += W - PT_m(Q_m) - V_m.
+        __syncthreads();
+        // Q_m = (a_m + PT_m(W - b_m)) / 2: four rows per group.
+        if (live)
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+            {
+                const int r = (is_u ? 0 : 4) + i, s = pt_src(r, c, bm);
+                const C2<Real> am = csub(U[bo + c * 8 + r], Yh[bo + c * 8 + r]);
+                const C2<Real> wb = csub(sW[s], csub(V[bo + s], Zh[bo + s]));
+                sQ[bo + c * 8 + r] = cscale(cadd(am, wb), Real(0.5));
+            }
+        __syncthreads();
+        // U_m = P_C(Q_m + Yh_m), Yh_m += Q_m - U_m; or V_m = P_C(W - PT_m(Q_m) +
+        // Zh_m), Zh_m += W - PT_m(Q_m) - V_m.
+        if (live)
+        {
+            C2<Real> *P = is_u ? U : V, *D = is_u ? Yh : Zh;
+            C2<Real> X[8], X0[8];
 #pragma unroll
             for (int r = 0; r < 8; ++r)
             {
-                X[r] = cadd(csub(sW[g][c * 8 + r], sQ[g][m - 1][pt_src(r, c, m)]), Zh[o + c * 8 + r]);
+                if (is_u)
+                    X[r] = cadd(sQ[bo + c * 8 + r], Yh[bo + c * 8 + r]);
+                else
+                    X[r] = cadd(csub(sW[c * 8 + r], sQ[bo + pt_src(r, c, bm)]), Zh[bo + c * 8 + r]);
                 X0[r] = X[r];
             }
-            project_box(X, c, gbase, gmask, sR[g]);
+            project_box(X, c, gbase, gmask, sR);
 #pragma unroll
             for (int r = 0; r < 8; ++r)
             {
                 if (last)
                 {
-                    const C2<Real> dz = csub(csub(X0[r], X[r]), Zh[o + c * 8 + r]);
-                    const C2<Real> dv = csub(X[r], V[o + c * 8 + r]);
-                    resid += float(dz.re * dz.re + dz.im * dz.im) +
-                             float(sigma * sigma * (dv.re * dv.re + dv.im * dv.im));
+                    // Residual term: the dual's step (primal) and the
+                    // projection's step times sigma (dual).
+                    const C2<Real> dy = csub(csub(X0[r], X[r]), D[bo + c * 8 + r]);
+                    const C2<Real> du = csub(X[r], P[bo + c * 8 + r]);
+                    terms[slot][box][r][c] = float(dy.re * dy.re + dy.im * dy.im) +
+                                             float(sigma * sigma * (du.re * du.re + du.im * du.im));
                 }
-                V[o + c * 8 + r] = X[r];
-                Zh[o + c * 8 + r] = csub(X0[r], X[r]);
+                P[bo + c * 8 + r] = X[r];
+                D[bo + c * 8 + r] = csub(X0[r], X[r]);
             }
         }
-        __syncwarp(gmask);
+        __syncthreads();
     }
-#pragma unroll
-    for (int r = 0; r < 8; ++r)
+    if (!live) return;
+    C2<Real> *Wg = static_cast<C2<Real> *>(a.W) + at * 64, *Qg = static_cast<C2<Real> *>(a.Q) + at * 192;
+    for (int i = self; i < 192; i += kBoxes * kLanes)
     {
-        Wg[c * 8 + r] = sW[g][c * 8 + r];
-#pragma unroll
-        for (int m = 0; m < 3; ++m) Qg[m * 64 + c * 8 + r] = sQ[g][m][c * 8 + r];
+        gU[i] = U[i];
+        gV[i] = V[i];
+        gY[i] = Yh[i];
+        gZ[i] = Zh[i];
+        Qg[i] = sQ[i];
+        if (i < 64) Wg[i] = sW[i];
     }
-    for (int off = 4; off > 0; off /= 2) resid += __shfl_xor_sync(gmask, resid, off);
-    if (c == 0) a.res[prob] = sqrtf(resid);
+    if (box == 0)
+    {
+        float resid = 0.f;
+        for (int b = 0; b < kBoxes; ++b)
+            for (int r = 0; r < 8; ++r) resid += terms[slot][b][r][c];
+        for (int off = 4; off > 0; off /= 2) resid += __shfl_xor_sync(gmask, resid, off);
+        if (c == 0) a.res[prob] = sqrtf(resid);
+    }
 }
 
 // Sum over the 8 lanes of a group.
@@ -399,16 +415,23 @@ __device__ double eigval8(C2<double> (&A)[8], int c, int gbase, unsigned gmask)
     return pick(A, c).re;
 }
 
-template <typename Real> __global__ void __launch_bounds__(kThreads) k_gmn_check(GmnCheck k)
+// Certificates, one problem per CTA: the twelve FP64 spectra of a certificate
+// (per m: Z_m, PT_m(Z_m), Q_m, W - PT_m(Q_m)) take one 8-lane group each. One
+// group for all twelve was a chain of 588 FP64 Jacobi rounds, 5 to 10 ms a
+// launch however few states were candidates (68 % of the solver's time).
+constexpr int kCheckThreads = 12 * kLanes;
+
+template <typename Real> __global__ void __launch_bounds__(kCheckThreads) k_gmn_check(GmnCheck k)
 {
+    __shared__ double dual_part[12], feas_part[12], s_primal;
     const int g = threadIdx.x / kLanes, c = threadIdx.x % kLanes;
-    const int prob = blockIdx.x * kProbPerBlock + g;
+    const int prob = blockIdx.x;
     const int lane = threadIdx.x & 31, gbase = lane & ~7;
     const unsigned gmask = 0xFFu << gbase;
-    if (prob >= k.count || k.done[prob]) return;
+    if (k.done[prob]) return;
     if (!k.force && (k.res[prob] > k.cand_tol || k.iter_now < k.next_check[prob]))
     {
-        if (c == 0) atomicAdd(k.remaining, 1);
+        if (threadIdx.x == 0) atomicAdd(k.remaining, 1);
         return;
     }
     const double sigma = k.sigma[prob];
@@ -417,47 +440,61 @@ template <typename Real> __global__ void __launch_bounds__(kThreads) k_gmn_check
     const C2<Real> *Q = static_cast<const C2<Real> *>(k.Q) + static_cast<std::size_t>(prob) * 192;
     const C2<Real> *Zh = static_cast<const C2<Real> *>(k.Zh) + static_cast<std::size_t>(prob) * 192;
     auto ld = [](const C2<Real> &x) { return C2<double>{static_cast<double>(x.re), static_cast<double>(x.im)}; };
-    // Primal Re Tr(rho W) = sum_{r,c} Re(rho[r][c] W[c][r]).
-    double p = 0.0;
-#pragma unroll
-    for (int r = 0; r < 8; ++r)
+    if (g == 0)
     {
-        const double2 a = rho[c * 8 + r];
-        const C2<double> w = ld(W[r * 8 + c]);
-        p += a.x * w.re - a.y * w.im;
+        // Primal Re Tr(rho W) = sum_{r,c} Re(rho[r][c] W[c][r]).
+        double p = 0.0;
+#pragma unroll
+        for (int r = 0; r < 8; ++r)
+        {
+            const double2 a = rho[c * 8 + r];
+            const C2<double> w = ld(W[r * 8 + c]);
+            p += a.x * w.re - a.y * w.im;
+        }
+        p = group_sum(p, gmask);
+        if (c == 0) s_primal = p;
     }
-    p = group_sum(p, gmask);
     // Dual: Z_m = sigma Zh_m - (sigma sum Zh + rho) / 3 at any entry.
     auto zshift = [&](int m, int idx) {
         C2<double> s{rho[idx].x, rho[idx].y};
         for (int mm = 0; mm < 3; ++mm) s = cadd(s, cscale(ld(Zh[mm * 64 + idx]), sigma));
         return csub(cscale(ld(Zh[m * 64 + idx]), sigma), cscale(s, 1.0 / 3.0));
     };
-    double d = 0.0, feas = 0.0;
-    for (int m = 1; m <= 3; ++m)
+    const int m = g / 4 + 1, kind = g % 4;
+    C2<double> A[8];
+#pragma unroll
+    for (int r = 0; r < 8; ++r)
     {
-        C2<double> A[8];
-#pragma unroll
-        for (int r = 0; r < 8; ++r) A[r] = zshift(m - 1, c * 8 + r);
-        double l = eigval8(A, c, gbase, gmask);
-        d -= group_sum(fmax(l, 0.0), gmask);
-#pragma unroll
-        for (int r = 0; r < 8; ++r) A[r] = zshift(m - 1, pt_src(r, c, m));
-        l = eigval8(A, c, gbase, gmask);
-        d -= group_sum(fmax(l, 0.0), gmask);
-        // Box violations of Q_m and W - PT_m(Q_m).
-#pragma unroll
-        for (int r = 0; r < 8; ++r) A[r] = ld(Q[(m - 1) * 64 + c * 8 + r]);
-        l = eigval8(A, c, gbase, gmask);
-        feas = fmax(feas, fmax(-l, l - 1.0));
-#pragma unroll
-        for (int r = 0; r < 8; ++r) A[r] = csub(ld(W[c * 8 + r]), ld(Q[(m - 1) * 64 + pt_src(r, c, m)]));
-        l = eigval8(A, c, gbase, gmask);
-        feas = fmax(feas, fmax(-l, l - 1.0));
+        const int at = c * 8 + r, pt = pt_src(r, c, m);
+        // Z_m and its partial transpose (dual bound), Q_m and W - PT_m(Q_m)
+        // (box violations).
+        if (kind < 2)
+            A[r] = zshift(m - 1, kind == 0 ? at : pt);
+        else if (kind == 2)
+            A[r] = ld(Q[(m - 1) * 64 + at]);
+        else
+            A[r] = csub(ld(W[at]), ld(Q[(m - 1) * 64 + pt]));
     }
-    feas = group_max(feas, gmask);
+    const double l = eigval8(A, c, gbase, gmask);
+    const double pos = group_sum(fmax(l, 0.0), gmask);
+    const double viol = group_max(fmax(-l, l - 1.0), gmask);
     if (c == 0)
     {
+        dual_part[g] = pos;
+        feas_part[g] = viol;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0)
+    {
+        const double p = s_primal;
+        double d = 0.0, feas = 0.0;
+        for (int i = 0; i < 12; ++i)
+        {
+            if (i % 4 < 2)
+                d -= dual_part[i];
+            else
+                feas = fmax(feas, feas_part[i]);
+        }
         const double gp = p - d;
         k.primal[prob] = p;
         k.dual[prob] = d;
@@ -603,20 +640,20 @@ int gmn_solve(const mipt_gb300_gmn_config &cfg, const double *h_rho, int count, 
                cfg.gap_tol, cfg.feas_tol, o, o + P, o + 2 * P, o + 3 * P, o + 4 * P, static_cast<int *>(rem.p),
                static_cast<const float *>(res.p), static_cast<float>(30.0 * std::max(cfg.gap_tol, cfg.feas_tol)),
                static_cast<int *>(nextc.p), static_cast<int *>(boff.p), std::max(1, cfg.check_every), 0};
-    const int blocks = static_cast<int>((P + kProbPerBlock - 1) / kProbPerBlock);
+    const int blocks = static_cast<int>((P + kIterProblems - 1) / kIterProblems);
     const int every = std::max(1, cfg.check_every);
     int it = 0;
-    const std::size_t smem = sizeof(C2<Real>) * 320 * kProbPerBlock;
+    const std::size_t smem = sizeof(C2<Real>) * kIterShared * kIterProblems;
     GMN_CUDA(cudaFuncSetAttribute(k_gmn_iterate<Real>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   static_cast<int>(smem)));
     while (it < cfg.max_iter)
     {
         const int n = std::min(every, cfg.max_iter - it);
-        k_gmn_iterate<Real><<<blocks, kThreads, smem>>>(a, n);
+        k_gmn_iterate<Real><<<blocks, kIterThreads, smem>>>(a, n);
         it += n;
         GMN_CUDA(cudaMemset(rem.p, 0, sizeof(int)));
         k.iter_now = it;
-        k_gmn_check<Real><<<blocks, kThreads>>>(k);
+        k_gmn_check<Real><<<count, kCheckThreads>>>(k);
         GMN_CUDA(cudaGetLastError());
         int remaining = 0;
         GMN_CUDA(cudaMemcpy(&remaining, rem.p, sizeof(int), cudaMemcpyDeviceToHost));
@@ -625,7 +662,7 @@ int gmn_solve(const mipt_gb300_gmn_config &cfg, const double *h_rho, int count, 
         {
             // Last pass: bounds for every state still uncertified.
             k.force = 1;
-            k_gmn_check<Real><<<blocks, kThreads>>>(k);
+            k_gmn_check<Real><<<count, kCheckThreads>>>(k);
             GMN_CUDA(cudaGetLastError());
         }
     }
