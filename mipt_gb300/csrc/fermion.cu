@@ -184,6 +184,9 @@ __global__ void __launch_bounds__(FF_THREADS)
             {
                 if (k == a || k == b) continue;
                 const Real uk = Ucol[k], vk = Vcol[k];
+                // Modes measured earlier in the layer (and those outside the
+                // light cone) have nothing to add.
+                if (uk == Real(0) && vk == Real(0)) continue;
                 for (int l = k + 1 + lane; l < M; l += 32)
                 {
                     if (l == a || l == b) continue;
@@ -210,15 +213,20 @@ __global__ void __launch_bounds__(FF_THREADS)
     }
 }
 
-// Batched FP64 C = alpha * A B + beta * D over square M x M matrices.
+// Batched FP64 C = alpha * A B + beta * D over square M x M matrices, at
+// GB300's FP64 rate. symmetric: A B is (G G of an exactly antisymmetric G, as
+// the first step gets it; entry (c, r) is the same sum of the same products as
+// (r, c)), so only the tiles on and below the diagonal are formed and the
+// others are their mirror images.
 constexpr int GT = 64;
 __global__ void __launch_bounds__(256) k_dgemm(int M, const double *__restrict__ A, const double *__restrict__ B,
                                                const double *__restrict__ D, double *__restrict__ C, double alpha,
-                                               double beta)
+                                               double beta, int symmetric)
 {
     __shared__ double As[16][GT + 1], Bs[16][GT + 1];
     const std::size_t off = static_cast<std::size_t>(blockIdx.z) * M * M;
     const int r0 = blockIdx.y * GT, c0 = blockIdx.x * GT;
+    if (symmetric && c0 > r0) return;
     const int tid = threadIdx.x, ty = tid / 16, tx = tid % 16;
     double acc[4][4] = {};
     for (int k0 = 0; k0 < M; k0 += 16)
@@ -242,9 +250,23 @@ __global__ void __launch_bounds__(256) k_dgemm(int M, const double *__restrict__
             if (r < M && c < M)
             {
                 const std::size_t e = off + static_cast<std::size_t>(r) * M + c;
-                C[e] = alpha * acc[i][j] + (D ? beta * D[e] : 0.0);
+                const double x = alpha * acc[i][j] + (D ? beta * D[e] : 0.0);
+                C[e] = x;
+                if (symmetric && r0 != c0) C[off + static_cast<std::size_t>(c) * M + r] = x;
             }
         }
+}
+
+// The product state of every trajectory: i gamma_{2j} gamma_{2j+1} = 1.
+template <typename Real> __global__ void k_ff_init(int M, Real *g, std::size_t n)
+{
+    const std::size_t per = static_cast<std::size_t>(M) * M;
+    for (std::size_t i = blockIdx.x * static_cast<std::size_t>(blockDim.x) + threadIdx.x; i < n;
+         i += static_cast<std::size_t>(gridDim.x) * blockDim.x)
+    {
+        const int e = static_cast<int>(i % per), r = e / M, c = e % M;
+        g[i] = (r ^ c) == 1 ? (r < c ? Real(1) : Real(-1)) : Real(0);
+    }
 }
 
 __global__ void k_f32_to_f64(const float *a, double *b, std::size_t n)
@@ -278,11 +300,14 @@ __global__ void k_antisym(int M, double *g64, float *g32, std::size_t count)
 
 // Entropy (bits) of a set of modes (mask over N <= 128 modes) from the FP64
 // covariance: S = -Gamma_M^2 assembled in shared memory, parallel-order real
-// Jacobi, S = 1/2 sum_i H2((1 + sqrt(mu_i))/2).
+// Jacobi, S = 1/2 sum_i H2((1 + sqrt(mu_i))/2). At GB300's FP64 rate (a round of
+// d = 128 is 2,048 warp instructions of 20 clocks), so rotations of pairs whose
+// entry is zero are left out: the modes measured in the last layer are exactly
+// decoupled from the others.
 struct FFEntJob
 {
     int traj;
-    int pad;
+    int out; // index of the entropy
     std::uint64_t mask[2];
 };
 
@@ -315,7 +340,7 @@ __global__ void __launch_bounds__(256) k_ff_entropy(int N, const double *__restr
     const int ld = d + 1;
     if (d == 0)
     {
-        if (tid == 0) out[blockIdx.x] = 0.0;
+        if (tid == 0) out[J.out] = 0.0;
         return;
     }
     const double *G = g64 + static_cast<std::size_t>(J.traj) * M * M;
@@ -401,6 +426,7 @@ __global__ void __launch_bounds__(256) k_ff_entropy(int N, const double *__restr
                 const int pi = w / d, k = w % d;
                 const int p = rp[pi], q = rq[pi];
                 const double c = rc[pi], s = rs[pi];
+                if (s == 0.0) continue; // no rotation (c = 1)
                 const double akp = Sm[k * ld + p], akq = Sm[k * ld + q];
                 Sm[k * ld + p] = c * akp - s * akq;
                 Sm[k * ld + q] = s * akp + c * akq;
@@ -411,6 +437,7 @@ __global__ void __launch_bounds__(256) k_ff_entropy(int N, const double *__restr
                 const int pi = w / d, k = w % d;
                 const int p = rp[pi], q = rq[pi];
                 const double c = rc[pi], s = rs[pi];
+                if (s == 0.0) continue;
                 const double apk = Sm[p * ld + k], aqk = Sm[q * ld + k];
                 Sm[p * ld + k] = c * apk - s * aqk;
                 Sm[q * ld + k] = s * apk + c * aqk;
@@ -436,7 +463,7 @@ __global__ void __launch_bounds__(256) k_ff_entropy(int N, const double *__restr
             if (1.0 - x > 1e-15) h -= (1.0 - x) * log2(1.0 - x);
             s += 0.5 * h;
         }
-        out[blockIdx.x] = fabs(s) < 1e-12 ? 0.0 : s;
+        out[J.out] = fabs(s) < 1e-12 ? 0.0 : s;
     }
 }
 
@@ -465,8 +492,8 @@ int purify(int M, int count, double *g64, double *tmp, double *tmp2, float *g32)
     dim3 grid((M + GT - 1) / GT, (M + GT - 1) / GT, count);
     for (int it = 0; it < 2; ++it)
     {
-        k_dgemm<<<grid, 256>>>(M, g64, g64, nullptr, tmp, 1.0, 0.0);      // tmp = G G
-        k_dgemm<<<grid, 256>>>(M, g64, tmp, g64, tmp2, 0.5, 1.5);         // tmp2 = (G tmp)/2 + 3G/2
+        k_dgemm<<<grid, 256>>>(M, g64, g64, nullptr, tmp, 1.0, 0.0, it == 0); // tmp = G G
+        k_dgemm<<<grid, 256>>>(M, g64, tmp, g64, tmp2, 0.5, 1.5, 0);      // tmp2 = (G tmp)/2 + 3G/2
         FF_CUDA(cudaGetLastError());
         FF_CUDA(cudaMemcpyAsync(g64, tmp2, sizeof(double) * M * M * count, cudaMemcpyDeviceToDevice));
     }
@@ -582,24 +609,12 @@ extern "C" int mipt_gb300_ff_run(const mipt_gb300_ff_config *cfg, const std::uin
     if (forced) FF_CUDA(cudaMemcpy(d_f.p, h_forced.data(), h_forced.size(), cudaMemcpyHostToDevice));
     FF_CUDA(cudaMemset(d_oc.p, 0, C * D * N));
     FF_CUDA(cudaMemset(d_pr.p, 0, sizeof(double) * C * D * N));
-    {
-        std::vector<double> g0(static_cast<std::size_t>(M) * M, 0.0);
-        for (int j = 0; j < N; ++j)
-        {
-            g0[(2 * j) * M + 2 * j + 1] = 1.0;
-            g0[(2 * j + 1) * M + 2 * j] = -1.0;
-        }
-        std::vector<float> g0f(g0.begin(), g0.end());
-        for (std::size_t b = 0; b < C; ++b)
-        {
-            if (fp64)
-                FF_CUDA(cudaMemcpy(d_g64.as<double>() + b * M * M, g0.data(), sizeof(double) * M * M,
-                                   cudaMemcpyHostToDevice));
-            else
-                FF_CUDA(cudaMemcpy(d_g32.as<float>() + b * M * M, g0f.data(), sizeof(float) * M * M,
-                                   cudaMemcpyHostToDevice));
-        }
-    }
+    const int cvt_blocks = static_cast<int>(std::min<std::size_t>((C * M * M + 255) / 256, 4096));
+    if (fp64)
+        k_ff_init<<<cvt_blocks, 256>>>(M, d_g64.as<double>(), C * M * M);
+    else
+        k_ff_init<<<cvt_blocks, 256>>>(M, d_g32.as<float>(), C * M * M);
+    FF_CUDA(cudaGetLastError());
     // Shared memory: the packed triangle (FP32 only), two columns, the
     // rotations and the group table.
     const std::size_t tri_bytes = rot_elem * (static_cast<std::size_t>(M) * (M - 1) / 2);
@@ -611,7 +626,6 @@ extern "C" int mipt_gb300_ff_run(const mipt_gb300_ff_config *cfg, const std::uin
         FF_CUDA(cudaFuncSetAttribute(k_ff_evolve<float>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      static_cast<int>(smem)));
     const int seg = cfg->repurify_every > 0 ? cfg->repurify_every : depth;
-    const int cvt_blocks = static_cast<int>(std::min<std::size_t>((C * M * M + 255) / 256, 4096));
     for (int t0 = 0; t0 < depth; t0 += seg)
     {
         const int t1 = std::min(depth, t0 + seg);
@@ -679,17 +693,31 @@ extern "C" int mipt_gb300_ff_run(const mipt_gb300_ff_config *cfg, const std::uin
     std::vector<double> ent(jobs.size(), 0.0);
     if (!jobs.empty())
     {
+        // One launch per size class (at most 8, 16, 32 or 64 modes): the matrix
+        // of a small block then leaves room for other CTAs on its SM.
+        auto modes = [](const FFEntJob &j) { return __builtin_popcountll(j.mask[0]) + __builtin_popcountll(j.mask[1]); };
+        for (std::size_t i = 0; i < jobs.size(); ++i) jobs[i].out = static_cast<int>(i);
+        std::stable_sort(jobs.begin(), jobs.end(), [&](const FFEntJob &x, const FFEntJob &y) { return modes(x) > modes(y); });
+        if (modes(jobs.front()) > 64) return api_fail(MIPT_GB300_E_INVALID, "entropy blocks above 64 modes are not supported");
         FF_CUDA(d_jobs.alloc(sizeof(FFEntJob) * jobs.size()));
         FF_CUDA(d_ent.alloc(sizeof(double) * jobs.size()));
         FF_CUDA(cudaMemcpy(d_jobs.p, jobs.data(), sizeof(FFEntJob) * jobs.size(), cudaMemcpyHostToDevice));
-        int dmax = 0;
-        for (const auto &j : jobs) dmax = std::max(dmax, 2 * (__builtin_popcountll(j.mask[0]) + __builtin_popcountll(j.mask[1])));
-        if (dmax > 128) return api_fail(MIPT_GB300_E_INVALID, "entropy blocks above 64 modes are not supported");
-        const std::size_t esm = sizeof(double) * std::max(1, dmax) * (std::max(1, dmax) + 1);
-        FF_CUDA(cudaFuncSetAttribute(k_ff_entropy, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(esm)));
-        k_ff_entropy<<<static_cast<int>(jobs.size()), 256, esm>>>(N, d_g64.as<double>(), d_jobs.as<FFEntJob>(),
-                                                                  d_ent.as<double>());
-        FF_CUDA(cudaGetLastError());
+        int begin = 0;
+        for (const int least : {33, 17, 9, 0})
+        {
+            const int end = static_cast<int>(std::partition_point(jobs.begin() + begin, jobs.end(),
+                                                                  [&](const FFEntJob &j) { return modes(j) >= least; }) -
+                                             jobs.begin());
+            if (end == begin) continue;
+            const std::size_t d = static_cast<std::size_t>(std::max(1, 2 * modes(jobs[begin])));
+            const std::size_t esm = sizeof(double) * d * (d + 1);
+            FF_CUDA(cudaFuncSetAttribute(k_ff_entropy, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         static_cast<int>(esm)));
+            k_ff_entropy<<<end - begin, 256, esm>>>(N, d_g64.as<double>(), d_jobs.as<FFEntJob>() + begin,
+                                                    d_ent.as<double>());
+            FF_CUDA(cudaGetLastError());
+            begin = end;
+        }
         FF_CUDA(cudaMemcpy(ent.data(), d_ent.p, sizeof(double) * ent.size(), cudaMemcpyDeviceToHost));
     }
     FF_CUDA(cudaDeviceSynchronize());
