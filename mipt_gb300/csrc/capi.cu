@@ -1432,12 +1432,13 @@ int mipt_gb300_engine_measure_layer(mipt_gb300_engine *e, const int *sites, int 
     const int kmax = default_tile_qubits(e->fp64);
     for (int c = 0; c < nchunks; ++c)
     {
+        const bool streams = hist_streams(e->n, kmax, kCoalesceQubits, M.chunk[c]);
         if (e->fp64)
             MG_CUDA(launch_hist<double>(static_cast<const Cx<double> *>(e->data()), 1, e->n, kmax, kCoalesceQubits, c,
-                                        e->col.as<Collapse>(), 1, e->meas.as<LayerMeas>(), 1, e->part.as<double>(), false, 0));
+                                        e->col.as<Collapse>(), 1, e->meas.as<LayerMeas>(), 1, e->part.as<double>(), streams, 0));
         else
             MG_CUDA(launch_hist<float>(static_cast<const Cx<float> *>(e->data()), 1, e->n, kmax, kCoalesceQubits, c,
-                                       e->col.as<Collapse>(), 1, e->meas.as<LayerMeas>(), 1, e->part.as<double>(), false, 0));
+                                       e->col.as<Collapse>(), 1, e->meas.as<LayerMeas>(), 1, e->part.as<double>(), streams, 0));
         MG_CUDA(launch_measure(1, e->n, nullptr, kmax, kCoalesceQubits, c, e->meas.as<LayerMeas>(), 1,
                                e->part.as<double>(), e->bins.as<double>(), kHistScratch, d_forced, 1,
                                e->col.as<Collapse>(), 1,
@@ -1824,10 +1825,8 @@ int upload_draws(mipt_gb300_batch *b, const std::vector<TrajectoryDraw> &draws, 
             {
                 M.uniform[cc] = d.uniforms[d.uniform_offset[t] + cc];
                 if (M.chunk[cc] >> ne) continue; // the parity chunk of a half-size state
-                PassGeom hg{};
-                histogram_geometry(ne, b->kmax, b->cmin, M.chunk[cc], hg);
-                for (int li = 0; li < hg.k; ++li)
-                    if ((M.chunk[cc] >> hg.pos[li]) & 1ull) b->direct_hist[static_cast<std::size_t>(t) * kMaxChunks + cc] = 0;
+                if (!hist_streams(ne, b->kmax, b->cmin, M.chunk[cc]))
+                    b->direct_hist[static_cast<std::size_t>(t) * kMaxChunks + cc] = 0;
             }
             hm[slot] = M;
             hf[slot] = forced ? forced[slot] : 0ull;

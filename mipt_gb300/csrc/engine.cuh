@@ -142,6 +142,11 @@ inline std::uint64_t nonlocal_mask(const PassGeom &g)
     return m;
 }
 
+// Whether the chunk's histogram can be summed while streaming (launch_hist's
+// `direct`): its sites inside a histogram tile are among the tile's nine lowest
+// bits, so each of 512 threads meets one bin only.
+bool hist_streams(int n, int kmax, int cmin, std::uint64_t chunk);
+
 template <typename Real>
 cudaError_t launch_hist(const Cx<Real> *states, int batch, int n, int kmax, int cmin, int chunk_index,
                         const Collapse *collapse_in, std::size_t collapse_stride, const LayerMeas *meas,
