@@ -724,6 +724,20 @@ int measure_collapse(void *state, int n, int q, double u, int *outcome, double *
 int default_tile_qubits(bool fp64) { return fp64 ? 13 : 14; }
 constexpr int kCoalesceQubits = 4;
 
+// Tile of a single state's passes: small enough that about 128 (FP64) or 64
+// (FP32) tiles spread over the SMs. At GB300's FP64 rate a 2^k tile takes
+// 2^k * 10 clocks per bond on its SM, so the one to eight tiles that 2^13
+// leaves up to n = 16 cost far more than the extra passes of smaller tiles: the
+// five bonds of an n = 10 FP64 layer took 101 us in one tile (the layer 189 us,
+// 119 us with this rule; n = 22 FP32 and larger are as before). Batches keep their
+// tuned tile whatever their size, so that a trajectory's rounding does not
+// depend on the batch.
+int engine_tile_qubits(int n, bool fp64)
+{
+    const int most = default_tile_qubits(fp64);
+    return std::min(most, fp64 ? std::max(8, n - 7) : std::max(10, n - 6));
+}
+
 // Bond lists of every colour of a batch geometry (1-D brickwork: even and odd
 // layers; lattice: four colours).
 std::vector<std::vector<Bond>> geometry_bonds(int n, int closed, int lx, int ly)
@@ -1352,7 +1366,7 @@ int mipt_gb300_engine_apply_bonds(mipt_gb300_engine *e, const int *pairs, int nb
     std::vector<PassPlan> plan;
     try
     {
-        plan = plan_layer(e->n, bonds, default_tile_qubits(e->fp64), kCoalesceQubits,
+        plan = plan_layer(e->n, bonds, engine_tile_qubits(e->n, e->fp64), kCoalesceQubits,
                           e->fp64 ? register_bits<double>() : register_bits<float>());
     }
     catch (const std::exception &ex)
