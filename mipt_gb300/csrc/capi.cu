@@ -265,7 +265,7 @@ __global__ void k_reset_layers(Collapse *col, LayerResult *res, std::size_t n)
 __global__ void k_scatter(const double *in, const int *idx, int n, double *out, int mode)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
+    if (i >= n || idx[i] < 0) return;
     const double v = in[i];
     out[idx[i]] = mode == 1 ? renyi2_from_purity(v) : v;
 }
@@ -281,11 +281,40 @@ struct EntReq
     int fermion;
     std::vector<int> kept;
     int out; // index into the output array
+    int out2 = -1; // order 1: where the same subsystem's Renyi-2 goes too (its rho is formed once), or -1
 };
+
+// The requests of one state with each Renyi-2 joined to the von Neumann
+// request of the same subsystem where both need rho (all but FP32 purities on
+// the tensor cores, which never form it); out and out2 index `reqs`.
+std::vector<EntReq> join_requests(const std::vector<EntReq> &reqs, int n, bool fp32)
+{
+    std::vector<EntReq> out;
+    std::vector<char> joined(reqs.size(), 0);
+    for (std::size_t i = 0; i < reqs.size(); ++i)
+    {
+        if (joined[i]) continue;
+        EntReq q = reqs[i];
+        q.out = static_cast<int>(i);
+        const int k = static_cast<int>(q.kept.size());
+        if (k > 0 && !(fp32 && gram_tc_supported(n, k)))
+            for (std::size_t j = i + 1; j < reqs.size() && q.out2 < 0; ++j)
+                if (!joined[j] && reqs[j].order != reqs[i].order && reqs[j].fermion == q.fermion &&
+                    reqs[j].kept == q.kept)
+                {
+                    joined[j] = 1;
+                    q.out = static_cast<int>(q.order == 1 ? i : j);
+                    q.out2 = static_cast<int>(q.order == 1 ? j : i);
+                    q.order = 1;
+                }
+        out.push_back(q);
+    }
+    return out;
+}
 
 struct Workspace
 {
-    DevBuf jobs, rho, scratch, vals, idx, eig, err, eig_err, rows, dims;
+    DevBuf jobs, rho, scratch, vals, idx, idx2, eig, err, eig_err, rows, dims;
     PinnedArena stage;
     // Host -> device copy of a small table through the pinned staging arena.
     cudaError_t upload(void *dst, const void *src, std::size_t bytes, cudaStream_t s)
@@ -428,12 +457,15 @@ int run_entropies(const Cx<Real> *states, int n, const std::vector<EntReq> &reqs
         {
             const std::size_t nb = std::min(per_launch, list.size() - b0);
             std::vector<GramJob> jobs(nb);
-            std::vector<int> idx(nb);
+            std::vector<int> idx(nb), idx2(nb);
+            bool both = false;
             for (std::size_t i = 0; i < nb; ++i)
             {
                 const EntReq *r = list[b0 + i];
                 jobs[i] = make_gram_job(r->traj, n, r->kept.data(), k, r->fermion != 0);
                 idx[i] = r->out;
+                idx2[i] = r->out2;
+                both = both || r->out2 >= 0;
             }
             MG_CUDA(ws.jobs.ensure(sizeof(GramJob) * nb));
             MG_CUDA(ws.idx.ensure(sizeof(int) * nb));
@@ -460,6 +492,15 @@ int run_entropies(const Cx<Real> *states, int n, const std::vector<EntReq> &reqs
             MG_CUDA(gram_rho<Real>(states, n, ws.jobs.as<GramJob>(), nbi, k, col, col_stride, ws.rho.as<double>(),
                                    ws.scratch.p, ws.scratch.bytes, s, large ? ws.dims.as<int>() : nullptr, many));
             launches += 2;
+            if (both)
+            {
+                // Renyi-2 of the same rho, before the eigensolver takes it.
+                MG_CUDA(ws.idx2.ensure(sizeof(int) * nb));
+                MG_CUDA(ws.upload(ws.idx2.p, idx2.data(), sizeof(int) * nb, s));
+                MG_CUDA(purity_of(ws.rho.as<double>(), d, nbi, ws.vals.as<double>(), s));
+                k_scatter<<<(nbi + 255) / 256, 256, 0, s>>>(ws.vals.as<double>(), ws.idx2.as<int>(), nbi, d_out, 1);
+                launches += 2;
+            }
             if (!vn)
             {
                 MG_CUDA(purity_of(ws.rho.as<double>(), d, nbi, ws.vals.as<double>(), s));
@@ -1005,6 +1046,23 @@ struct mipt_gb300_batch
     std::vector<int> sector, folded;
     bool per_point() const { return !obs_point.empty() || cfg.observe_every > 0; }
     std::vector<EntReq> reqs; // for one point, trajectory index filled per launch
+    // The requests of `count` trajectories at observation point `point` of `of`.
+    std::vector<EntReq> requests_at(int point, int of, int count) const
+    {
+        const std::vector<EntReq> one = join_requests(reqs, cfg.n_qubits, cfg.fp64 == 0);
+        std::vector<EntReq> all;
+        all.reserve(one.size() * count);
+        for (int i = 0; i < count; ++i)
+            for (EntReq q : one)
+            {
+                const int base = (i * of + point) * reqs_per_point;
+                q.traj = i;
+                q.out += base;
+                if (q.out2 >= 0) q.out2 += base;
+                all.push_back(std::move(q));
+            }
+        return all;
+    }
     int col_half_vn = -1, col_half_s2 = -1;
     std::vector<int> tmi_vn, tmi_s2; // 7 request slots (A,B,C,D,AB,AC,BC) per cyclic offset
     int tmi_cycles = 0;
@@ -2164,15 +2222,7 @@ int batch_execute(mipt_gb300_batch *b, cudaStream_t s)
         }
         if (b->reqs_per_point > 0)
         {
-            std::vector<EntReq> reqs;
-            for (int i = 0; i < count; ++i)
-                for (int r = 0; r < b->reqs_per_point; ++r)
-                {
-                    EntReq q = b->reqs[r];
-                    q.traj = i;
-                    q.out = (i * b->points + point) * b->reqs_per_point + r;
-                    reqs.push_back(q);
-                }
+            const std::vector<EntReq> reqs = b->requests_at(point, b->points, count);
             Mark m(b, K_OBS, s);
             const int rc = run_entropies<Real>(states, n, reqs, pending, pstride, b->ws, s, b->ent.as<double>(), L);
             if (rc) return rc;
@@ -2279,15 +2329,7 @@ int batch_execute(mipt_gb300_batch *b, cudaStream_t s)
     // collapse still pending (so the measured sites leave the Gram), parity-
     // sector states after their expansion.
     auto final_entropies = [&](const Collapse *fc, std::size_t fstride) -> int {
-        std::vector<EntReq> reqs;
-        for (int i = 0; i < count; ++i)
-            for (int r = 0; r < b->reqs_per_point; ++r)
-            {
-                EntReq q = b->reqs[r];
-                q.traj = i;
-                q.out = i * b->reqs_per_point + r;
-                reqs.push_back(q);
-            }
+        const std::vector<EntReq> reqs = b->requests_at(0, 1, count);
         Mark m(b, K_OBS, s);
         return run_entropies<Real>(states, n, reqs, fc, fstride, b->ws, s, b->ent.as<double>(), L);
     };
