@@ -158,11 +158,15 @@ __global__ void __launch_bounds__(kGramThreads)
            const Collapse *__restrict__ col, std::size_t col_stride, int splits, std::uint64_t kchunk, int mode,
            Acc *__restrict__ part_out, double *__restrict__ pur_out, int compact, int *__restrict__ dims_out)
 {
-    constexpr int TK = GramK<Real>::TK;
-    constexpr int KB = GramK<Real>::BITS;
+    // Staged operands: exact FP64 sums of FP32 states widen each amplitude once,
+    // here (a conversion takes the FP64 pipe as long as an FMA, and the inner
+    // loop would repeat it sixteen times).
+    using SReal = typename std::conditional<kMixed, Real, Acc>::type;
+    constexpr int TK = GramK<SReal>::TK;
+    constexpr int KB = GramK<SReal>::BITS;
     __shared__ GramJob J;
-    __shared__ Cx<Real> As[TK][TM + 1];
-    __shared__ Cx<Real> Bs[TK][TM + 1];
+    __shared__ Cx<SReal> As[TK][TM + 1];
+    __shared__ Cx<SReal> Bs[TK][TM + 1];
     __shared__ std::uint64_t roffA[TM], roffB[TM], crossA[TM], crossB[TM], elo[TK];
     __shared__ double red[kGramThreads / 32];
     __shared__ std::uint64_t s_fixed;
@@ -300,7 +304,16 @@ __global__ void __launch_bounds__(kGramThreads)
     __syncthreads();
 
     const Cx<Real> *psi = states + (static_cast<std::size_t>(J.traj) << n);
-    const int ty = tid / 16, tx = tid % 16;
+    // 4 x 4 entries per thread; a diagonal tile has only its 136 lower-triangle
+    // sub-blocks, dealt to the first five warps. (With the operands widened
+    // once: 34 launches of 64 FP32 Grams of up to 256 rows 102 -> 77 ms.)
+    int ty = tid / 16, tx = tid % 16;
+    bool active = true;
+    if (tr == tc)
+    {
+        active = tid < 136;
+        if (active) tile_coords(tid, ty, tx);
+    }
     // kMixed: products summed in FP32 runs of 2 * TK = 64 environment
     // columns, each run added to the FP64 totals (the reference's
     // mixed-precision sweep, cpp/include/mipt/cuda/reduce_sweep.cuh:59-96);
@@ -356,14 +369,15 @@ __global__ void __launch_bounds__(kGramThreads)
                 if (c0 + i < d)
                     vb = gather(psi, eo | roffB[i], cl, check, has_col, (__popcll(e & crossB[i]) & 1) != 0);
             }
-            As[kk][i] = va;
-            Bs[kk][i] = vb;
+            As[kk][i] = Cx<SReal>{static_cast<SReal>(va.re), static_cast<SReal>(va.im)};
+            Bs[kk][i] = Cx<SReal>{static_cast<SReal>(vb.re), static_cast<SReal>(vb.im)};
         }
         __syncthreads();
+        if (active)
 #pragma unroll 4
         for (int kk = 0; kk < TK; ++kk)
         {
-            Cx<Real> a[4], b[4];
+            Cx<SReal> a[4], b[4];
 #pragma unroll
             for (int i = 0; i < 4; ++i)
             {
@@ -394,7 +408,8 @@ __global__ void __launch_bounds__(kGramThreads)
         }
         if constexpr (kMixed)
         {
-            if (++run_chunks == kRunChunks || e0 + TK >= eend)
+            if (!active) ++run_chunks; // nothing to add
+            else if (++run_chunks == kRunChunks || e0 + TK >= eend)
             {
 #pragma unroll
                 for (int i = 0; i < 4; ++i)
@@ -441,7 +456,7 @@ __global__ void __launch_bounds__(kGramThreads)
             for (int j = 0; j < 4; ++j)
             {
                 const int r = r0 + ty * 4 + i, c = c0 + tx * 4 + j;
-                if (r < D && c < D && r >= c)
+                if (active && r < D && c < D && r >= c)
                 {
                     out[(static_cast<std::size_t>(r) * D + c) * 2] = accr[i][j];
                     out[(static_cast<std::size_t>(r) * D + c) * 2 + 1] = acci[i][j];
@@ -457,7 +472,7 @@ __global__ void __launch_bounds__(kGramThreads)
             for (int j = 0; j < 4; ++j)
             {
                 const int r = r0 + ty * 4 + i, c = c0 + tx * 4 + j;
-                if (r < d && c < d && r >= c)
+                if (active && r < d && c < d && r >= c)
                 {
                     const double w = (r == c) ? 1.0 : 2.0;
                     const double re = static_cast<double>(accr[i][j]), im = static_cast<double>(acci[i][j]);
