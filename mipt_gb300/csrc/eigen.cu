@@ -108,7 +108,7 @@ __device__ bool parts_barrier(unsigned *ctr, unsigned parts, unsigned &epoch, in
 __global__ void __launch_bounds__(kTriThreads)
     k_tridiag(double2 *__restrict__ mats, int d, double *__restrict__ diag, double *__restrict__ off, int parts,
               double2 *__restrict__ pglob, unsigned *__restrict__ bars, int *__restrict__ err,
-              const int *__restrict__ dims)
+              const int *__restrict__ dims, int least)
 {
     extern __shared__ double2 sh[];
     double2 *v = sh;     // Householder vector (length m)
@@ -127,6 +127,7 @@ __global__ void __launch_bounds__(kTriThreads)
     // Rows that hold data (the rest of the d x d block is zero: their
     // eigenvalues are 0). The row stride stays d.
     const int dm = dims != nullptr ? dims[mat] : d;
+    if (dm <= least) return; // k_tridiag_cluster's
 
     for (int j = 0; j + 1 < dm; ++j)
     {
@@ -266,17 +267,40 @@ __global__ void __launch_bounds__(kTriThreads)
 // What bounds it is the FP64 pipe (a warp instruction takes 20 clocks of an
 // SM, however many lanes are on), so whatever is not the sweep runs on as few
 // warps as hold data: the reflector's roots and divisions on one warp, sums on
-// the warps below row m. Measured against the reduction in global memory:
+// the warps below row m.
+// With a work list, a cluster takes either one matrix of more than 128 rows,
+// all its CTAs on it, or one smaller matrix per CTA: measured sites leave the
+// spectra of one batch at different sizes, and the launch lasted as long as
+// its few full-size ones took on four SMs each while most of the others idled
+// (34 launches of 64 matrices of up to 256 rows 259 -> 251 ms: full-size ones
+// are now one or two waves of clusters of eight).
+// Measured against the reduction in global memory, without the list:
 // 34 launches of 64 matrices of up to 256 rows 533 -> 259 ms, 48 launches of
 // 800 of up to 64 rows 156 -> 62 ms, one of 256 rows 5.4 -> 3.8 ms.
 template <int NCB, int THREADS>
 __global__ void __launch_bounds__(THREADS)
     k_tridiag_cluster(const double2 *__restrict__ mats, int d, double *__restrict__ diag, double *__restrict__ off,
-                      const int *__restrict__ dims)
+                      const int *__restrict__ dims, const int *__restrict__ list, int nb)
 {
     namespace cg = cooperative_groups;
     cg::cluster_group cluster = cg::this_cluster();
-    const int C = static_cast<int>(cluster.num_blocks()), r = static_cast<int>(cluster.block_rank());
+    int C = static_cast<int>(cluster.num_blocks()), r = static_cast<int>(cluster.block_rank());
+    int mat = blockIdx.x / C;
+    if (list != nullptr)
+    {
+        // list[0], list[1]: large and small matrices; the large ones from
+        // list[2] up, the small ones from list[nb + 1] down.
+        if (mat < list[0])
+            mat = list[2 + mat];
+        else
+        {
+            const int i = (mat - list[0]) * C + r;
+            if (i >= list[1]) return;
+            mat = list[nb + 1 - i];
+            C = 1;
+            r = 0;
+        }
+    }
     constexpr int NW = THREADS / 32;
     constexpr int HB = NCB < 4 ? NCB : 4; // column blocks in flight together, at most
     constexpr int NP = (32 * NCB + THREADS - 1) / THREADS;
@@ -288,7 +312,6 @@ __global__ void __launch_bounds__(THREADS)
     double2 *part = pivot + (C > 1 ? 2 * DS : 0);                 // [2][C][DS] every CTA's partial p (C > 1)
     double2 *rows = part + (C > 1 ? 2 * C * DS : 0);              // packed rows
     __shared__ double red[NW], s_nt, s_beta;
-    const int mat = blockIdx.x / C;
     const double2 *a = mats + static_cast<std::size_t>(mat) * d * d;
     double *dg = diag + static_cast<std::size_t>(mat) * d;
     double *of = off + static_cast<std::size_t>(mat) * d;
@@ -593,7 +616,29 @@ __global__ void __launch_bounds__(THREADS)
         of[dm - 1] = 0.0;
         for (int i = dm; i < d; ++i) dg[i] = of[i] = 0.0;
     }
-    cluster.sync(); // no CTA leaves while another may read its rows
+    if (C > 1) cluster.sync(); // no CTA leaves while another may write to it
+}
+
+// Work list of k_tridiag_cluster: matrices of at most kSmallRows rows, those of
+// up to kClusterRows, and (left out) larger ones. The order within a class is
+// not fixed; every matrix is reduced the same way whatever its place.
+constexpr int kSmallRows = 128, kClusterRows = 256;
+
+__global__ void __launch_bounds__(256) k_eig_list(const int *__restrict__ dims, int d, int nb, int *__restrict__ list)
+{
+    __shared__ int count[2];
+    if (threadIdx.x < 2) count[threadIdx.x] = 0;
+    __syncthreads();
+    for (int i = threadIdx.x; i < nb; i += blockDim.x)
+    {
+        const int dm = dims != nullptr ? dims[i] : d;
+        if (dm <= kSmallRows)
+            list[nb + 1 - atomicAdd(&count[1], 1)] = i;
+        else if (dm <= kClusterRows)
+            list[2 + atomicAdd(&count[0], 1)] = i;
+    }
+    __syncthreads();
+    if (threadIdx.x < 2) list[threadIdx.x] = count[threadIdx.x];
 }
 
 // Eigenvalues of every reduced matrix, one thread per eigenvalue (grid:
@@ -682,9 +727,12 @@ std::size_t cluster_smem(int d, int C, int warps)
 
 template <int NCB, int THREADS>
 cudaError_t launch_cluster(const double2 *rho, int d, int nb, int C, double *diag, double *off, cudaStream_t s,
-                           const int *dims)
+                           const int *dims, const int *list = nullptr)
 {
-    const std::size_t smem = cluster_smem(d, C, THREADS / 32);
+    // With a list, a CTA may also hold a small matrix by itself.
+    const std::size_t smem = std::max(cluster_smem(32 * NCB, C, THREADS / 32),
+                                      list ? cluster_smem(kSmallRows, 1, 0) + sizeof(double2) * (4 + THREADS / 32) * 32 * NCB
+                                           : std::size_t{0});
     cudaError_t e = cudaFuncSetAttribute(k_tridiag_cluster<NCB, THREADS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          static_cast<int>(smem));
     if (e != cudaSuccess) return e;
@@ -704,15 +752,15 @@ cudaError_t launch_cluster(const double2 *rho, int d, int nb, int C, double *dia
     at.val.clusterDim.y = at.val.clusterDim.z = 1;
     cfg.attrs = &at;
     cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, k_tridiag_cluster<NCB, THREADS>, rho, d, diag, off, dims);
+    return cudaLaunchKernelEx(&cfg, k_tridiag_cluster<NCB, THREADS>, rho, d, diag, off, dims, list, nb);
 }
 } // namespace
 
 std::size_t hermitian_eig_scratch_doubles(int d, int nb)
 {
     // diag and off (d each), p vectors (2 d), barrier counters (1 double
-    // each, used as unsigned).
-    return (4 * static_cast<std::size_t>(d) + 1) * nb;
+    // each, used as unsigned), the work list (nb + 2 ints).
+    return (4 * static_cast<std::size_t>(d) + 2) * nb + 1;
 }
 
 cudaError_t hermitian_eig_entropy(double *rho, int d, int nb, double *entropy_out, double *eig_out, double *scratch,
@@ -725,26 +773,42 @@ cudaError_t hermitian_eig_entropy(double *rho, int d, int nb, double *entropy_ou
     double *off = scratch + static_cast<std::size_t>(d) * nb;
     double2 *pglob = reinterpret_cast<double2 *>(scratch + 2 * static_cast<std::size_t>(d) * nb);
     unsigned *bars = reinterpret_cast<unsigned *>(scratch + 4 * static_cast<std::size_t>(d) * nb);
+    int *list = reinterpret_cast<int *>(scratch + (4 * static_cast<std::size_t>(d) + 1) * nb);
+    int kernels = 0;
     int dev = 0, sms = 0;
     cudaError_t e = cudaSuccess;
     if (cudaGetDevice(&dev) != cudaSuccess ||
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0)
         sms = 152;
-    if (d <= 256)
+    const double2 *r2 = reinterpret_cast<const double2 *>(rho);
+    if (d <= 128)
     {
-        // The smallest cluster whose shared memory holds the matrix (four CTAs
-        // for 256 rows, else one); more CTAs, down to 16 rows each, while SMs
+        // One CTA holds the matrix; more, down to 16 rows each, while SMs
         // would stay idle.
-        int C = d > 128 ? 4 : 1;
+        int C = 1;
         while (C < 16 && nb * C * 2 <= sms && d / (2 * C) >= 16) C *= 2;
-        const double2 *r2 = reinterpret_cast<const double2 *>(rho);
-        e = d <= 32    ? launch_cluster<1, 32>(r2, d, nb, C, diag, off, s, dims)
-            : d == 64  ? launch_cluster<2, 128>(r2, d, nb, C, diag, off, s, dims)
-            : d == 128 ? launch_cluster<4, 256>(r2, d, nb, C, diag, off, s, dims)
-                       : launch_cluster<8, 256>(r2, d, nb, C, diag, off, s, dims);
+        e = d <= 32   ? launch_cluster<1, 32>(r2, d, nb, C, diag, off, s, dims)
+            : d == 64 ? launch_cluster<2, 128>(r2, d, nb, C, diag, off, s, dims)
+                      : launch_cluster<4, 256>(r2, d, nb, C, diag, off, s, dims);
+        ++kernels;
     }
-    else
+    else if (d == 256 && nb * 16 <= sms)
     {
+        e = launch_cluster<8, 256>(r2, d, nb, 16, diag, off, s, dims);
+        ++kernels;
+    }
+    else if (d == 256 || dims != nullptr)
+    {
+        k_eig_list<<<1, 256, 0, s>>>(dims, d, nb, list);
+        e = cudaGetLastError();
+        if (e == cudaSuccess) e = launch_cluster<8, 256>(r2, d, nb, 8, diag, off, s, dims, list);
+        kernels += 2;
+    }
+    if (e != cudaSuccess) return e;
+    if (d > 256)
+    {
+        int least = dims != nullptr ? kClusterRows : 0;
+        ++kernels;
         const std::size_t smem = 2 * sizeof(double2) * d;
         e = cudaFuncSetAttribute(k_tridiag, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
         if (e != cudaSuccess) return e;
@@ -763,14 +827,14 @@ cudaError_t hermitian_eig_entropy(double *rho, int d, int nb, double *entropy_ou
             e = cudaMemsetAsync(bars, 0, sizeof(unsigned) * nb, s);
             if (e != cudaSuccess) return e;
             int dd = d;
-            void *args[] = {&rho, &dd, &diag, &off, &parts, &pglob, &bars, &err, &dims};
+            void *args[] = {&rho, &dd, &diag, &off, &parts, &pglob, &bars, &err, &dims, &least};
             e = cudaLaunchCooperativeKernel(reinterpret_cast<const void *>(&k_tridiag), dim3(nb * parts),
                                             dim3(kTriThreads), args, smem, s);
         }
         else
         {
             k_tridiag<<<nb, kTriThreads, smem, s>>>(reinterpret_cast<double2 *>(rho), d, diag, off, 1, nullptr, nullptr,
-                                                    err, dims);
+                                                    err, dims, least);
             e = cudaGetLastError();
         }
     }
@@ -787,7 +851,7 @@ cudaError_t hermitian_eig_entropy(double *rho, int d, int nb, double *entropy_ou
     double *terms = reinterpret_cast<double *>(pglob);
     k_tridiag_sturm<<<dim3(nb, chunks), tpb, sm, s>>>(diag, off, d, terms, entropy_out, err, dims, eig_out != nullptr);
     e = cudaGetLastError();
-    if (launched) *launched = chunks == 1 ? 2 : 3;
+    if (launched) *launched = kernels + (chunks == 1 ? 1 : 2);
     if (e != cudaSuccess || chunks == 1) return e;
     k_entropy_sum<<<nb, 128, 0, s>>>(terms, d, entropy_out);
     return cudaGetLastError();
