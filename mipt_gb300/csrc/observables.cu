@@ -1273,7 +1273,9 @@ int gram_splits(int n, int k, int njobs, bool rho)
     }
     const std::uint64_t E = 1ull << (n - k);
     const int tiles = gram_tiles(k) * njobs;
-    while (tiles * splits < 2 * 152 && E / (2ull * splits) >= static_cast<std::uint64_t>(TK) * 8) splits *= 2;
+    // At least 64 columns per split: one n = 16 half cut (ten tiles of 256
+    // columns) ran on ten SMs for 1.1 ms with 256.
+    while (tiles * splits < 2 * 152 && E / (2ull * splits) >= 64) splits *= 2;
     return splits;
 }
 } // namespace
