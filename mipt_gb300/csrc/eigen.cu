@@ -38,7 +38,6 @@
 #include <algorithm>
 #include <cmath>
 #include <cstdint>
-#include <type_traits>
 
 namespace mg
 {
@@ -256,27 +255,33 @@ __global__ void __launch_bounds__(kTriThreads)
 // of C CTAs per matrix, CTA r holding the lower-triangle rows i = r (mod C)
 // packed. Rows are eliminated from the last one up, so the block that is left
 // always starts at row and column 0 (aligned with the lanes) and the row that
-// gives the next reflector lies in one CTA. One sweep over the lower triangle per step
-// applies the previous step's rank-2 update and accumulates p = B v for this
-// one, from each entry both as B_ik and as conj(B_ki): sixteen FP64 FMAs per
-// entry read and written once. A lane owns columns k = lane (mod 32): the
-// column sums stay in registers over a warp's rows, and the row sums of two
-// rows share one six-add shuffle tree. CTAs exchange their partial p once per
-// step, behind one cluster barrier; the partials alternate between two
-// buffers, so a CTA that runs ahead never overwrites what another still reads.
+// gives the next reflector lies in one CTA. One sweep over the lower triangle
+// per step applies the previous step's rank-2 update and accumulates p = B v
+// for this one, from each entry both as B_ik and as conj(B_ki): sixteen FP64
+// FMAs per entry read and written once. A lane owns columns k = lane (mod 32):
+// the column sums stay in registers over a warp's rows, and the row sums of
+// two rows share one six-add shuffle tree.
+// The partial p and the next pivot row go round the cluster in two steps, each
+// behind a cluster barrier: every CTA sends each other one its part of a
+// segment of the columns, and the segment's CTA sends the sums to all. Remote
+// traffic is slow: sixteen CTAs that each sent everything to everyone spent
+// 13k of a step's 31.5k clocks on it, and a remote load takes about 800.
 // What bounds it is the FP64 pipe (a warp instruction takes 20 clocks of an
 // SM, however many lanes are on), so whatever is not the sweep runs on as few
 // warps as hold data: the reflector's roots and divisions on one warp, sums on
-// the warps below row m.
+// the warps below row m. Of a step of a 256-row matrix on sixteen CTAs the
+// sweep and its column sums take about half, the reflector a fifth, the
+// exchange a fifth.
 // With a work list, a cluster takes either one matrix of more than 128 rows,
 // all its CTAs on it, or one smaller matrix per CTA: measured sites leave the
 // spectra of one batch at different sizes, and the launch lasted as long as
 // its few full-size ones took on four SMs each while most of the others idled
 // (34 launches of 64 matrices of up to 256 rows 259 -> 251 ms: full-size ones
 // are now one or two waves of clusters of eight).
-// Measured against the reduction in global memory, without the list:
-// 34 launches of 64 matrices of up to 256 rows 533 -> 259 ms, 48 launches of
-// 800 of up to 64 rows 156 -> 62 ms, one of 256 rows 5.4 -> 3.8 ms.
+// Measured against the reduction in global memory: 34 launches of 64 matrices
+// of up to 256 rows 533 -> 228 ms, 48 launches of 800 of up to 64 rows
+// 156 -> 57 ms, one of 256 rows 5.4 -> 3.4 ms. (Before the exchange by segments
+// and the single instance of the block's code: 251, 62 and 3.8 ms.)
 template <int NCB, int THREADS>
 __global__ void __launch_bounds__(THREADS)
     k_tridiag_cluster(const double2 *__restrict__ mats, int d, double *__restrict__ diag, double *__restrict__ off,
@@ -302,15 +307,16 @@ __global__ void __launch_bounds__(THREADS)
         }
     }
     constexpr int NW = THREADS / 32;
-    constexpr int HB = NCB < 4 ? NCB : 4; // column blocks in flight together, at most
     constexpr int NP = (32 * NCB + THREADS - 1) / THREADS;
     extern __shared__ __align__(16) double2 csm[];
     constexpr int DS = 32 * NCB;                                  // >= d; every lane may read a vector
     double2 *v = csm, *vp = v + DS, *wp = vp + DS, *prow = wp + DS; // reflector, previous v and w, row sums
     double2 *pcw = prow + DS;                                     // [NW][DS] column sums per warp
-    double2 *pivot = pcw + NW * DS;                               // [2][DS] pivot rows (C > 1)
-    double2 *part = pivot + (C > 1 ? 2 * DS : 0);                 // [2][C][DS] every CTA's partial p (C > 1)
-    double2 *rows = part + (C > 1 ? 2 * C * DS : 0);              // packed rows
+    // C > 1: the pivot row, p, and this CTA's segment of both as it comes in
+    // ([C][segment] partial p) and as it goes out.
+    double2 *pivot = pcw + NW * DS, *pfull = pivot + DS, *part = pfull + DS, *rowseg = part + DS + 16;
+    double2 *pseg = rowseg + DS / 2;
+    double2 *rows = C > 1 ? pseg + DS / 2 : pcw + NW * DS;        // packed rows
     __shared__ double red[NW], s_nt, s_beta;
     const double2 *a = mats + static_cast<std::size_t>(mat) * d * d;
     double *dg = diag + static_cast<std::size_t>(mat) * d;
@@ -338,19 +344,16 @@ __global__ void __launch_bounds__(THREADS)
         for (int k = lane; k <= i; k += 32) rows[row_at(li, r) + k] = a[static_cast<std::size_t>(i) * d + k];
     }
     for (int k = tid; k < DS; k += THREADS) v[k] = vp[k] = wp[k] = make_double2(0.0, 0.0);
-    // Row i to every CTA's pivot buffer (its owner calls it).
-    auto push_row = [&](int i, int buf) {
-        const double2 *src = rows + row_at(i / C, r);
-        for (int k = tid; k <= i; k += THREADS)
-        {
-            const double2 t = src[k];
-            for (int q = 0; q < C; ++q) cluster.map_shared_rank(pivot + buf * DS, q)[k] = t;
-        }
-    };
     if (C > 1)
     {
+        // The first pivot row goes to every CTA.
         __syncthreads();
-        if ((dm - 1) % C == r) push_row(dm - 1, dm & 1);
+        if ((dm - 1) % C == r)
+            for (int k = tid; k < dm; k += THREADS)
+            {
+                const double2 t = rows[row_at((dm - 1) / C, r) + k];
+                for (int q = 0; q < C; ++q) cluster.map_shared_rank(pivot, q)[k] = t;
+            }
         cluster.sync();
     }
     else
@@ -359,7 +362,7 @@ __global__ void __launch_bounds__(THREADS)
     for (int m = dm - 1; m >= 1; --m)
     {
         // Row m with the previous update applied; x = its conjugate transpose.
-        const double2 *rm = C > 1 ? pivot + ((m + 1) & 1) * DS : rows + row_at(m, 0);
+        const double2 *rm = C > 1 ? pivot : rows + row_at(m, 0);
         const int aw = (m + 31) / 32 < NW ? (m + 31) / 32 : NW; // warps with an entry below m
         if (warp < aw)
         {
@@ -443,68 +446,43 @@ __global__ void __launch_bounds__(THREADS)
             const int ic = i1 < 0 ? i0 : i1;
             const double2 v1 = v[ic], vp1 = vp[ic], wp1 = wp[ic];
             double s0r = 0.0, s0i = 0.0, s1r = 0.0, s1i = 0.0;
-            // N column blocks from c0 on: independent chains for the 64-clock
-            // latency, and no block that the row pair does not reach.
-            auto blocks = [&](auto first, auto count) {
-                constexpr int c0 = decltype(first)::value, N = decltype(count)::value;
-                double ar[2][N], ai[2][N];
+            // One instance of the block's code per column block (a variant per
+            // block count let more of them overlap, but the code outgrew the
+            // instruction cache: 3.6 ms for one 256-row matrix against 3.4).
 #pragma unroll
-                for (int cc = 0; cc < N; ++cc)
-                {
-                    const int c = c0 + cc, k = 32 * c + lane;
-                    const double2 vk = v[k], vpk = vp[k], wpk = wp[k];
-                    // Entries past the diagonal load and add zeros.
-                    auto entry = [&](double2 *q, int i, double2 vi, double2 vpi, double2 wpi, double &sr, double &si) {
-                        double2 b = make_double2(0.0, 0.0);
-                        if (k <= i) b = q[k];
-                        b.x = fma(-vpi.x, wpk.x, b.x);
-                        b.x = fma(-vpi.y, wpk.y, b.x);
-                        b.x = fma(-wpi.x, vpk.x, b.x);
-                        b.x = fma(-wpi.y, vpk.y, b.x);
-                        b.y = fma(-vpi.y, wpk.x, b.y);
-                        b.y = fma(vpi.x, wpk.y, b.y);
-                        b.y = fma(-wpi.y, vpk.x, b.y);
-                        b.y = fma(wpi.x, vpk.y, b.y);
-                        b.x = k <= i ? b.x : 0.0;
-                        b.y = k < i ? b.y : 0.0;
-                        if (k <= i) q[k] = b;
-                        sr = b.x * vk.x;
-                        sr = fma(-b.y, vk.y, sr);
-                        si = b.x * vk.y;
-                        si = fma(b.y, vk.x, si);
-                        const double bx = k < i ? b.x : 0.0;
-                        pc[c].x = fma(bx, vi.x, pc[c].x);
-                        pc[c].x = fma(b.y, vi.y, pc[c].x);
-                        pc[c].y = fma(bx, vi.y, pc[c].y);
-                        pc[c].y = fma(-b.y, vi.x, pc[c].y);
-                    };
-                    entry(q0, i0, v0, vp0, wp0, ar[0][cc], ai[0][cc]);
-                    entry(q1, i1, v1, vp1, wp1, ar[1][cc], ai[1][cc]);
-                }
-#pragma unroll
-                for (int cc = 0; cc < N; ++cc)
-                {
-                    s0r += ar[0][cc];
-                    s0i += ai[0][cc];
-                    s1r += ar[1][cc];
-                    s1i += ai[1][cc];
-                }
-            };
-            const int nblk = (ic >> 5) + 1;
-            using std::integral_constant;
-            auto tail = [&](auto first, int left) {
-                if (left == 1)
-                    blocks(first, integral_constant<int, 1>{});
-                else if (HB >= 2 && left == 2)
-                    blocks(first, integral_constant<int, (HB >= 2 ? 2 : 1)>{});
-                else if (HB >= 3 && left == 3)
-                    blocks(first, integral_constant<int, (HB >= 3 ? 3 : 1)>{});
-                else
-                    blocks(first, integral_constant<int, HB>{});
-            };
-            tail(integral_constant<int, 0>{}, nblk < HB ? nblk : HB);
-            if constexpr (NCB > HB)
-                if (nblk > HB) tail(integral_constant<int, HB>{}, nblk - HB);
+            for (int c = 0; c < NCB; ++c)
+            {
+                if (32 * c > ic) break;
+                const int k = 32 * c + lane;
+                const double2 vk = v[k], vpk = vp[k], wpk = wp[k];
+                // Entries past the diagonal load and add zeros.
+                auto entry = [&](double2 *q, int i, double2 vi, double2 vpi, double2 wpi, double &sr, double &si) {
+                    double2 b = make_double2(0.0, 0.0);
+                    if (k <= i) b = q[k];
+                    b.x = fma(-vpi.x, wpk.x, b.x);
+                    b.x = fma(-vpi.y, wpk.y, b.x);
+                    b.x = fma(-wpi.x, vpk.x, b.x);
+                    b.x = fma(-wpi.y, vpk.y, b.x);
+                    b.y = fma(-vpi.y, wpk.x, b.y);
+                    b.y = fma(vpi.x, wpk.y, b.y);
+                    b.y = fma(-wpi.y, vpk.x, b.y);
+                    b.y = fma(wpi.x, vpk.y, b.y);
+                    b.x = k <= i ? b.x : 0.0;
+                    b.y = k < i ? b.y : 0.0;
+                    if (k <= i) q[k] = b;
+                    sr = fma(b.x, vk.x, sr);
+                    sr = fma(-b.y, vk.y, sr);
+                    si = fma(b.x, vk.y, si);
+                    si = fma(b.y, vk.x, si);
+                    const double bx = k < i ? b.x : 0.0;
+                    pc[c].x = fma(bx, vi.x, pc[c].x);
+                    pc[c].x = fma(b.y, vi.y, pc[c].x);
+                    pc[c].y = fma(bx, vi.y, pc[c].y);
+                    pc[c].y = fma(-b.y, vi.x, pc[c].y);
+                };
+                entry(q0, i0, v0, vp0, wp0, s0r, s0i);
+                entry(q1, i1, v1, vp1, wp1, s1r, s1i);
+            }
             // Four sums over the warp: value (lane >> 3) ends in its lanes.
             const bool up = lane & 16, up2 = lane & 8;
             double x = up ? s1r : s0r, y = up ? s1i : s0i;
@@ -551,30 +529,44 @@ __global__ void __launch_bounds__(THREADS)
         }
         if (C > 1)
         {
-            double2 *mine = part + ((m & 1) * C + r) * DS;
+            const int seg = (m + C - 1) / C; // columns r * seg .. of CTA r
+            const bool owner = (m - 1) % C == r;
+            const double2 *next = rows + row_at((m - 1) / C, r);
 #pragma unroll
             for (int u = 0; u < NP; ++u)
             {
                 const int k = u * THREADS + tid;
                 if (k >= m) continue;
-                for (int q = 0; q < C; ++q) cluster.map_shared_rank(mine, q)[k] = p[u];
+                const int q = k / seg, e = k - q * seg;
+                cluster.map_shared_rank(part, q)[r * seg + e] = p[u];
+                if (owner) cluster.map_shared_rank(rowseg, q)[e] = next[k];
             }
-            if ((m - 1) % C == r) push_row(m - 1, m & 1);
             cluster.sync();
-            const double2 *all = part + (m & 1) * C * DS;
-#pragma unroll
-            for (int u = 0; u < NP; ++u)
+            if (tid < seg && r * seg + tid < m)
             {
-                const int k = u * THREADS + tid;
-                p[u] = make_double2(0.0, 0.0);
-                if (k >= m) continue;
+                double2 a0 = make_double2(0.0, 0.0), a1 = a0;
                 for (int q = 0; q < C; q += 2)
                 {
-                    const double2 t0 = all[q * DS + k], t1 = all[(q + 1) * DS + k];
-                    p[u].x += t0.x + t1.x;
-                    p[u].y += t0.y + t1.y;
+                    const double2 t0 = part[q * seg + tid], t1 = part[(q + 1) * seg + tid];
+                    a0.x += t0.x;
+                    a0.y += t0.y;
+                    a1.x += t1.x;
+                    a1.y += t1.y;
                 }
+                pseg[tid] = make_double2(a0.x + a1.x, a0.y + a1.y);
             }
+            __syncthreads();
+            for (int t = tid; t < seg * C; t += THREADS)
+            {
+                const int q = t / seg, e = t - q * seg, k = r * seg + e;
+                if (k >= m) continue;
+                cluster.map_shared_rank(pfull, q)[k] = pseg[e];
+                cluster.map_shared_rank(pivot, q)[k] = rowseg[e];
+            }
+            cluster.sync();
+#pragma unroll
+            for (int u = 0; u < NP; ++u)
+                if (u * THREADS + tid < m) p[u] = pfull[u * THREADS + tid];
         }
         const double beta = s_beta;
         // p = beta B v, K = beta/2 Re(v^H p) (real for Hermitian B), w = p - K v.
@@ -720,9 +712,9 @@ __global__ void __launch_bounds__(128) k_entropy_sum(const double *__restrict__ 
 // Shared memory of k_tridiag_cluster for d rows over C CTAs.
 std::size_t cluster_smem(int d, int C, int warps)
 {
-    const int lr = d / C, vectors = 4 + warps + (C > 1 ? 2 + 2 * C : 0);
+    const int lr = d / C, vectors = 4 + warps + (C > 1 ? 4 : 0);
     const std::size_t packed = static_cast<std::size_t>(lr) * C + static_cast<std::size_t>(C) * lr * (lr - 1) / 2;
-    return sizeof(double2) * (packed + static_cast<std::size_t>(vectors) * std::max(d, 32));
+    return sizeof(double2) * (packed + static_cast<std::size_t>(vectors) * std::max(d, 32) + (C > 1 ? 16 : 0));
 }
 
 template <int NCB, int THREADS>
