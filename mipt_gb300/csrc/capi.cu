@@ -15,6 +15,7 @@
 #include <tuple>
 #include <mutex>
 #include <cmath>
+#include <cstddef>
 #include <cstring>
 #include <map>
 #include <memory>
@@ -983,6 +984,20 @@ int api_cuda_fail(cudaError_t e, const char *what) { return cuda_fail(e, what); 
 } // namespace mg
 
 // ======================================================================= engine
+namespace
+{
+// A measured layer of a single state on the device.
+struct EngineLayer
+{
+    Collapse col;
+    LayerMeas meas;
+    std::uint64_t forced;
+    LayerResult res;
+    int err;
+};
+constexpr std::size_t kEngineGateOffset = 256;
+} // namespace
+
 struct mipt_gb300_engine
 {
     bool fp64 = false;
@@ -990,7 +1005,7 @@ struct mipt_gb300_engine
     void *owned = nullptr;
     void *borrowed = nullptr;
     std::size_t owned_bytes = 0;
-    DevBuf gates, meas, col, res, part, bins, err;
+    DevBuf gates, ctl, part, bins; // gates: the error flag, then the matrices
     ~mipt_gb300_engine()
     {
         if (owned) cudaFree(owned);
@@ -1431,29 +1446,33 @@ int mipt_gb300_engine_apply_bonds(mipt_gb300_engine *e, const int *pairs, int nb
     {
         return fail(MIPT_GB300_E_INVALID, ex.what());
     }
-    MG_CUDA(e->err.ensure(sizeof(int) + sizeof(std::uint64_t)));
-    MG_CUDA(cudaMemset(e->err.p, 0, sizeof(int)));
+    // The error flag and the gates go up in one copy, and the flag's copy back
+    // is the wait for the passes: of a ten-qubit layer's 119 us, most went into such
+    // calls (95 with these and the measured layer's merged).
+    const std::size_t count = 32 * static_cast<std::size_t>(nb);
+    std::vector<unsigned char> up(kEngineGateOffset + count * (e->fp64 ? sizeof(double) : sizeof(float)));
     if (e->fp64)
-    {
-        MG_CUDA(e->gates.ensure(sizeof(double) * 32 * nb));
-        MG_CUDA(cudaMemcpy(e->gates.p, m, sizeof(double) * 32 * nb, cudaMemcpyHostToDevice));
-        for (const auto &p : plan)
-            MG_CUDA(launch_pass<double>(static_cast<Cx<double> *>(e->data()), 1, p, e->gates.as<Cx<double>>(), 0,
-                                        nullptr, 0, nullptr, 0, nullptr, 0, e->err.as<int>(), 0));
-    }
+        std::memcpy(up.data() + kEngineGateOffset, m, sizeof(double) * count);
     else
     {
-        std::vector<float> f(32 * static_cast<std::size_t>(nb));
-        for (std::size_t i = 0; i < f.size(); ++i) f[i] = static_cast<float>(m[i]);
-        MG_CUDA(e->gates.ensure(sizeof(float) * f.size()));
-        MG_CUDA(cudaMemcpy(e->gates.p, f.data(), sizeof(float) * f.size(), cudaMemcpyHostToDevice));
-        for (const auto &p : plan)
-            MG_CUDA(launch_pass<float>(static_cast<Cx<float> *>(e->data()), 1, p, e->gates.as<Cx<float>>(), 0, nullptr,
-                                       0, nullptr, 0, nullptr, 0, e->err.as<int>(), 0));
+        float *f = reinterpret_cast<float *>(up.data() + kEngineGateOffset);
+        for (std::size_t i = 0; i < count; ++i) f[i] = static_cast<float>(m[i]);
     }
-    MG_CUDA(cudaDeviceSynchronize());
+    MG_CUDA(e->gates.ensure(up.size()));
+    MG_CUDA(cudaMemcpy(e->gates.p, up.data(), up.size(), cudaMemcpyHostToDevice));
+    int *d_err = e->gates.as<int>();
+    const unsigned char *gates = e->gates.as<unsigned char>() + kEngineGateOffset;
+    for (const auto &p : plan)
+        if (e->fp64)
+            MG_CUDA(launch_pass<double>(static_cast<Cx<double> *>(e->data()), 1, p,
+                                        reinterpret_cast<const Cx<double> *>(gates), 0, nullptr, 0, nullptr, 0,
+                                        nullptr, 0, d_err, 0));
+        else
+            MG_CUDA(launch_pass<float>(static_cast<Cx<float> *>(e->data()), 1, p,
+                                       reinterpret_cast<const Cx<float> *>(gates), 0, nullptr, 0, nullptr, 0, nullptr,
+                                       0, d_err, 0));
     int err = 0;
-    MG_CUDA(cudaMemcpy(&err, e->err.p, sizeof(int), cudaMemcpyDeviceToHost));
+    MG_CUDA(cudaMemcpy(&err, d_err, sizeof(int), cudaMemcpyDeviceToHost));
     if (err) return fail(MIPT_GB300_E_INTERNAL, "tile load wait timed out");
     return 0;
 }
@@ -1486,45 +1505,46 @@ int mipt_gb300_engine_measure_layer(mipt_gb300_engine *e, const int *sites, int 
         M.chunk[c] = m;
         M.uniform[c] = uniforms[c];
     }
-    MG_CUDA(e->meas.ensure(sizeof(LayerMeas)));
-    MG_CUDA(e->col.ensure(sizeof(Collapse)));
-    MG_CUDA(e->res.ensure(sizeof(LayerResult)));
+    // Everything the layer starts from goes up in one copy, its result and
+    // error flag come back in one.
+    MG_CUDA(e->ctl.ensure(sizeof(EngineLayer)));
     MG_CUDA(e->part.ensure(sizeof(double) * kHistScratch));
     MG_CUDA(e->bins.ensure(sizeof(double) * kHistScratch));
-    MG_CUDA(e->err.ensure(sizeof(int) + sizeof(std::uint64_t)));
-    MG_CUDA(cudaMemcpy(e->meas.p, &M, sizeof(LayerMeas), cudaMemcpyHostToDevice));
-    std::uint64_t *d_forced = nullptr;
-    if (forced)
-    {
-        d_forced = reinterpret_cast<std::uint64_t *>(static_cast<char *>(e->err.p) + 8);
-        MG_CUDA(cudaMemcpy(d_forced, &forced_mask, sizeof(std::uint64_t), cudaMemcpyHostToDevice));
-    }
-    k_reset_layers<<<1, 32>>>(e->col.as<Collapse>(), e->res.as<LayerResult>(), 1);
-    MG_CUDA(cudaMemset(e->err.p, 0, sizeof(int)));
+    EngineLayer up{};
+    up.col.scale = 1.0;
+    up.forced = forced_mask;
+    up.meas = M;
+    MG_CUDA(cudaMemcpy(e->ctl.p, &up, sizeof(EngineLayer), cudaMemcpyHostToDevice));
+    EngineLayer *ctl = e->ctl.as<EngineLayer>();
+    const std::uint64_t *d_forced = forced ? &ctl->forced : nullptr;
     const int kmax = default_tile_qubits(e->fp64);
     for (int c = 0; c < nchunks; ++c)
     {
         const bool streams = hist_streams(e->n, kmax, kCoalesceQubits, M.chunk[c]);
         if (e->fp64)
             MG_CUDA(launch_hist<double>(static_cast<const Cx<double> *>(e->data()), 1, e->n, kmax, kCoalesceQubits, c,
-                                        e->col.as<Collapse>(), 1, e->meas.as<LayerMeas>(), 1, e->part.as<double>(), streams, 0));
+                                        &ctl->col, 1, &ctl->meas, 1, e->part.as<double>(), streams, 0));
         else
             MG_CUDA(launch_hist<float>(static_cast<const Cx<float> *>(e->data()), 1, e->n, kmax, kCoalesceQubits, c,
-                                       e->col.as<Collapse>(), 1, e->meas.as<LayerMeas>(), 1, e->part.as<double>(), streams, 0));
-        MG_CUDA(launch_measure(1, e->n, nullptr, kmax, kCoalesceQubits, c, e->meas.as<LayerMeas>(), 1,
+                                       &ctl->col, 1, &ctl->meas, 1, e->part.as<double>(), streams, 0));
+        MG_CUDA(launch_measure(1, e->n, nullptr, kmax, kCoalesceQubits, c, &ctl->meas, 1,
                                e->part.as<double>(), e->bins.as<double>(), kHistScratch, d_forced, 1,
-                               e->col.as<Collapse>(), 1,
-                               e->res.as<LayerResult>(), 1, e->err.as<int>(), 0));
+                               &ctl->col, 1,
+                               &ctl->res, 1, &ctl->err, 0));
     }
     if (e->fp64)
-        MG_CUDA(launch_collapse<double>(static_cast<Cx<double> *>(e->data()), 1ull << e->n, 1, e->col.as<Collapse>(), 1, 0));
+        MG_CUDA(launch_collapse<double>(static_cast<Cx<double> *>(e->data()), 1ull << e->n, 1, &ctl->col, 1, 0));
     else
-        MG_CUDA(launch_collapse<float>(static_cast<Cx<float> *>(e->data()), 1ull << e->n, 1, e->col.as<Collapse>(), 1, 0));
-    LayerResult r{};
-    int err = 0;
-    MG_CUDA(cudaMemcpy(&r, e->res.p, sizeof(LayerResult), cudaMemcpyDeviceToHost));
-    MG_CUDA(cudaMemcpy(&err, e->err.p, sizeof(int), cudaMemcpyDeviceToHost));
-    if (err) return fail(MIPT_GB300_E_NUMERIC, "measurement layer found a zero-norm state or no outcome with weight");
+        MG_CUDA(launch_collapse<float>(static_cast<Cx<float> *>(e->data()), 1ull << e->n, 1, &ctl->col, 1, 0));
+    struct
+    {
+        LayerResult r;
+        int err;
+    } back{};
+    static_assert(offsetof(EngineLayer, err) == offsetof(EngineLayer, res) + sizeof(LayerResult), "copied together");
+    MG_CUDA(cudaMemcpy(&back, &ctl->res, sizeof(LayerResult) + sizeof(int), cudaMemcpyDeviceToHost));
+    const LayerResult &r = back.r;
+    if (back.err) return fail(MIPT_GB300_E_NUMERIC, "measurement layer found a zero-norm state or no outcome with weight");
     if (outcomes)
         for (int i = 0; i < ns; ++i) outcomes[i] = static_cast<int>((r.outcome >> sites[i]) & 1ull);
     if (surprisal) *surprisal = r.surprisal;
