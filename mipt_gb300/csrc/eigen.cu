@@ -633,18 +633,18 @@ __global__ void __launch_bounds__(256) k_eig_list(const int *__restrict__ dims, 
     if (threadIdx.x < 2) list[threadIdx.x] = count[threadIdx.x];
 }
 
-// Eigenvalues of every reduced matrix, one thread per eigenvalue (grid:
-// matrices x chunks of blockDim eigenvalues), and the entropy terms
+// Eigenvalues of every reduced matrix, 2^gl threads per eigenvalue (grid:
+// matrices x chunks of blockDim threads), and the entropy terms
 // -lambda log2 lambda over lambda > 1e-15; with one chunk per matrix the sum
 // too. The implicit QL iteration that this replaces is one serial chain of
 // about d^2 plane rotations per matrix at GB300's 64-clock FP64 latency. The 34
 // launches of 64 matrices of up to 256 rows: QL 972 ms, this 43 ms; one matrix
-// of 256 rows: 1.4 to 20 ms, this 0.9 ms.
+// of 256 rows: 1.4 to 20 ms, this 0.33 ms.
 constexpr double kEigCutoff = 1e-15;
 
 __global__ void __launch_bounds__(128)
     k_tridiag_sturm(double *__restrict__ diag, const double *__restrict__ off, int d, double *__restrict__ terms,
-                    double *__restrict__ entropy, int *__restrict__ err, const int *__restrict__ dims, int want_all)
+                    double *__restrict__ entropy, int *__restrict__ err, const int *__restrict__ dims, int want_all, int gl)
 {
     extern __shared__ __align__(16) double2 de[];
     float2 *df = reinterpret_cast<float2 *>(de + d);
@@ -679,13 +679,16 @@ __global__ void __launch_bounds__(128)
         df[i] = sturm_entry32(de[i], inv, i);
     }
     __syncthreads();
-    const int idx = blockIdx.y * blockDim.x + threadIdx.x;
-    double term = 0.0;
-    if (finite && idx < dm)
+    const int at = blockIdx.y * blockDim.x + threadIdx.x, idx = at >> gl;
+    const bool writes = (at & ((1 << gl) - 1)) == 0;
+    const double bound = top * (1.0 + 1e-14), cutoff = want_all ? -2.0 * bound : kEigCutoff;
+    double term = 0.0, l = 0.0;
+    if (gl > 0 && finite && top > 0.0)
+        l = sturm_eigenvalue_lanes(de, df, dm, idx < dm ? idx : dm - 1, top, bound, cutoff, gl, idx < dm);
+    else if (finite && top > 0.0 && idx < dm)
+        l = sturm_eigenvalue(de, df, dm, idx, top, bound, cutoff);
+    if (finite && writes && idx < dm)
     {
-        const double bound = top * (1.0 + 1e-14);
-        const double l =
-            top > 0.0 ? sturm_eigenvalue(de, df, dm, idx, top, bound, want_all ? -2.0 * bound : kEigCutoff) : 0.0;
         if (want_all) diag[static_cast<std::size_t>(jb) * d + idx] = l;
         if (l > kEigCutoff) term = -l * log2(l);
     }
@@ -695,7 +698,7 @@ __global__ void __launch_bounds__(128)
         const double s = block_sum(term, red);
         if (threadIdx.x == 0) entropy[jb] = !finite ? NAN : (fabs(s) < 1e-12 ? 0.0 : s);
     }
-    else if (idx < d)
+    else if (writes && idx < d)
         terms[static_cast<std::size_t>(jb) * d + idx] = finite ? term : NAN;
 }
 
@@ -833,15 +836,23 @@ cudaError_t hermitian_eig_entropy(double *rho, int d, int nb, double *entropy_ou
     if (e != cudaSuccess) return e;
     // One thread per eigenvalue: CTAs of up to 128, or of one warp each while
     // that spreads a few matrices over idle SMs (two warps of one SM would
-    // share its FP64 pipe).
-    const int tpb = static_cast<long long>(nb) * ((d + 31) / 32) <= 2 * sms ? 32 : std::min(128, (d + 31) / 32 * 32);
-    const int chunks = (d + tpb - 1) / tpb;
+    // share its FP64 pipe). Four to 32 lanes per eigenvalue while the warps are
+    // still no more than the SMs: one matrix of 256 rows (16 lanes, 128 warps)
+    // 0.91 -> 0.33 ms. With more warps than that the FP64 pipes
+    // are busy, and one lane's search needs the fewest counts in all; two lanes
+    // would narrow a bracket only threefold per count.
+    int gl = 0;
+    while (gl < 5 && (static_cast<long long>(nb) * d << (gl + 1)) <= 32ll * sms) ++gl;
+    if (gl < 2) gl = 0;
+    const long long warps = static_cast<long long>(nb) * ((d + 31) / 32);
+    const int tpb = gl > 0 || warps <= 2 * sms ? 32 : std::min(128, (d + 31) / 32 * 32);
+    const int chunks = ((d << gl) + tpb - 1) / tpb;
     const std::size_t sm = (sizeof(double2) + sizeof(float2)) * d;
     e = cudaFuncSetAttribute(k_tridiag_sturm, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(sm));
     if (e != cudaSuccess) return e;
     // The terms take the place of the p vectors, which the reduction is done with.
     double *terms = reinterpret_cast<double *>(pglob);
-    k_tridiag_sturm<<<dim3(nb, chunks), tpb, sm, s>>>(diag, off, d, terms, entropy_out, err, dims, eig_out != nullptr);
+    k_tridiag_sturm<<<dim3(nb, chunks), tpb, sm, s>>>(diag, off, d, terms, entropy_out, err, dims, eig_out != nullptr, gl);
     e = cudaGetLastError();
     if (launched) *launched = kernels + (chunks == 1 ? 1 : 2);
     if (e != cudaSuccess || chunks == 1) return e;

@@ -82,7 +82,6 @@ bool compensated_rho_sums()
 }
 
 constexpr int TM = kGramTile;
-constexpr int TK = 32;
 constexpr int kGramThreads = 256;
 
 // K-step of the Gram tile: 32 environment columns for FP32 operands, 16 for

@@ -1,5 +1,5 @@
 // Eigenvalues of real symmetric tridiagonal matrices by Sturm counts, one
-// thread per eigenvalue.
+// thread per eigenvalue, or several where SMs would be idle.
 //
 // Givens' bisection on the number of sign changes of the leading principal
 // minors p_i(x) of T - x (p_i = (d_i - x) p_{i-1} - e_{i-1}^2 p_{i-2}):
@@ -191,6 +191,60 @@ __device__ __forceinline__ double sturm_eigenvalue(const double2 *__restrict__ d
                 x = static_cast<double>(sqrtf(static_cast<float>(lo)) * sqrtf(static_cast<float>(hi)));
         }
         probe(x, isolated);
+    }
+    return 0.5 * (lo + hi);
+}
+
+// The same by 2^gl neighbouring lanes: counts at 2^gl points of the bracket at
+// once (multisection) narrow it 2^gl + 1 fold, so with 16 lanes nine FP64
+// counts end a search, none of which depends on how p_d grows or on how many
+// eigenvalues the bracket holds. Every lane of the warp calls this; a group
+// without an eigenvalue to find (on = false) counts along.
+__device__ __forceinline__ double sturm_eigenvalue_lanes(const double2 *__restrict__ de, const float2 *__restrict__ df,
+                                                         int d, int index, double norm, double bound, double cutoff,
+                                                         int gl, bool on)
+{
+    const int G = 1 << gl, lane = threadIdx.x & 31, sub = lane & (G - 1);
+    const unsigned low = G == 32 ? 0xffffffffu : (1u << G) - 1u;
+    // The first lane of the group whose count is above `index`; G if none.
+    auto first_above = [&](bool above) {
+        const unsigned m = (__ballot_sync(0xffffffffu, above) >> (lane - sub)) & low;
+        return m ? __ffs(m) - 1 : G;
+    };
+    // As many rounds as narrow the FP32 bracket 2^20 fold.
+    float a = cutoff > 0.0 ? -1e-6f : -1.001f, b = 1.001f;
+    const float stepf = 1.f / static_cast<float>(G + 1);
+    for (float left = 1 << 20; left > 1.f; left *= stepf)
+    {
+        const float w = (b - a) * stepf;
+        const int f = first_above(sturm_count32(df, d, a + w * static_cast<float>(sub + 1)) > index);
+        b = f == G ? b : a + w * static_cast<float>(f + 1);
+        a = f == 0 ? a : a + w * static_cast<float>(f);
+    }
+    const double tol = 1.1102230246251565e-16 * norm;
+    double lo = -bound, hi = bound;
+    // First points over the FP32 bracket, its ends among them.
+    double x0 = (static_cast<double>(a) - kSturmSlack) * norm;
+    double dx = (static_cast<double>(b) + kSturmSlack) * norm;
+    if (x0 < cutoff) x0 = cutoff;
+    dx = dx > x0 ? (dx - x0) / static_cast<double>(G - 1) : 0.0;
+    const double step = 1.0 / static_cast<double>(G + 1);
+    for (int it = 0; it < 64; ++it)
+    {
+        if (!__any_sync(0xffffffffu, on)) break;
+        const int f = first_above(sturm_eval(de, d, fma(dx, static_cast<double>(sub), x0)).count > index);
+        const double nlo = f == 0 ? lo : fma(dx, static_cast<double>(f - 1), x0);
+        const double nhi = f == G ? hi : fma(dx, static_cast<double>(f), x0);
+        // Done at the tolerance, or where rounding keeps the bracket from narrowing.
+        const double w = nhi - nlo;
+        if (on)
+        {
+            on = !(nhi <= cutoff) && w > tol && (it == 0 || w < hi - lo);
+            lo = nlo;
+            hi = nhi;
+        }
+        dx = w * step;
+        x0 = lo + dx;
     }
     return 0.5 * (lo + hi);
 }

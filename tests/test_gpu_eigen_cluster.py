@@ -56,3 +56,9 @@ def test_batches(mg, orc, n, count, p):
     for i in (0, count // 2, count - 1):
         ref = orc.run_trajectory(int(seeds[i]), n, 2, p, True, 16, 1, 1)
         np.testing.assert_allclose(got[i], ref["obs"][:, 0], rtol=0, atol=1e-10)
+
+
+@pytest.mark.parametrize("n,count", [(6, 2), (10, 9), (10, 10), (12, 19), (12, 20), (16, 4), (16, 5)])
+def test_lanes_per_eigenvalue(mg, orc, n, count):
+    """Around the counts at which an eigenvalue is searched by 32 to 4 lanes or by one."""
+    test_batches(mg, orc, n, count, 0.15)
