@@ -328,7 +328,7 @@ def run_gb300(args):
         # launches (two layers: sparse, dense, sparse, dense) at 16
         # trajectories, 3.06 GB per launch on average = 191 MB per trajectory;
         # a launch streams each state it visits once, so it scales with the
-        # batch (profiles/k_pass_rounds_L24_traffic_batch16.md).
+        # batch (profiles/k_pass_quads_L24_traffic_batch16.md).
         traffic = PASS_TRAFFIC_PER_TRAJ * B
         roofline = {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
                     "traffic": traffic,

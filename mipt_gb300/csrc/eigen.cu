@@ -23,8 +23,8 @@
 //               interleaved re/im, the lower triangle read and updated) in
 //               global memory: one CTA per matrix, or several with barriers
 //               between them.
-//   k_tridiag_sturm  one thread per eigenvalue (tridiag.cuh), then the
-//               entropy.
+//   k_tridiag_sturm  one thread or a few lanes per eigenvalue (tridiag.cuh),
+//               then the entropy.
 //
 // All reductions run in a fixed order, so results are reproducible.
 // FP64 throughout: GB300's FP64 rate bounds the reduction at about 16/3 d^3
