@@ -491,7 +491,8 @@ int run_entropies(const Cx<Real> *states, int n, const std::vector<EntReq> &reqs
             const bool large = vn && d > jacobi_max_dim();
             if (large) MG_CUDA(ws.dims.ensure(sizeof(int) * nb));
             MG_CUDA(gram_rho<Real>(states, n, ws.jobs.as<GramJob>(), nbi, k, col, col_stride, ws.rho.as<double>(),
-                                   ws.scratch.p, ws.scratch.bytes, s, large ? ws.dims.as<int>() : nullptr, many));
+                                   ws.scratch.p, ws.scratch.bytes, s, many ? RhoUse::kPlainPurity : RhoUse::kSpectrum,
+                                   large ? ws.dims.as<int>() : nullptr));
             launches += 2;
             if (both)
             {
@@ -614,7 +615,7 @@ int compat_rdm(const void *state, int n, const int *kept, int k, int fermion, do
     MG_CUDA(c.ws.rho.ensure(sizeof(double) * 2 * d * d));
     MG_CUDA(c.ws.scratch.ensure(gram_scratch_bytes(n, k, 1, true)));
     MG_CUDA(gram_rho<Real>(static_cast<const Cx<Real> *>(state), n, c.ws.jobs.as<GramJob>(), 1, k, nullptr, 0,
-                           c.ws.rho.as<double>(), c.ws.scratch.p, c.ws.scratch.bytes, 0));
+                           c.ws.rho.as<double>(), c.ws.scratch.p, c.ws.scratch.bytes, 0, RhoUse::kEntries));
     MG_CUDA(cudaMemcpy(host_rho, c.ws.rho.p, sizeof(double) * 2 * d * d, cudaMemcpyDeviceToHost));
     return 0;
 }

@@ -1289,7 +1289,7 @@ std::size_t gram_scratch_bytes(int n, int k, int njobs, bool rho)
 template <typename Real>
 cudaError_t gram_rho(const Cx<Real> *states, int n, const GramJob *d_jobs, int njobs, int k,
                      const Collapse *collapse, std::size_t collapse_stride, double *rho_out, void *scratch,
-                     std::size_t scratch_bytes, cudaStream_t s, int *dims_out, bool plain_runs)
+                     std::size_t scratch_bytes, cudaStream_t s, RhoUse use, int *dims_out)
 {
     if (njobs <= 0) return cudaSuccess;
     const int splits = gram_splits(n, k, njobs, true);
@@ -1298,7 +1298,8 @@ cudaError_t gram_rho(const Cx<Real> *states, int n, const GramJob *d_jobs, int n
     const std::uint64_t E = 1ull << (n - k);
     const std::uint64_t kchunk = (E + splits - 1) / splits;
     dim3 grid(gram_tiles(k), splits, njobs);
-    const int compact = measured_compact_enabled() ? 1 : 0;
+    const int compact = use != RhoUse::kEntries && measured_compact_enabled() ? 1 : 0;
+    const bool plain_runs = use == RhoUse::kPlainPurity;
     // rho feeds -lambda log lambda: plain FP32 runs of 64 products left
     // about 5e-7 relative error in its entries, which moved the S_vN of
     // near-pure reduced states by up to 2e-5 at n = 20. FP32 states sum in
@@ -2542,7 +2543,7 @@ cudaError_t gram_purity_tc(const Cx<float> *states, int n, const GramJob *d_jobs
 
 #define MG_INST(R)                                                                                               \
     template cudaError_t gram_rho<R>(const Cx<R> *, int, const GramJob *, int, int, const Collapse *, std::size_t, \
-                                     double *, void *, std::size_t, cudaStream_t, int *, bool);                  \
+                                     double *, void *, std::size_t, cudaStream_t, RhoUse, int *);                \
     template cudaError_t gram_purity<R>(const Cx<R> *, int, const GramJob *, int, int, const Collapse *,          \
                                         std::size_t, double *, void *, std::size_t, cudaStream_t);               \
     template cudaError_t rho3_sweep<R>(const Cx<R> *, int, int, const int *, int, int, const Collapse *,          \

@@ -38,17 +38,28 @@ inline int gram_tiles(int k)
     return t * (t + 1) / 2;
 }
 
+// What a rho is wanted for. kEntries: the matrix itself, on the kept modes in
+// the caller's order. kSpectrum: its spectrum or purity only. kPlainPurity: its
+// purity only, and FP32 states' products may be summed in plain FP32 runs
+// (k <= 6).
+enum class RhoUse
+{
+    kEntries,
+    kSpectrum,
+    kPlainPurity
+};
+
 // rho for every job (all jobs share k): full FP64 d x d Hermitian matrices
-// written to rho_out[job][d][d] (row-major complex). With a pending collapse,
-// non-fermionic jobs leave out the sites it measured (the state is a product
-// on them, so the spectrum and purity are those of the reduced matrix): rho
-// then holds that 2^k' x 2^k' matrix in its leading rows and columns, zeros
-// elsewhere, and dims_out[job] (nullable) receives 2^k'. plain_runs: FP32
-// states' products may be summed in plain FP32 runs (purities; k <= 6 only).
+// written to rho_out[job][d][d] (row-major complex). Unless its entries are
+// wanted, a non-fermionic job leaves out the sites that a pending collapse
+// measured (the state is a product on them) and forms the matrix of the
+// smaller side, kept or environment (the same non-zero spectrum): rho_out then
+// holds that 2^k' x 2^k' matrix in its leading rows and columns, zeros
+// elsewhere, and dims_out[job] (nullable) receives 2^k'.
 template <typename Real>
 cudaError_t gram_rho(const Cx<Real> *states, int n, const GramJob *d_jobs, int njobs, int k,
                      const Collapse *collapse, std::size_t collapse_stride, double *rho_out, void *scratch,
-                     std::size_t scratch_bytes, cudaStream_t s, int *dims_out = nullptr, bool plain_runs = false);
+                     std::size_t scratch_bytes, cudaStream_t s, RhoUse use, int *dims_out = nullptr);
 
 // Purity Tr(rho^2) of every job without materialising rho.
 template <typename Real>
