@@ -23,6 +23,7 @@
 #include <cmath>
 #include <cstdlib>
 #include <cstring>
+#include <limits>
 #include <stdexcept>
 
 namespace mg
@@ -1003,7 +1004,7 @@ __global__ void __launch_bounds__(256) k_jacobi(const double *__restrict__ rho, 
 
 // ------------------------------------------------------------- three sites
 constexpr int R3_THREADS = 128;
-constexpr int R3_RUN = 16;      // environment columns per FP32 run
+constexpr int R3_RUN = 16;      // most environment columns per run
 constexpr int R3_VALUES = 72;   // re, im of the 36 lower-triangle entries
 constexpr int R3_GROUPS = 8;    // chunk groups of the final sum
 
@@ -1016,17 +1017,41 @@ __device__ __forceinline__ void comp_add(float x, float &s, float &c)
     s = t;
 }
 
+// x in FP64 by its bit pattern (a conversion takes the FP64 pipe 17 clocks a
+// warp); subnormal numbers, infinities and NaN are converted.
+__device__ __forceinline__ double widen(float x)
+{
+    const unsigned u = __float_as_uint(x), a = u & 0x7fffffffu;
+    if (a != 0u && a - 0x00800000u >= 0x7f000000u) return static_cast<double>(x);
+    const unsigned hi = (u & 0x80000000u) | (a != 0u ? (a >> 3) + 0x38000000u : 0u);
+    return __hiloint2double(static_cast<int>(hi), static_cast<int>(a << 29));
+}
+
+// Columns per run of the FP32 sums: at most 16, and no more than the 2^(n-3)
+// columns would give 256 threads (of 1 to 256 CTAs of 4096 columns or more),
+// each measured mode halving it, so that a plain FP32 run never grows at small
+// sizes or where a collapse leaves few columns.
+__device__ __forceinline__ int rho3_run(int n, int nfree)
+{
+    const int most = n <= 15 ? n - 11 : (n - 19 > 4 ? n - 19 : 4);
+    const int r = most - (n - 3 - nfree);
+    return 1 << (r < 0 ? 0 : (r > 4 ? 4 : r));
+}
+static_assert(R3_RUN == 1 << 4, "rho3_run");
+
 // One chunk of environment columns of one triple: each thread holds the
 // lower triangle of its columns' sum in registers. Sites that a pending
 // collapse measured keep their outcome, so only the matching columns are
 // visited; the scattered column counter advances by a masked increment.
-// FP32 states: sums of 16 columns in FP32 (packed FMAs) join a compensated
-// pair of FP32 numbers per value in shared memory, and the pairs are added
-// the same way over the threads: FP64 additions cost an SM 20 clocks a warp
-// (and FP32 -> FP64 conversions 17), so the former FP64 shuffle trees over 72
-// values per warp took most of the time. FP64 states: FP64 sums throughout.
+// FP32 states: sums of up to 16 columns in FP32 (packed FMAs) join a compensated
+// pair of FP32 numbers per value in shared memory; over the threads the pairs'
+// sums are added in FP64, their (small) compensations in FP32. FP64 additions
+// cost an SM 20 clocks a warp and FP32 -> FP64 conversions 17, so FP64 shuffle
+// trees over 72 values per warp took most of the time; eight lanes per value
+// and a widening by bit pattern need a tenth of those clocks. FP64 states: FP64
+// sums throughout, runs of 16 columns added to totals in shared memory.
 // Measured on GB300, 20 ring triples of an n = 20 FP32 state, the whole call:
-// 306 -> 88 us.
+// 310 -> 112 us (93 us with the threads' pairs added as FP32 pairs).
 template <typename Real>
 __global__ void __launch_bounds__(R3_THREADS)
     k_rho3(const Cx<Real> *__restrict__ states, int n, const int *__restrict__ subs, int fermion,
@@ -1099,9 +1124,13 @@ __global__ void __launch_bounds__(R3_THREADS)
 #pragma unroll
     for (int i = 0; i < 36; ++i) ar[i] = ai[i] = Real(0);
     float2 *pairs = reinterpret_cast<float2 *>(r3_smem) + tid;
-    if constexpr (kF32)
+    double *totals = r3_smem + tid;
 #pragma unroll 4
-        for (int t = 0; t < R3_VALUES; ++t) pairs[t * R3_THREADS] = make_float2(0.f, 0.f);
+    for (int t = 0; t < R3_VALUES; ++t)
+        if constexpr (kF32)
+            pairs[t * R3_THREADS] = make_float2(0.f, 0.f);
+        else
+            totals[t * R3_THREADS] = 0.0;
     auto flush = [&]() {
         if constexpr (kF32)
         {
@@ -1116,7 +1145,18 @@ __global__ void __launch_bounds__(R3_THREADS)
                 ar[t] = ai[t] = 0.f;
             }
         }
+        else
+        {
+#pragma unroll
+            for (int t = 0; t < 36; ++t)
+            {
+                totals[(2 * t) * R3_THREADS] += ar[t];
+                totals[(2 * t + 1) * R3_THREADS] += ai[t];
+                ar[t] = ai[t] = 0.0;
+            }
+        }
     };
+    const int most = kF32 ? rho3_run(n, nfree) : R3_RUN;
     int run = 0;
     if (inside)
         for (std::uint64_t c = beg; c < end; ++c)
@@ -1158,59 +1198,46 @@ __global__ void __launch_bounds__(R3_THREADS)
                         ai[t] = fma(-v[r].re, v[cc].im, ai[t]);
                     }
                 }
-            if (kF32 && ++run == R3_RUN)
+            if (++run == most)
             {
                 flush();
                 run = 0;
             }
         }
-    if constexpr (kF32)
-    {
-        if (run > 0) flush();
-    }
-    else
-    {
-#pragma unroll
-        for (int t = 0; t < 36; ++t)
-        {
-            r3_smem[(2 * t) * R3_THREADS + tid] = ar[t];
-            r3_smem[(2 * t + 1) * R3_THREADS + tid] = ai[t];
-        }
-    }
+    if (run > 0) flush();
     __syncthreads();
     double *out = part + ((static_cast<std::size_t>(traj) * gridDim.y + tri) * chunks + blockIdx.x) * R3_VALUES;
-    for (int t = warp; t < R3_VALUES; t += R3_THREADS / 32)
+    // Eight lanes per value, four values per warp. Values take the sixteen
+    // blocks of eight threads in turn, so that two of them meet no bank twice.
+    static_assert(R3_THREADS == 16 * 8 && R3_VALUES % 4 == 0, "lanes per value");
+    for (int t = 4 * warp + (lane >> 3); t < R3_VALUES; t += 4 * (R3_THREADS / 32))
     {
-        if constexpr (kF32)
-        {
-            const float2 *p = reinterpret_cast<const float2 *>(r3_smem) + t * R3_THREADS + lane;
-            float x = 0.f, e = 0.f;
+        const int at = t * R3_THREADS + (lane & 7);
+        double x4[4] = {0.0, 0.0, 0.0, 0.0};
+        float e = 0.f;
 #pragma unroll
-            for (int i = 0; i < R3_THREADS / 32; ++i)
+        for (int i = 0; i < 16; ++i)
+        {
+            const int a = at + 8 * ((i + t) & 15);
+            if constexpr (kF32)
             {
-                const float2 y = p[32 * i];
-                comp_add(y.x, x, e);
+                const float2 y = reinterpret_cast<const float2 *>(r3_smem)[a];
+                x4[i & 3] += widen(y.x);
                 e += y.y;
             }
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1)
-            {
-                const float y = __shfl_xor_sync(0xffffffffu, x, o), f = __shfl_xor_sync(0xffffffffu, e, o);
-                comp_add(y, x, e);
-                e += f;
-            }
-            if (lane == 0) out[t] = static_cast<double>(x) + static_cast<double>(e);
+            else
+                x4[i & 3] += r3_smem[a];
         }
-        else
+        double x = (x4[0] + x4[1]) + (x4[2] + x4[3]);
+#pragma unroll
+        for (int o = 4; o > 0; o >>= 1)
         {
-            const double *p = r3_smem + t * R3_THREADS + lane;
-            double x = 0.0;
-#pragma unroll
-            for (int i = 0; i < R3_THREADS / 32; ++i) x += p[32 * i];
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
-            if (lane == 0) out[t] = x;
+            x += __shfl_xor_sync(0xffffffffu, x, o);
+            if constexpr (kF32) e += __shfl_xor_sync(0xffffffffu, e, o);
         }
+        // A sum that left the FP32 range has no compensation (it is NaN).
+        if (kF32 && isfinite(x)) x += static_cast<double>(e);
+        if ((lane & 7) == 0) out[t] = x;
     }
 }
 
@@ -1249,11 +1276,13 @@ __global__ void __launch_bounds__(R3_VALUES *R3_GROUPS)
 }
 
 // Chunks per triple: about three CTAs per SM over all triples, at least one
-// FP32 run (or 4 FP64 columns) per thread.
+// FP32 run (or 4 FP64 columns) per thread. FP64 sums have no compensation, so
+// up to 256 chunks keep them at no more than four runs per thread.
 int rho3_chunks(int n, long long triples, bool fp64)
 {
     const std::uint64_t steps = n - 3 > 7 ? 1ull << (n - 10) : 1ull;
-    const std::uint64_t want = std::max<long long>(1, (3 * 152 + triples - 1) / triples);
+    std::uint64_t want = std::max<long long>(1, (3 * 152 + triples - 1) / triples);
+    if (fp64) want = std::max<std::uint64_t>(want, std::min<std::uint64_t>(256, steps / (4 * R3_RUN)));
     return static_cast<int>(std::max<std::uint64_t>(1, std::min<std::uint64_t>(want, steps / (fp64 ? 4 : R3_RUN))));
 }
 
@@ -1415,10 +1444,13 @@ cudaError_t jacobi_entropy(const double *rho, int d, int njobs, double *entropy_
 
 std::size_t rho3_scratch_bytes(int n, int batch, int count)
 {
-    // Enough for any smaller batch too: chunks * triples stays below the
-    // CTAs wanted plus the triples.
+    // Enough for any smaller batch and either precision: chunks * triples
+    // stays below the CTAs wanted plus the triples, or is the triples times
+    // the chunks that FP64 sums take however many triples there are.
     const std::size_t triples = static_cast<std::size_t>(count) * batch;
-    return sizeof(double) * R3_VALUES * std::min(3 * 152 + triples, triples * rho3_chunks(n, 1, true));
+    const std::size_t spread = std::min(3 * 152 + triples, triples * rho3_chunks(n, 1, true));
+    const std::size_t least = rho3_chunks(n, std::numeric_limits<long long>::max() / 2, true);
+    return sizeof(double) * R3_VALUES * std::max(spread, triples * least);
 }
 
 template <typename Real>
