@@ -772,9 +772,9 @@ constexpr int kCoalesceQubits = 4;
 // 2^k * 10 clocks per bond on its SM, so the one to eight tiles that 2^13
 // leaves up to n = 16 cost far more than the extra passes of smaller tiles: the
 // five bonds of an n = 10 FP64 layer took 101 us in one tile (the layer 189 us,
-// 119 us with this rule; n = 22 FP32 and larger are as before). Batches keep their
-// tuned tile whatever their size, so that a trajectory's rounding does not
-// depend on the batch.
+// 119 us with this rule; FP64 from n = 20 on and FP32 from n = 20 on are as
+// before). Batches keep their tuned tile whatever their size, so that a
+// trajectory's rounding does not depend on the batch.
 int engine_tile_qubits(int n, bool fp64)
 {
     const int most = default_tile_qubits(fp64);
@@ -1042,9 +1042,9 @@ struct mipt_gb300_batch
     PinnedBuf h_gates, h_meas, h_forced, h_res;
     std::vector<std::uint64_t> measured;
     std::vector<char> any_meas, fusable;
-    // [layer][chunk]: every trajectory's chunk lies outside the histogram tile
-    // (one total per tile, streamed without shared-memory staging).
-    std::vector<char> direct_hist;
+    // [layer][chunk]: the chunk's histogram streams for every trajectory, so its
+    // launch has no room for staged tiles.
+    std::vector<char> unstaged_hist;
     std::vector<int> max_chunks;
     bool has_forced = false;
     int points = 0;
@@ -1800,7 +1800,7 @@ int upload_draws(mipt_gb300_batch *b, const std::vector<TrajectoryDraw> &draws, 
     b->measured.assign(static_cast<std::size_t>(count) * T, 0);
     b->any_meas.assign(T, 0);
     b->fusable.assign(T, 1);
-    b->direct_hist.assign(static_cast<std::size_t>(T) * kMaxChunks, 1);
+    b->unstaged_hist.assign(static_cast<std::size_t>(T) * kMaxChunks, 1);
     b->max_chunks.assign(T, 0);
     b->has_forced = forced != nullptr;
     // Parity-sector execution needs every trajectory in a definite sector.
@@ -1919,7 +1919,7 @@ int upload_draws(mipt_gb300_batch *b, const std::vector<TrajectoryDraw> &draws, 
                 M.uniform[cc] = d.uniforms[d.uniform_offset[t] + cc];
                 if (M.chunk[cc] >> ne) continue; // the parity chunk of a half-size state
                 if (!hist_streams(ne, b->kmax, b->cmin, M.chunk[cc]))
-                    b->direct_hist[static_cast<std::size_t>(t) * kMaxChunks + cc] = 0;
+                    b->unstaged_hist[static_cast<std::size_t>(t) * kMaxChunks + cc] = 0;
             }
             hm[slot] = M;
             hf[slot] = forced ? forced[slot] : 0ull;
@@ -2322,7 +2322,7 @@ int batch_execute(mipt_gb300_batch *b, cudaStream_t s)
                     Mark m(b, K_HIST, s);
                     MG_CUDA(launch_hist<Real>(xs, count, ne, b->kmax, b->cmin, ci, col + t, T, meas + t, T,
                                               b->part.as<double>(),
-                                              b->direct_hist[static_cast<std::size_t>(t) * kMaxChunks + ci] != 0, s,
+                                              b->unstaged_hist[static_cast<std::size_t>(t) * kMaxChunks + ci] != 0, s,
                                               sec));
                     ++L;
                 }
@@ -2416,7 +2416,7 @@ std::vector<long long> structure_key(const mipt_gb300_batch *b)
     for (char c : b->any_meas) k.push_back(c);
     for (char c : b->fusable) k.push_back(c);
     for (int c : b->max_chunks) k.push_back(c);
-    for (char c : b->direct_hist) k.push_back(c);
+    for (char c : b->unstaged_hist) k.push_back(c);
     for (int c : b->obs_point) k.push_back(c);
     for (char c : b->custom_init) k.push_back(c);
     for (int i = 0; i < b->count && b->cfg.circuit == 2; ++i)

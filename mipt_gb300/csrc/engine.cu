@@ -1316,12 +1316,26 @@ __global__ void __launch_bounds__(512, 1)
 }
 
 
+// Whether a tile's histogram can be summed while it streams: the chunk's sites
+// inside the tile are among its nine lowest bits, so each of 512 threads meets
+// one bin only.
+__host__ __device__ bool tile_streams(const PassGeom &g, std::uint64_t chunk)
+{
+    for (int i = 0; i < g.k; ++i)
+        if (((chunk >> g.pos[i]) & 1ull) && (i >= 9 || (1 << g.k) < kPassThreads)) return false;
+    return true;
+}
+
+// unstaged: every trajectory's chunk streams, so the launch has no room for a
+// tile. Whether a chunk streams is its own matter all the same: the two paths
+// add in different orders, and a trajectory's sums must not depend on the
+// others of its batch.
 template <typename Real>
 __global__ void __launch_bounds__(kPassThreads) k_hist(const Cx<Real> *__restrict__ states, int n, int kmax, int cmin,
                                                        int ci, const Collapse *__restrict__ col_in,
                                                        std::size_t col_stride, const LayerMeas *__restrict__ meas,
                                                        std::size_t meas_stride, double *__restrict__ partials,
-                                                       int direct, const signed char *__restrict__ sector)
+                                                       int unstaged, const signed char *__restrict__ sector)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ PassGeom g;
@@ -1338,7 +1352,7 @@ __global__ void __launch_bounds__(kPassThreads) k_hist(const Cx<Real> *__restric
     if (threadIdx.x == 0) histogram_geometry(n, kmax, cmin, par_chunk ? 0ull : chunk, g);
     __syncthreads();
     Cx<Real> *tile = reinterpret_cast<Cx<Real> *>(smem_raw);
-    std::uint32_t *seg = reinterpret_cast<std::uint32_t *>(direct ? smem_raw : smem_raw + (sizeof(Cx<Real>) << g.k));
+    std::uint32_t *seg = reinterpret_cast<std::uint32_t *>(unstaged ? smem_raw : smem_raw + (sizeof(Cx<Real>) << g.k));
     const std::uint64_t tix = blockIdx.x;
     const std::uint64_t dim = 1ull << n;
     const Cx<Real> *psi = states + static_cast<std::size_t>(b) * dim;
@@ -1352,7 +1366,7 @@ __global__ void __launch_bounds__(kPassThreads) k_hist(const Cx<Real> *__restric
     __syncthreads();
     if (par_chunk)
     {
-        // Tile bins (top qubit 0, 1) in the order of the direct sum below.
+        // Tile bins (top qubit 0, 1), one sum per thread and bin.
         const int P = sector ? sector[b] : 0;
         const std::uint64_t nloc = 1ull << g.k, cmask = (1ull << g.c) - 1ull;
         const Real scale = static_cast<Real>(cl.scale);
@@ -1387,12 +1401,11 @@ __global__ void __launch_bounds__(kPassThreads) k_hist(const Cx<Real> *__restric
     for (int i = 0; i < g.k; ++i)
         if ((chunk >> g.pos[i]) & 1ull) lm[m_loc++] = i;
     double *part = partials + static_cast<std::size_t>(b) * kHistScratch + (tix << m_loc);
-    if (direct)
+    if (tile_streams(g, chunk))
     {
-        // The measured sites inside the tile are among its nine lowest bits
-        // (hist_streams), so thread t's amplitudes t, t + 512, ... all belong to
-        // one bin: they stream from global memory, eight loads in flight, into
-        // one sum per thread, and the threads' sums are added by bin. Staging
+        // Thread t's amplitudes t, t + 512, ... all belong to one bin: they
+        // stream from global memory, eight loads in flight, into one sum per
+        // thread, and the threads' sums are added by bin. Staging
         // the tile (128 KB, one CTA per SM) kept loads and sums apart: one
         // n = 26 FP32 layer went from 2.21 to 1.69 ms.
         __shared__ double sums[kPassThreads];
@@ -1810,9 +1823,7 @@ bool hist_streams(int n, int kmax, int cmin, std::uint64_t chunk)
 {
     PassGeom g{};
     histogram_geometry(n, kmax, cmin, chunk, g);
-    for (int i = 0; i < g.k; ++i)
-        if (((chunk >> g.pos[i]) & 1ull) && (i >= 9 || (1 << g.k) < kPassThreads)) return false;
-    return true;
+    return tile_streams(g, chunk);
 }
 
 int local_measured_count(const PassGeom &g, std::uint64_t chunk)
@@ -2454,18 +2465,18 @@ cudaError_t launch_pass(Cx<Real> *states, int batch, const PassPlan &plan, const
 template <typename Real>
 cudaError_t launch_hist(const Cx<Real> *states, int batch, int n, int kmax, int cmin, int chunk_index,
                         const Collapse *collapse_in, std::size_t collapse_stride, const LayerMeas *meas,
-                        std::size_t meas_stride, double *partials, bool direct, cudaStream_t s,
+                        std::size_t meas_stride, double *partials, bool unstaged, cudaStream_t s,
                         const signed char *sector)
 {
     const int k = std::min(kmax, n);
-    // Direct (hist_streams): only the segment table.
-    const std::size_t smem = direct ? (sizeof(std::uint32_t) << std::max(0, k - std::min(cmin, k)))
+    // Unstaged (hist_streams for every state): only the segment table.
+    const std::size_t smem = unstaged ? (sizeof(std::uint32_t) << std::max(0, k - std::min(cmin, k)))
                                     : pass_smem<Real>(k);
     cudaError_t e = ensure_smem_attr<Real>(reinterpret_cast<const void *>(&k_hist<Real>), smem);
     if (e != cudaSuccess) return e;
     dim3 grid(1u << (n - k), batch);
     k_hist<Real><<<grid, kPassThreads, smem, s>>>(states, n, kmax, cmin, chunk_index, collapse_in, collapse_stride,
-                                                  meas, meas_stride, partials, direct ? 1 : 0, sector);
+                                                  meas, meas_stride, partials, unstaged ? 1 : 0, sector);
     return cudaGetLastError();
 }
 

@@ -142,15 +142,15 @@ inline std::uint64_t nonlocal_mask(const PassGeom &g)
     return m;
 }
 
-// Whether the chunk's histogram can be summed while streaming (launch_hist's
-// `direct`): its sites inside a histogram tile are among the tile's nine lowest
-// bits, so each of 512 threads meets one bin only.
+// Whether the chunk's histogram is summed while streaming: its sites inside a
+// histogram tile are among the tile's nine lowest bits. launch_hist's
+// `unstaged` says that this holds for every state's chunk.
 bool hist_streams(int n, int kmax, int cmin, std::uint64_t chunk);
 
 template <typename Real>
 cudaError_t launch_hist(const Cx<Real> *states, int batch, int n, int kmax, int cmin, int chunk_index,
                         const Collapse *collapse_in, std::size_t collapse_stride, const LayerMeas *meas,
-                        std::size_t meas_stride, double *partials, bool direct, cudaStream_t s,
+                        std::size_t meas_stride, double *partials, bool unstaged, cudaStream_t s,
                         const signed char *sector = nullptr);
 
 // Samples (or replays) the outcome of chunk `chunk_index` from the partial
