@@ -653,7 +653,10 @@ __global__ void __launch_bounds__(128)
     const int dm = dims != nullptr ? dims[jb] : d;
     const double *dg = diag + static_cast<std::size_t>(jb) * d;
     const double *of = off + static_cast<std::size_t>(jb) * d;
-    // |T| (largest row sum; a NaN or an infinity anywhere makes `sum` one).
+    // |T| (largest row sum; a NaN or an infinity anywhere makes `sum` one). The
+    // search runs on the matrix times a power of four that brings |T| into
+    // [1/4, 1), so the counts' range does not depend on the state's norm; a
+    // power of four also scales the search's geometric means exactly.
     double top = 0.0, sum = 0.0;
     for (int i = threadIdx.x; i < dm; i += blockDim.x)
     {
@@ -661,7 +664,6 @@ __global__ void __launch_bounds__(128)
         const double t = fabs(dg[i]) + e0 + e1;
         top = fmax(top, t);
         sum += t;
-        de[i] = make_double2(dg[i], e0 * e0);
     }
     sum = block_sum(sum, red);
 #pragma unroll
@@ -672,16 +674,22 @@ __global__ void __launch_bounds__(128)
     top = red[0];
     for (int q = 1; q < static_cast<int>(blockDim.x >> 5); ++q) top = fmax(top, red[q]);
     const bool finite = sum - sum == 0.0;
+    int shift = 0;
+    if (finite && top > 0.0) frexp(top, &shift);
+    shift = shift < -1000 ? -1000 : shift + (shift & 1); // below 2^-1000 every eigenvalue is under the cut-off
+    const double scale = scalbn(1.0, -shift);
+    top *= scale;
     const double floor2 = kTinyE2 * top * top, inv = top > 0.0 ? 1.0 / top : 0.0;
     for (int i = threadIdx.x; i < dm; i += blockDim.x)
     {
-        if (i > 0 && de[i].y < floor2) de[i].y = floor2;
+        const double e = i > 0 ? of[i - 1] * scale : 0.0;
+        de[i] = make_double2(dg[i] * scale, i > 0 ? fmax(e * e, floor2) : 0.0);
         df[i] = sturm_entry32(de[i], inv, i);
     }
     __syncthreads();
     const int at = blockIdx.y * blockDim.x + threadIdx.x, idx = at >> gl;
     const bool writes = (at & ((1 << gl) - 1)) == 0;
-    const double bound = top * (1.0 + 1e-14), cutoff = want_all ? -2.0 * bound : kEigCutoff;
+    const double bound = top * (1.0 + 1e-14), cutoff = want_all ? -2.0 * bound : kEigCutoff * scale;
     double term = 0.0, l = 0.0;
     if (gl > 0 && finite && top > 0.0)
         l = sturm_eigenvalue_lanes(de, df, dm, idx < dm ? idx : dm - 1, top, bound, cutoff, gl, idx < dm);
@@ -689,6 +697,7 @@ __global__ void __launch_bounds__(128)
         l = sturm_eigenvalue(de, df, dm, idx, top, bound, cutoff);
     if (finite && writes && idx < dm)
     {
+        l = scalbn(l, shift);
         if (want_all) diag[static_cast<std::size_t>(jb) * d + idx] = l;
         if (l > kEigCutoff) term = -l * log2(l);
     }

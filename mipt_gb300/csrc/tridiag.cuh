@@ -22,8 +22,9 @@ namespace mg
 {
 
 // Squared off-diagonals are at least this times |T|^2: a zero minor is then
-// followed by a non-zero one, 16 unscaled steps stay in range, and an
-// eigenvalue moves by at most 1e-17 |T|. FP32 counts: 4 steps, 1e-7 |T|.
+// followed by a non-zero one, and an eigenvalue moves by at most 1e-17 |T|. With
+// |T| in [1/4, 1], as the caller scales it, 16 unscaled steps stay in range
+// (between 1e-282 and 4^16). FP32 counts: 4 steps, 1e-7 |T|.
 constexpr double kTinyE2 = 1e-34;
 constexpr float kTinyE2f = 1e-14f;
 constexpr int kSturmRescale = 16;
@@ -109,7 +110,7 @@ __device__ __forceinline__ float2 sturm_entry32(double2 de, double inv_norm, int
 }
 
 // Eigenvalue `index` (ascending) of the matrix, all of whose eigenvalues lie
-// in (-bound, bound), norm being about |T|; eigenvalues below `cutoff` may
+// in (-bound, bound), norm being |T| (1/4 to 1); eigenvalues below `cutoff` may
 // come back as any value below it.
 __device__ __forceinline__ double sturm_eigenvalue(const double2 *__restrict__ de, const float2 *__restrict__ df,
                                                    int d, int index, double norm, double bound, double cutoff)
@@ -157,6 +158,8 @@ __device__ __forceinline__ double sturm_eigenvalue(const double2 *__restrict__ d
     // end any search.
     int tries = 0;
     double w_try = 0.0;
+    // Geometric means, in FP32, of brackets that span much of the range.
+    const double least = fmax(0.01 * cutoff, 1e-30);
     for (int it = -2; it < 160; ++it)
     {
         const double w = hi - lo;
@@ -187,7 +190,7 @@ __device__ __forceinline__ double sturm_eigenvalue(const double2 *__restrict__ d
                 const double y = lo + w * static_cast<double>(1.f / (1.f + r));
                 x = y < lo + half ? lo + half : (y > hi - half ? hi - half : y);
             }
-            else if (lo > 1e-17 && hi > 16.0 * lo)
+            else if (lo > least && hi > 16.0 * lo)
                 x = static_cast<double>(sqrtf(static_cast<float>(lo)) * sqrtf(static_cast<float>(hi)));
         }
         probe(x, isolated);
