@@ -528,9 +528,8 @@ int run_entropies(const Cx<Real> *states, int n, const std::vector<EntReq> &reqs
                     MG_CUDA(cudaMemsetAsync(ws.eig_err.p, 0, sizeof(int), s));
                 }
                 int launched = 0;
-                MG_CUDA(hermitian_eig_entropy(ws.rho.as<double>(), d, nbi, ws.vals.as<double>(), nullptr,
-                                              ws.eig.as<double>(), ws.eig_err.as<int>(), s, ws.dims.as<int>(),
-                                              &launched));
+                MG_CUDA(hermitian_eig_entropy(ws.rho.as<double>(), d, nbi, ws.vals.as<double>(), ws.eig.as<double>(),
+                                              ws.eig_err.as<int>(), s, ws.dims.as<int>(), &launched));
                 launches += launched;
                 k_scatter<<<(nbi + 255) / 256, 256, 0, s>>>(ws.vals.as<double>(), ws.idx.as<int>(), nbi, d_out, 0);
                 ++launches;

@@ -643,8 +643,8 @@ __global__ void __launch_bounds__(256) k_eig_list(const int *__restrict__ dims, 
 constexpr double kEigCutoff = 1e-15;
 
 __global__ void __launch_bounds__(128)
-    k_tridiag_sturm(double *__restrict__ diag, const double *__restrict__ off, int d, double *__restrict__ terms,
-                    double *__restrict__ entropy, int *__restrict__ err, const int *__restrict__ dims, int want_all, int gl)
+    k_tridiag_sturm(const double *__restrict__ diag, const double *__restrict__ off, int d, double *__restrict__ terms,
+                    double *__restrict__ entropy, int *__restrict__ err, const int *__restrict__ dims, int gl)
 {
     extern __shared__ __align__(16) double2 de[];
     float2 *df = reinterpret_cast<float2 *>(de + d);
@@ -689,7 +689,7 @@ __global__ void __launch_bounds__(128)
     __syncthreads();
     const int at = blockIdx.y * blockDim.x + threadIdx.x, idx = at >> gl;
     const bool writes = (at & ((1 << gl) - 1)) == 0;
-    const double bound = top * (1.0 + 1e-14), cutoff = want_all ? -2.0 * bound : kEigCutoff * scale;
+    const double bound = top * (1.0 + 1e-14), cutoff = kEigCutoff * scale;
     double term = 0.0, l = 0.0;
     if (gl > 0 && finite && top > 0.0)
         l = sturm_eigenvalue_lanes(de, df, dm, idx < dm ? idx : dm - 1, top, bound, cutoff, gl, idx < dm);
@@ -698,7 +698,6 @@ __global__ void __launch_bounds__(128)
     if (finite && writes && idx < dm)
     {
         l = scalbn(l, shift);
-        if (want_all) diag[static_cast<std::size_t>(jb) * d + idx] = l;
         if (l > kEigCutoff) term = -l * log2(l);
     }
     if (!finite && blockIdx.y == 0 && threadIdx.x == 0) atomicOr(err, 1);
@@ -767,13 +766,13 @@ std::size_t hermitian_eig_scratch_doubles(int d, int nb)
     return (4 * static_cast<std::size_t>(d) + 2) * nb + 1;
 }
 
-cudaError_t hermitian_eig_entropy(double *rho, int d, int nb, double *entropy_out, double *eig_out, double *scratch,
+cudaError_t hermitian_eig_entropy(double *rho, int d, int nb, double *entropy_out, double *scratch,
                                   int *err, cudaStream_t s, const int *dims, int *launched)
 {
     if (launched) *launched = 0;
     if (nb <= 0) return cudaSuccess;
     if (d < 2 || d > 4096) return cudaErrorInvalidValue;
-    double *diag = eig_out ? eig_out : scratch;
+    double *diag = scratch;
     double *off = scratch + static_cast<std::size_t>(d) * nb;
     double2 *pglob = reinterpret_cast<double2 *>(scratch + 2 * static_cast<std::size_t>(d) * nb);
     unsigned *bars = reinterpret_cast<unsigned *>(scratch + 4 * static_cast<std::size_t>(d) * nb);
@@ -861,7 +860,7 @@ cudaError_t hermitian_eig_entropy(double *rho, int d, int nb, double *entropy_ou
     if (e != cudaSuccess) return e;
     // The terms take the place of the p vectors, which the reduction is done with.
     double *terms = reinterpret_cast<double *>(pglob);
-    k_tridiag_sturm<<<dim3(nb, chunks), tpb, sm, s>>>(diag, off, d, terms, entropy_out, err, dims, eig_out != nullptr, gl);
+    k_tridiag_sturm<<<dim3(nb, chunks), tpb, sm, s>>>(diag, off, d, terms, entropy_out, err, dims, gl);
     e = cudaGetLastError();
     if (launched) *launched = kernels + (chunks == 1 ? 1 : 2);
     if (e != cudaSuccess || chunks == 1) return e;

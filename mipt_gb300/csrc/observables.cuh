@@ -106,16 +106,14 @@ cudaError_t jacobi_entropy(const double *rho, int d, int njobs, double *entropy_
 // Von Neumann entropies (bits) of Hermitian matrices rho[job][d][d]
 // (destroyed; d a power of two) for 2 <= d <= 4096: FP64 Householder
 // tridiagonalisation, then Sturm counts, one thread per eigenvalue (eigen.cu).
-// eig_out (nullable) receives each matrix's eigenvalues (ascending); scratch
-// holds hermitian_eig_scratch_doubles(d, njobs) doubles. A matrix that is not
-// finite sets bit 1 of *err and gives NaN; a timed-out barrier between the CTAs
-// of one matrix sets bit 2. launched (nullable) receives the kernel launches.
-// dims (nullable): the rows of each matrix that hold data (the rest of
-// its d x d block is zero); the eigensolver then runs on those only.
+// scratch holds hermitian_eig_scratch_doubles(d, njobs) doubles. A matrix that
+// is not finite sets bit 1 of *err and gives NaN; a timed-out barrier between
+// the CTAs of one matrix sets bit 2. launched (nullable) receives the kernel
+// launches. dims (nullable): the rows of each matrix that hold data (the rest
+// of its d x d block is zero); the eigensolver then runs on those only.
 std::size_t hermitian_eig_scratch_doubles(int d, int njobs);
-cudaError_t hermitian_eig_entropy(double *rho, int d, int njobs, double *entropy_out, double *eig_out,
-                                  double *scratch, int *err, cudaStream_t s, const int *dims = nullptr,
-                                  int *launched = nullptr);
+cudaError_t hermitian_eig_entropy(double *rho, int d, int njobs, double *entropy_out, double *scratch, int *err,
+                                  cudaStream_t s, const int *dims = nullptr, int *launched = nullptr);
 
 // Three-site RDMs of every trajectory, for `count` triples subs[3*i..].
 // out[traj][i][8][8] complex row-major. fermion selects the fermionic trace

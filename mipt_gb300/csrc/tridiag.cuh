@@ -110,8 +110,8 @@ __device__ __forceinline__ float2 sturm_entry32(double2 de, double inv_norm, int
 }
 
 // Eigenvalue `index` (ascending) of the matrix, all of whose eigenvalues lie
-// in (-bound, bound), norm being |T| (1/4 to 1); eigenvalues below `cutoff` may
-// come back as any value below it.
+// in (-bound, bound), norm being |T| (1/4 to 1); eigenvalues below `cutoff`
+// (0 or more) may come back as any value below it.
 __device__ __forceinline__ double sturm_eigenvalue(const double2 *__restrict__ de, const float2 *__restrict__ df,
                                                    int d, int index, double norm, double bound, double cutoff)
 {
@@ -140,7 +140,7 @@ __device__ __forceinline__ double sturm_eigenvalue(const double2 *__restrict__ d
             side = -1;
         }
     };
-    float a = cutoff > 0.0 ? -1e-6f : -1.001f, b = 1.001f;
+    float a = -1e-6f, b = 1.001f; // nothing below the (positive) cutoff is looked for
     for (int it = 0; it < 20; ++it)
     {
         const float x = 0.5f * (a + b);
@@ -215,7 +215,7 @@ __device__ __forceinline__ double sturm_eigenvalue_lanes(const double2 *__restri
         return m ? __ffs(m) - 1 : G;
     };
     // As many rounds as narrow the FP32 bracket 2^20 fold.
-    float a = cutoff > 0.0 ? -1e-6f : -1.001f, b = 1.001f;
+    float a = -1e-6f, b = 1.001f; // nothing below the (positive) cutoff is looked for
     const float stepf = 1.f / static_cast<float>(G + 1);
     for (float left = 1 << 20; left > 1.f; left *= stepf)
     {
