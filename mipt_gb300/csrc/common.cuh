@@ -18,6 +18,11 @@ __device__ __forceinline__ std::uint64_t device_ns()
     return t;
 }
 
+// Raises a kernel's dynamic shared memory limit to at least `bytes` (engine.cu).
+// The limit belongs to the kernel on its device, not to the calling thread, so
+// it is never lowered: another thread may be between this call and its launch.
+cudaError_t allow_dynamic_smem(const void *kernel, std::size_t bytes);
+
 // Interleaved complex amplitude; float2 / double2 layout in HBM.
 template <typename Real> struct Cx;
 template <> struct __align__(8) Cx<float>

@@ -736,8 +736,7 @@ cudaError_t launch_cluster(const double2 *rho, int d, int nb, int C, double *dia
     const std::size_t smem = std::max(cluster_smem(32 * NCB, C, THREADS / 32),
                                       list ? cluster_smem(kSmallRows, 1, 0) + sizeof(double2) * (4 + THREADS / 32) * 32 * NCB
                                            : std::size_t{0});
-    cudaError_t e = cudaFuncSetAttribute(k_tridiag_cluster<NCB, THREADS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         static_cast<int>(smem));
+    cudaError_t e = allow_dynamic_smem(reinterpret_cast<const void *>(&k_tridiag_cluster<NCB, THREADS>), smem);
     if (e != cudaSuccess) return e;
     if (C > 8)
     {
@@ -813,7 +812,7 @@ cudaError_t hermitian_eig_entropy(double *rho, int d, int nb, double *entropy_ou
         int least = dims != nullptr ? kClusterRows : 0;
         ++kernels;
         const std::size_t smem = 2 * sizeof(double2) * d;
-        e = cudaFuncSetAttribute(k_tridiag, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+        e = allow_dynamic_smem(reinterpret_cast<const void *>(&k_tridiag), smem);
         if (e != cudaSuccess) return e;
         // Fewer matrices than SMs: spread each matrix over `parts` resident CTAs
         // (cooperative launch), at least 16 trailing rows per CTA.
@@ -856,7 +855,7 @@ cudaError_t hermitian_eig_entropy(double *rho, int d, int nb, double *entropy_ou
     const int tpb = gl > 0 || warps <= 2 * sms ? 32 : std::min(128, (d + 31) / 32 * 32);
     const int chunks = ((d << gl) + tpb - 1) / tpb;
     const std::size_t sm = (sizeof(double2) + sizeof(float2)) * d;
-    e = cudaFuncSetAttribute(k_tridiag_sturm, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(sm));
+    e = allow_dynamic_smem(reinterpret_cast<const void *>(&k_tridiag_sturm), sm);
     if (e != cudaSuccess) return e;
     // The terms take the place of the p vectors, which the reduction is done with.
     double *terms = reinterpret_cast<double *>(pglob);

@@ -17,6 +17,7 @@
 #include <cmath>
 #include <cstdlib>
 #include <cstring>
+#include <mutex>
 #include <stdexcept>
 
 #include <cuda.h>
@@ -1778,12 +1779,17 @@ std::size_t pass_smem(int k)
     return (sizeof(Cx<Real>) << k) + (sizeof(std::uint32_t) << k);
 }
 
-template <typename Real>
-cudaError_t ensure_smem_attr(const void *fn, std::size_t bytes)
-{
-    return cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes));
-}
 } // namespace
+
+cudaError_t allow_dynamic_smem(const void *kernel, std::size_t bytes)
+{
+    static std::mutex lock;
+    const std::lock_guard<std::mutex> held(lock);
+    cudaFuncAttributes now{};
+    const cudaError_t e = cudaFuncGetAttributes(&now, kernel);
+    if (e != cudaSuccess || static_cast<std::size_t>(now.maxDynamicSharedSizeBytes) >= bytes) return e;
+    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes));
+}
 
 __host__ __device__ void histogram_geometry(int n, int kmax, int cmin, std::uint64_t chunk, PassGeom &g)
 {
@@ -2364,7 +2370,7 @@ cudaError_t launch_rounds(Cx<Real> *states, int batch, const PassPlan &plan, con
     const void *fn = reinterpret_cast<const void *>(&k_pass_rounds<Real, RB, PAR>);
     const std::size_t smem = (sizeof(Cx<Real>) << plan.geom.k) +
                              (sparse ? sizeof(std::uint32_t) * (static_cast<std::size_t>(batch) + 1) : 0);
-    cudaError_t e = ensure_smem_attr<Real>(fn, smem);
+    cudaError_t e = allow_dynamic_smem(fn, smem);
     if (e != cudaSuccess) return e;
     const int threads = 1 << (plan.geom.k - RB);
     const dim3 pgrid = pass_grid(fn, threads, smem, dim3(1u << plan.geom.n_nl, batch));
@@ -2393,7 +2399,7 @@ cudaError_t launch_quads(Cx<float> *states, int batch, const PassPlan &plan, con
     const int threads = 1 << (plan.geom.k - 5);
     const std::size_t smem =
         quad_smem(plan) + (sparse ? sizeof(std::uint32_t) * (static_cast<std::size_t>(batch) + 1) : 0);
-    cudaError_t e = ensure_smem_attr<float>(fn, smem);
+    cudaError_t e = allow_dynamic_smem(fn, smem);
     if (e != cudaSuccess) return e;
     const dim3 pgrid = pass_grid(fn, threads, smem, dim3(1u << plan.geom.n_nl, batch));
     k_pass_quads<TMA, PAR><<<pgrid, threads, smem, s>>>(states, plan, layer_gates, gate_stride, collapse_in,
@@ -2454,7 +2460,7 @@ cudaError_t launch_pass(Cx<Real> *states, int batch, const PassPlan &plan, const
         }
     }
     const std::size_t smem = pass_smem<Real>(plan.geom.k);
-    cudaError_t e = ensure_smem_attr<Real>(reinterpret_cast<const void *>(&k_pass<Real>), smem);
+    cudaError_t e = allow_dynamic_smem(reinterpret_cast<const void *>(&k_pass<Real>), smem);
     if (e != cudaSuccess) return e;
     k_pass<Real><<<grid, kPassThreads, smem, s>>>(states, plan.geom, plan.gates, layer_gates, gate_stride,
                                                   collapse_in, collapse_stride, meas, meas_stride, partials,
@@ -2472,7 +2478,7 @@ cudaError_t launch_hist(const Cx<Real> *states, int batch, int n, int kmax, int 
     // Unstaged (hist_streams for every state): only the segment table.
     const std::size_t smem = unstaged ? (sizeof(std::uint32_t) << std::max(0, k - std::min(cmin, k)))
                                     : pass_smem<Real>(k);
-    cudaError_t e = ensure_smem_attr<Real>(reinterpret_cast<const void *>(&k_hist<Real>), smem);
+    cudaError_t e = allow_dynamic_smem(reinterpret_cast<const void *>(&k_hist<Real>), smem);
     if (e != cudaSuccess) return e;
     dim3 grid(1u << (n - k), batch);
     k_hist<Real><<<grid, kPassThreads, smem, s>>>(states, n, kmax, cmin, chunk_index, collapse_in, collapse_stride,

@@ -620,11 +620,9 @@ extern "C" int mipt_gb300_ff_run(const mipt_gb300_ff_config *cfg, const std::uin
     const std::size_t tri_bytes = rot_elem * (static_cast<std::size_t>(M) * (M - 1) / 2);
     const std::size_t smem = (fp64 ? 0 : tri_bytes) + rot_elem * (2 * M + G * 16) + G * 4 + 16;
     if (fp64)
-        FF_CUDA(cudaFuncSetAttribute(k_ff_evolve<double>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     static_cast<int>(smem)));
+        FF_CUDA(allow_dynamic_smem(reinterpret_cast<const void *>(&k_ff_evolve<double>), smem));
     else
-        FF_CUDA(cudaFuncSetAttribute(k_ff_evolve<float>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     static_cast<int>(smem)));
+        FF_CUDA(allow_dynamic_smem(reinterpret_cast<const void *>(&k_ff_evolve<float>), smem));
     const int seg = cfg->repurify_every > 0 ? cfg->repurify_every : depth;
     for (int t0 = 0; t0 < depth; t0 += seg)
     {
@@ -711,8 +709,7 @@ extern "C" int mipt_gb300_ff_run(const mipt_gb300_ff_config *cfg, const std::uin
             if (end == begin) continue;
             const std::size_t d = static_cast<std::size_t>(std::max(1, 2 * modes(jobs[begin])));
             const std::size_t esm = sizeof(double) * d * (d + 1);
-            FF_CUDA(cudaFuncSetAttribute(k_ff_entropy, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         static_cast<int>(esm)));
+            FF_CUDA(allow_dynamic_smem(reinterpret_cast<const void *>(&k_ff_entropy), esm));
             k_ff_entropy<<<end - begin, 256, esm>>>(N, d_g64.as<double>(), d_jobs.as<FFEntJob>() + begin,
                                                     d_ent.as<double>());
             FF_CUDA(cudaGetLastError());

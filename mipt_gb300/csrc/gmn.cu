@@ -644,8 +644,7 @@ int gmn_solve(const mipt_gb300_gmn_config &cfg, const double *h_rho, int count, 
     const int every = std::max(1, cfg.check_every);
     int it = 0;
     const std::size_t smem = sizeof(C2<Real>) * kIterShared * kIterProblems;
-    GMN_CUDA(cudaFuncSetAttribute(k_gmn_iterate<Real>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  static_cast<int>(smem)));
+    GMN_CUDA(allow_dynamic_smem(reinterpret_cast<const void *>(&k_gmn_iterate<Real>), smem));
     while (it < cfg.max_iter)
     {
         const int n = std::min(every, cfg.max_iter - it);

@@ -1436,7 +1436,7 @@ cudaError_t jacobi_entropy(const double *rho, int d, int njobs, double *entropy_
     if (njobs <= 0) return cudaSuccess;
     if (d > 64) return cudaErrorInvalidValue;
     const std::size_t smem = sizeof(double2) * d * (d + 1);
-    cudaError_t e = cudaFuncSetAttribute(k_jacobi, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+    cudaError_t e = allow_dynamic_smem(reinterpret_cast<const void *>(&k_jacobi), smem);
     if (e != cudaSuccess) return e;
     k_jacobi<<<njobs, 256, smem, s>>>(rho, d, entropy_out, eig_out);
     return cudaGetLastError();
@@ -1463,7 +1463,7 @@ cudaError_t rho3_sweep(const Cx<Real> *states, int n, int batch, const int *d_su
     if (sizeof(double) * R3_VALUES * static_cast<std::size_t>(chunks) * count * batch > scratch_bytes)
         return cudaErrorInvalidValue;
     constexpr int smem = sizeof(double) * R3_VALUES * R3_THREADS;
-    cudaError_t e = cudaFuncSetAttribute(k_rho3<Real>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    cudaError_t e = allow_dynamic_smem(reinterpret_cast<const void *>(&k_rho3<Real>), smem);
     if (e != cudaSuccess) return e;
     dim3 grid(chunks, count, batch);
     k_rho3<Real><<<grid, R3_THREADS, smem, s>>>(states, n, d_subs, fermion, collapse, collapse_stride, chunks,
@@ -2503,8 +2503,7 @@ cudaError_t gram_purity_tc(const Cx<float> *states, int n, const GramJob *d_jobs
     {
         // Pre-split operand rows, jobs in groups that fit `rows`.
         const int group = static_cast<int>(std::min<std::size_t>(static_cast<std::size_t>(njobs), rows_bytes / per_job));
-        cudaError_t e = cudaFuncSetAttribute(k_gram_tc_pre, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             static_cast<int>(TP_SMEM));
+        cudaError_t e = allow_dynamic_smem(reinterpret_cast<const void *>(&k_gram_tc_pre), TP_SMEM);
         if (e != cudaSuccess) return e;
         CompactJob *cjobs = reinterpret_cast<CompactJob *>(static_cast<char *>(scratch) +
                                                            sizeof(double) * static_cast<std::size_t>(gram_tc_tiles(k)) *
@@ -2561,8 +2560,7 @@ cudaError_t gram_purity_tc(const Cx<float> *states, int n, const GramJob *d_jobs
                                    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
     }
     auto kernel = tma ? k_gram_tc<true> : k_gram_tc<false>;
-    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         static_cast<int>(TC_SMEM));
+    cudaError_t e = allow_dynamic_smem(reinterpret_cast<const void *>(kernel), TC_SMEM);
     if (e != cudaSuccess) return e;
     dim3 grid(gram_tc_blocks(k), 2, njobs);
     kernel<<<grid, TC_THREADS, TC_SMEM, s>>>(states, n, d_jobs, collapse, collapse_stride,
