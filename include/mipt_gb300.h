@@ -253,6 +253,10 @@ int mipt_gb300_batch_parity_encoded(const mipt_gb300_batch *batch);
  * out"). The device stays usable: the next execute runs normally. */
 int mipt_gb300_test_withhold_tile_loads(int count);
 
+/* The same for one half of that tile: halves is 1 (the lower half), 2 (the
+ * upper) or 3 (both). */
+int mipt_gb300_test_withhold_tile_halves(int count, int halves);
+
 /* Draw `count` trajectories (trajectory i from seeds[i] with measurement
  * rate p[i]) on host threads exactly as the reference's HaarCircuit1D
  * (cpp/include/mipt/circuit.hpp:129-140,415-439) -- or, for circuit 2/4, its

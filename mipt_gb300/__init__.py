@@ -119,6 +119,7 @@ def lib():
     L.mipt_gb300_batch_group_destroy.argtypes = [vp]
     L.mipt_gb300_batch_group_destroy.restype = None
     L.mipt_gb300_test_withhold_tile_loads.argtypes = [ci]
+    L.mipt_gb300_test_withhold_tile_halves.argtypes = [ci, ci]
     _lib = L
     return L
 

@@ -1587,10 +1587,13 @@ int set_rho3_subs(mipt_gb300_batch *b, const std::vector<int> &subs)
 extern "C" {
 int mipt_gb300_batch_parity_encoded(const mipt_gb300_batch *b) { return (b && b->enc) ? 1 : 0; }
 
-int mipt_gb300_test_withhold_tile_loads(int count)
+int mipt_gb300_test_withhold_tile_loads(int count) { return mipt_gb300_test_withhold_tile_halves(count, 3); }
+
+int mipt_gb300_test_withhold_tile_halves(int count, int halves)
 {
     if (count < 0) return fail(MIPT_GB300_E_INVALID, "count must be >= 0");
-    set_withheld_tile_loads(count);
+    if (halves < 1 || halves > 3) return fail(MIPT_GB300_E_INVALID, "halves must be 1, 2 or 3");
+    set_withheld_tile_loads(count, halves);
     return 0;
 }
 

@@ -938,7 +938,7 @@ __global__ void __launch_bounds__(512, 1)
                  std::size_t col_stride, const LayerMeas *__restrict__ meas, std::size_t meas_stride,
                  double *__restrict__ partials, int fuse_hist, int batch, const __grid_constant__ CUtensorMap tmap,
                  const __grid_constant__ TileTma tt, int *err, std::uint64_t col_keep, int col_scaled, int sparse,
-                 int withhold_first_load)
+                 int withheld)
 {
     // The swizzle pattern repeats every 1024 bytes.
     extern __shared__ __align__(1024) unsigned char smem_quads[];
@@ -1010,9 +1010,9 @@ __global__ void __launch_bounds__(512, 1)
             asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         }
         tile_fail = 0;
-        // withhold_first_load (a test hook): CTA 0 does not issue its first
-        // tile load, so its bounded wait runs out and the pass reports it.
-        if (first_item < items) fetch_item(first_item, withhold_first_load != 0 && first_item == 0 ? 0 : 3);
+        // withheld (a test hook): CTA 0 does not issue the loads of these halves
+        // of its first tile, so its bounded wait runs out and the pass reports it.
+        if (first_item < items) fetch_item(first_item, first_item == 0 ? 3 & ~withheld : 3);
     }
     int b = -1, m_loc = 0;
     bool hist = false;
@@ -1242,8 +1242,12 @@ __global__ void __launch_bounds__(512, 1)
                             if (tid == 0)
                             {
                                 atomicOr(err, 8);
-                                // Let loads in flight land before leaving.
-                                tile_bar_wait(&bar[0], phase);
+                                // Let loads in flight land before leaving. Group 1 gets here
+                                // only if the first round is the last one too; where halves
+                                // are loaded apart, the next item's first half is then on its
+                                // way, in bar[0]'s next phase.
+                                const bool ahead = grp == 1 && P.split && next < items;
+                                tile_bar_wait(&bar[0], ahead ? phase ^ 1u : phase);
                                 tile_bar_wait(&bar[1], phase);
                             }
                             return;
@@ -2349,15 +2353,17 @@ bool encode_tile_map(CUtensorMap &map, TileTma &t, const Cx<float> *states, int 
                               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-// Test hook: the next `count` TMA-fed pass launches withhold CTA 0's first
-// tile load (set_withheld_tile_loads), so their bounded tile waits run out.
-std::atomic<int> g_withheld_loads{0};
+// Test hook: the next launches of TMA-fed passes withhold loads of CTA 0's
+// first tile (set_withheld_tile_loads), so their bounded tile waits run out:
+// 4 * launches + mask of halves.
+std::atomic<long long> g_withheld_loads{0};
 
+// The halves that this launch withholds.
 int take_withheld_load()
 {
-    int c = g_withheld_loads.load();
-    while (c > 0 && !g_withheld_loads.compare_exchange_weak(c, c - 1)) {}
-    return c > 0 ? 1 : 0;
+    long long c = g_withheld_loads.load();
+    while (c >= 4 && !g_withheld_loads.compare_exchange_weak(c, c - 4)) {}
+    return c >= 4 ? static_cast<int>(c & 3) : 0;
 }
 
 // Launches k_pass_rounds<Real, RB, PAR> on its grid.
@@ -2512,7 +2518,7 @@ cudaError_t launch_collapse(Cx<Real> *states, std::uint64_t dim, int batch, cons
     return cudaGetLastError();
 }
 
-void set_withheld_tile_loads(int count) { g_withheld_loads.store(count > 0 ? count : 0); }
+void set_withheld_tile_loads(int count, int halves) { g_withheld_loads.store(4ll * count + (halves & 3)); }
 
 #define MG_INSTANTIATE(R)                                                                                        \
     template cudaError_t launch_init_zero<R>(Cx<R> *, std::uint64_t, int, cudaStream_t);                         \

@@ -125,10 +125,11 @@ cudaError_t launch_pass(Cx<Real> *states, int batch, const PassPlan &plan, const
                         int *err, cudaStream_t s, std::uint64_t col_keep = ~0ull, int col_scaled = 1,
                         int sparse = 0, int parity_mode = 0);
 
-// Test hook: the next `count` TMA-fed pass launches do not issue CTA 0's
-// first tile load; its bounded wait (well under a second) runs out, the CTA
-// sets bit 8 of the error flag and returns. No load is left in flight.
-void set_withheld_tile_loads(int count);
+// Test hook: the next `count` TMA-fed pass launches do not issue CTA 0's loads
+// of these halves (mask, 3: both) of its first tile; its bounded wait (well under
+// a second) runs out, the CTA sets bit 8 of the error flag and returns. No load
+// is left in flight.
+void set_withheld_tile_loads(int count, int halves);
 
 // Whether launch_pass accepts sparse / residual-collapse arguments for this
 // plan and batch size.
