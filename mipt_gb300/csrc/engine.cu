@@ -639,17 +639,17 @@ __device__ std::uint32_t build_item_prefix(std::uint32_t *pref, std::uint32_t *r
 // the CTA at flat index c runs items c, c + C, ... with C the number of CTAs,
 // so one launch shape serves both one item per CTA (C = items) and a
 // persistent grid.
-template <typename Real, int RB, bool PAR>
+template <bool PAR>
 __global__ void __launch_bounds__(256)
-    k_pass_rounds(Cx<Real> *__restrict__ states, PassPlan P, const Cx<Real> *__restrict__ gates,
+    k_pass_rounds(Cx<double> *__restrict__ states, PassPlan P, const Cx<double> *__restrict__ gates,
                   std::size_t gate_stride, const Collapse *__restrict__ col_in, std::size_t col_stride,
                   const LayerMeas *__restrict__ meas, std::size_t meas_stride, double *__restrict__ partials,
                   int fuse_hist, int batch, std::uint64_t col_keep, int col_scaled, int sparse)
 {
-    constexpr int NA = 1 << RB;
+    constexpr int RB = register_bits<double>(), NA = 1 << RB;
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    Cx<Real> *tile = reinterpret_cast<Cx<Real> *>(smem_raw);
-    __shared__ Cx<Real> U[kMaxPassGates][16];
+    Cx<double> *tile = reinterpret_cast<Cx<double> *>(smem_raw);
+    __shared__ Cx<double> U[kMaxPassGates][16];
     __shared__ double red[8];
 
     const PassGeom &g = P.geom;
@@ -662,7 +662,7 @@ __global__ void __launch_bounds__(256)
     {
         // The item prefix table follows the tile in dynamic shared memory.
         __shared__ std::uint32_t sred[32];
-        std::uint32_t *pref = reinterpret_cast<std::uint32_t *>(smem_raw + (sizeof(Cx<Real>) << g.k));
+        std::uint32_t *pref = reinterpret_cast<std::uint32_t *>(smem_raw + (sizeof(Cx<double>) << g.k));
         for (int i = 0; i < g.n_nl; ++i) sp.nlq |= 1ull << g.nl[i];
         items = build_item_prefix(pref, sred, g, sp.nlq, col_in, col_stride, batch);
         sp.pref = pref;
@@ -676,7 +676,7 @@ __global__ void __launch_bounds__(256)
         std::uint64_t tix;
         decode_item(item, sp_on, sp, g, col_in, col_stride, batch, b, tix);
         __syncthreads(); // the previous item's shared-memory reads are complete
-        Cx<Real> *psi = states + (static_cast<std::size_t>(b) << g.n);
+        Cx<double> *psi = states + (static_cast<std::size_t>(b) << g.n);
         const std::uint64_t base = scatter_bits(tix, g.nl, g.n_nl);
         const int tpar = PAR ? ((__popcll(base) + __popc(static_cast<unsigned>(tid))) & 1) : 0;
         if (b != cur_b)
@@ -700,9 +700,9 @@ __global__ void __launch_bounds__(256)
                 cl.parity = 0;
             }
         }
-        const Real scale = static_cast<Real>(cl.scale);
+        const double scale = cl.scale;
 
-        Cx<Real> amp[NA];
+        Cx<double> amp[NA];
         {
             const Round &R = P.round[0];
             std::uint64_t gt = base;
@@ -764,35 +764,19 @@ __global__ void __launch_bounds__(256)
                     amp[r] = tile[p];
                 }
             }
-            if constexpr (PAR)
+            if (R.slot[0] >= 0)
             {
-                if (R.slot[0] >= 0)
-                {
-                    if (P.gates.kind[R.slot[0]])
-                        apply_parity_slot<0>(amp, U[R.slot[0]], tpar);
-                    else
-                        apply_slot<0>(amp, U[R.slot[0]]);
-                }
-                if (RB >= 4 && R.slot[1] >= 0)
-                {
-                    if (P.gates.kind[R.slot[1]])
-                        apply_parity_slot<(RB >= 4 ? 1 : 0)>(amp, U[R.slot[1]], tpar);
-                    else
-                        apply_slot<(RB >= 4 ? 1 : 0)>(amp, U[R.slot[1]]);
-                }
-                if (RB >= 6 && R.slot[2] >= 0)
-                {
-                    if (P.gates.kind[R.slot[2]])
-                        apply_parity_slot<(RB >= 6 ? 2 : 0)>(amp, U[R.slot[2]], tpar);
-                    else
-                        apply_slot<(RB >= 6 ? 2 : 0)>(amp, U[R.slot[2]]);
-                }
+                if (PAR && P.gates.kind[R.slot[0]])
+                    apply_parity_slot<0>(amp, U[R.slot[0]], tpar);
+                else
+                    apply_slot<0>(amp, U[R.slot[0]]);
             }
-            else
+            if (R.slot[1] >= 0)
             {
-                if (R.slot[0] >= 0) apply_slot<0>(amp, U[R.slot[0]]);
-                if (RB >= 4 && R.slot[1] >= 0) apply_slot<(RB >= 4 ? 1 : 0)>(amp, U[R.slot[1]]);
-                if (RB >= 6 && R.slot[2] >= 0) apply_slot<(RB >= 6 ? 2 : 0)>(amp, U[R.slot[2]]);
+                if (PAR && P.gates.kind[R.slot[1]])
+                    apply_parity_slot<1>(amp, U[R.slot[1]], tpar);
+                else
+                    apply_slot<1>(amp, U[R.slot[1]]);
             }
         }
 
@@ -821,7 +805,7 @@ __global__ void __launch_bounds__(256)
             if (M.nchunks > 0)
             {
                 __syncthreads(); // the tile buffer is free
-                Real *val = reinterpret_cast<Real *>(smem_raw);
+                double *val = reinterpret_cast<double *>(smem_raw);
                 std::uint32_t jt = 0;
                 for (int i = 0; i < TB; ++i)
                     if ((tid >> i) & 1) jt |= 1u << Z.tid[i];
@@ -846,7 +830,6 @@ __global__ void __launch_bounds__(256)
         }
     }
 }
-
 
 // Shared-memory place of one tile bit of k_pass_quads' tile: the 128-byte
 // swizzle of the TMA loads, which flips the 16-byte chunk index (tile bits 1..3)
@@ -2366,23 +2349,23 @@ int take_withheld_load()
     return c >= 4 ? static_cast<int>(c & 3) : 0;
 }
 
-// Launches k_pass_rounds<Real, RB, PAR> on its grid.
-template <typename Real, int RB, bool PAR>
-cudaError_t launch_rounds(Cx<Real> *states, int batch, const PassPlan &plan, const Cx<Real> *layer_gates,
+// Launches k_pass_rounds<PAR> on its grid.
+template <bool PAR>
+cudaError_t launch_rounds(Cx<double> *states, int batch, const PassPlan &plan, const Cx<double> *layer_gates,
                           std::size_t gate_stride, const Collapse *collapse_in, std::size_t collapse_stride,
                           const LayerMeas *meas, std::size_t meas_stride, double *partials, int fuse_hist,
                           cudaStream_t s, std::uint64_t col_keep, int col_scaled, int sparse)
 {
-    const void *fn = reinterpret_cast<const void *>(&k_pass_rounds<Real, RB, PAR>);
-    const std::size_t smem = (sizeof(Cx<Real>) << plan.geom.k) +
+    const void *fn = reinterpret_cast<const void *>(&k_pass_rounds<PAR>);
+    const std::size_t smem = (sizeof(Cx<double>) << plan.geom.k) +
                              (sparse ? sizeof(std::uint32_t) * (static_cast<std::size_t>(batch) + 1) : 0);
     cudaError_t e = allow_dynamic_smem(fn, smem);
     if (e != cudaSuccess) return e;
-    const int threads = 1 << (plan.geom.k - RB);
+    const int threads = 1 << (plan.geom.k - register_bits<double>());
     const dim3 pgrid = pass_grid(fn, threads, smem, dim3(1u << plan.geom.n_nl, batch));
-    k_pass_rounds<Real, RB, PAR><<<pgrid, threads, smem, s>>>(states, plan, layer_gates, gate_stride, collapse_in,
-                                                          collapse_stride, meas, meas_stride, partials, fuse_hist,
-                                                          batch, col_keep, col_scaled, sparse);
+    k_pass_rounds<PAR><<<pgrid, threads, smem, s>>>(states, plan, layer_gates, gate_stride, collapse_in,
+                                                    collapse_stride, meas, meas_stride, partials, fuse_hist, batch,
+                                                    col_keep, col_scaled, sparse);
     return cudaGetLastError();
 }
 
@@ -2418,9 +2401,9 @@ cudaError_t launch_quads(Cx<float> *states, int batch, const PassPlan &plan, con
 bool sparse_pass_supported(const PassPlan &plan, bool fp32, int batch)
 {
     if (plan.rounds <= 0 || plan.geom.n_nl <= 0 || batch < 1) return false;
-    if (plan.rb != (fp32 ? 4 : 5)) return false;
+    if (plan.rb != (fp32 ? register_bits<float>() : register_bits<double>())) return false;
     if ((static_cast<std::uint64_t>(batch) << plan.geom.n_nl) >= (1ull << 31)) return false;
-    // Tile, histogram values, alignment and place table (FP32) + item table.
+    // Tile (FP32: histogram values and place table too) + item table.
     const std::size_t table = sizeof(std::uint32_t) * (static_cast<std::size_t>(batch) + 1);
     if (!fp32) return (sizeof(Cx<double>) << plan.geom.k) + table <= (200u << 10);
     return quad_smem(plan) + table <= (220u << 10);
@@ -2442,7 +2425,7 @@ cudaError_t launch_pass(Cx<Real> *states, int batch, const PassPlan &plan, const
         const bool par = parity_mode != 0;
         if constexpr (sizeof(Real) == 4)
         {
-            if (plan.rb != 4) return cudaErrorInvalidValue;
+            if (plan.rb != register_bits<Real>()) return cudaErrorInvalidValue;
             CUtensorMap map;
             TileTma tt{};
             const bool tma = use_persistent_pass() && use_tile_tma() && err != nullptr &&
@@ -2457,10 +2440,10 @@ cudaError_t launch_pass(Cx<Real> *states, int batch, const PassPlan &plan, const
         }
         else
         {
-            if (plan.rb != 5) return cudaErrorInvalidValue;
+            if (plan.rb != register_bits<Real>()) return cudaErrorInvalidValue;
 #define MG_ROUNDS(PARV)                                                                                               \
-    launch_rounds<Real, 5, PARV>(states, batch, plan, layer_gates, gate_stride, collapse_in, collapse_stride, meas,    \
-                                 meas_stride, partials, fuse_hist, s, col_keep, col_scaled, sparse)
+    launch_rounds<PARV>(states, batch, plan, layer_gates, gate_stride, collapse_in, collapse_stride, meas,             \
+                        meas_stride, partials, fuse_hist, s, col_keep, col_scaled, sparse)
             return par ? MG_ROUNDS(true) : MG_ROUNDS(false);
 #undef MG_ROUNDS
         }

@@ -68,7 +68,7 @@ std::vector<PassPlan> plan_layer(int n, const std::vector<Bond> &bonds, int kmax
 
 // Register bits per thread of the pass kernels (FP32 k_pass_quads: 4, FP64
 // k_pass_rounds: 5).
-template <typename Real> inline int register_bits() { return sizeof(Real) == 4 ? 4 : 5; }
+template <typename Real> constexpr int register_bits() { return sizeof(Real) == 4 ? 4 : 5; }
 
 // Tile geometry used for a stand-alone histogram of the sites in `chunk`:
 // low contiguous qubits, then as many unmeasured qubits as fit, so that few
@@ -93,14 +93,6 @@ struct LayerResult
     std::uint64_t outcome;   // bit q = measured value of site q (0 where unmeasured)
     double surprisal;        // -log P(joint outcome of the layer)
     double prob[kMaxChunks]; // branch / total of each chunk
-};
-
-template <typename Real>
-struct EngineLaunch
-{
-    Cx<Real> *states;
-    std::uint64_t dim;
-    int batch;
 };
 
 // Kernel launchers (engine.cu).
