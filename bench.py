@@ -328,7 +328,7 @@ def run_gb300(args):
         # launches (two layers: sparse, dense, sparse, dense) at 16
         # trajectories, 3.06 GB per launch on average = 191 MB per trajectory;
         # a launch streams each state it visits once, so it scales with the
-        # batch (profiles/k_pass_quads_L24_traffic_batch16.md).
+        # batch.
         traffic = PASS_TRAFFIC_PER_TRAJ * B
         roofline = {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
                     "traffic": traffic,
@@ -357,7 +357,7 @@ def run_gb300(args):
                 "alg_flops_per_step": gram_flops, "unreduced_flops_per_step": full_flops,
                 "tensor_pipe_active_pct_unreduced": GRAM_TENSOR_PIPE_PCT,
                 "tensor_pipe_source": "ncu sm__pipe_tensor_cycles_active, 2-trajectory capture of the unreduced "
-                                      "half-chain Gram (profiles/k_gram_tc_L24_halfcut_batch2.md)"}
+                                      "half-chain Gram"}
 
         # Plain FP64 per-trajectory path on the same GPU, one trajectory:
         # device time (CUDA events around the execute, as for `value`) and

@@ -588,7 +588,7 @@ int compat_entropy(const void *state, int n, const int *kept, int k, int fermion
         int err = 0;
         MG_CUDA(cudaMemcpy(&err, c.ws.eig_err.p, sizeof(int), cudaMemcpyDeviceToHost));
         if (err & 2) return fail(MIPT_GB300_E_INTERNAL, "eigensolver barrier wait timed out");
-        if (err) return fail(MIPT_GB300_E_NUMERIC, "an eigenvalue iteration did not converge");
+        if (err) return fail(MIPT_GB300_E_NUMERIC, "a reduced density matrix is not finite");
     }
     return 0;
 }
@@ -2644,7 +2644,7 @@ int mipt_gb300_batch_fetch(mipt_gb300_batch *b, std::uint64_t *measured, std::ui
     {
         MG_CUDA(cudaMemcpy(&err, b->ws.eig_err.p, sizeof(int), cudaMemcpyDeviceToHost));
         if (err & 2) return fail(MIPT_GB300_E_INTERNAL, "eigensolver barrier wait timed out");
-        if (err) return fail(MIPT_GB300_E_NUMERIC, "an eigenvalue iteration did not converge");
+        if (err) return fail(MIPT_GB300_E_NUMERIC, "a reduced density matrix is not finite");
     }
     const int count = b->count, T = b->T;
     if (measured) std::copy(b->measured.begin(), b->measured.end(), measured);

@@ -1051,7 +1051,7 @@ static_assert(R3_RUN == 1 << 4, "rho3_run");
 // and a widening by bit pattern need a tenth of those clocks. FP64 states: FP64
 // sums throughout, runs of 16 columns added to totals in shared memory.
 // Measured on GB300, 20 ring triples of an n = 20 FP32 state, the whole call:
-// 310 -> 112 us (93 us with the threads' pairs added as FP32 pairs).
+// 310 -> 112 us (88 to 93 us with the threads' pairs added as FP32 pairs).
 template <typename Real>
 __global__ void __launch_bounds__(R3_THREADS)
     k_rho3(const Cx<Real> *__restrict__ states, int n, const int *__restrict__ subs, int fermion,
@@ -1336,9 +1336,10 @@ cudaError_t gram_rho(const Cx<Real> *states, int n, const GramJob *d_jobs, int n
     // states exactly in FP64.
     // Compensated runs (rho entries to about 1e-13 of their scale) for tall
     // Grams (environment >= 64x the kept dimension), where the Gram's work
-    // dominates; exact FP64 sums otherwise: their entries are cleaner, and the
-    // QL sweeps, which dominate square Grams, resolve fewer noise-level
-    // eigenvalues (half-chain spectra of L = 16 and 18: 1.7x faster QL).
+    // dominates; exact FP64 sums otherwise, where the eigensolver does and the
+    // cleaner entries cost little of the call (64 FP32 half chains of n = 16 at
+    // 17 points: 194 ms; 166 ms with compensated runs, which moves the
+    // entropies by up to 1.3e-11).
     bool comp = false;
     if constexpr (sizeof(Real) == 4) comp = compensated_rho_sums() && n - k >= k + 6;
     if (k <= kSmallMaxK)
