@@ -1018,13 +1018,16 @@ __device__ __forceinline__ void comp_add(float x, float &s, float &c)
 }
 
 // x in FP64 by its bit pattern (a conversion takes the FP64 pipe 17 clocks a
-// warp); subnormal numbers, infinities and NaN are converted.
+// warp): the exponent moves by 1023 - 127, subnormal numbers are scaled to
+// normal ones first, infinities and NaN keep the largest exponent.
 __device__ __forceinline__ double widen(float x)
 {
-    const unsigned u = __float_as_uint(x), a = u & 0x7fffffffu;
-    if (a != 0u && a - 0x00800000u >= 0x7f000000u) return static_cast<double>(x);
-    const unsigned hi = (u & 0x80000000u) | (a != 0u ? (a >> 3) + 0x38000000u : 0u);
-    return __hiloint2double(static_cast<int>(hi), static_cast<int>(a << 29));
+    const unsigned a = __float_as_uint(x) & 0x7fffffffu;
+    const bool small = a < 0x00800000u;
+    const unsigned b = __float_as_uint(small ? x * 0x1p64f : x) & 0x7fffffffu;
+    unsigned hi = (b >> 3) + (small ? 832u << 20 : 896u << 20);
+    hi = b == 0u ? 0u : (a >= 0x7f800000u ? (b >> 3) | 0x7ff00000u : hi);
+    return __hiloint2double(static_cast<int>(hi | (__float_as_uint(x) & 0x80000000u)), static_cast<int>(b << 29));
 }
 
 // Columns per run of the FP32 sums: at most 16, and no more than the 2^(n-3)
@@ -1051,7 +1054,8 @@ static_assert(R3_RUN == 1 << 4, "rho3_run");
 // and a widening by bit pattern need a tenth of those clocks. FP64 states: FP64
 // sums throughout, runs of 16 columns added to totals in shared memory.
 // Measured on GB300, 20 ring triples of an n = 20 FP32 state, the whole call:
-// 310 -> 112 us (88 to 93 us with the threads' pairs added as FP32 pairs).
+// 310 -> 96 us (91 us with the threads' pairs added as FP32 pairs, 109 us with a
+// branch to conversions in widen).
 template <typename Real>
 __global__ void __launch_bounds__(R3_THREADS)
     k_rho3(const Cx<Real> *__restrict__ states, int n, const int *__restrict__ subs, int fermion,
@@ -1213,20 +1217,22 @@ __global__ void __launch_bounds__(R3_THREADS)
     for (int t = 4 * warp + (lane >> 3); t < R3_VALUES; t += 4 * (R3_THREADS / 32))
     {
         const int at = t * R3_THREADS + (lane & 7);
-        double x4[4] = {0.0, 0.0, 0.0, 0.0};
+        double x4[4];
         float e = 0.f;
 #pragma unroll
         for (int i = 0; i < 16; ++i)
         {
             const int a = at + 8 * ((i + t) & 15);
+            double y;
             if constexpr (kF32)
             {
-                const float2 y = reinterpret_cast<const float2 *>(r3_smem)[a];
-                x4[i & 3] += widen(y.x);
-                e += y.y;
+                const float2 p = reinterpret_cast<const float2 *>(r3_smem)[a];
+                y = widen(p.x);
+                e += p.y;
             }
             else
-                x4[i & 3] += r3_smem[a];
+                y = r3_smem[a];
+            x4[i & 3] = i < 4 ? y : x4[i & 3] + y;
         }
         double x = (x4[0] + x4[1]) + (x4[2] + x4[3]);
 #pragma unroll

@@ -46,3 +46,9 @@ def test_fp32_run_length(n):
 @pytest.mark.parametrize("fp64", [True, False])
 def test_overflow_is_infinite(fp64):
     assert first_entry(12, {0: 2.0 ** (600 if fp64 else 70), 5: 1.0}, fp64) == np.inf
+
+
+@pytest.mark.parametrize("exponent", [-60, -63, -65, -70, -74])
+def test_small_sums_are_exact(exponent):
+    """Sums around and below the smallest normal FP32 number."""
+    assert first_entry(12, {0: 2.0 ** exponent, 1: 2.0 ** exponent}, False) == 2.0 ** (2 * exponent + 1)
